@@ -47,6 +47,7 @@ struct Run3 {
   const int *chl;      // [cap][8] children
   const int *par;      // [cap] parent
   const int *off;      // [cap][3] offset of the box's cells in its parent (child offset)
+  const int4 *org;     // [cap] the box's first cell in its level's grid (x, y, z, 0-based), level - lo
   const double *geo;   // [cap][4] r_min[3], dr
   const double *lt;    // transport table, rows x 4, column-major
   const float *lt32;   // its FP32 copy (the mixed form's lookups)
@@ -1113,6 +1114,8 @@ __global__ void __launch_bounds__(NTH3) k3_reduce_final(Run3 R, int nb, int kind
   }
 }
 
+#include "a5g3_mg.cuh"
+
 // The step size of the next launches (device scalar, so that one captured
 // graph serves every step).
 __global__ void k3_set_dt(double *scal, double dt) { scal[S_DT] = dt; }
@@ -1149,6 +1152,7 @@ struct a5g3_ctx {
   double *d_cc = nullptr, *d_fc = nullptr, *d_lt = nullptr, *d_scal = nullptr, *d_part = nullptr;
   int *d_nc = nullptr, *d_nbr = nullptr, *d_chl = nullptr, *d_par = nullptr, *d_off = nullptr;
   int *d_ids = nullptr;
+  int4 *d_org = nullptr;
   double *d_geo = nullptr;
   int lt_rows = 0;
   double lt_xmin = 0, lt_inv_dx = 0;
@@ -1167,6 +1171,28 @@ struct a5g3_ctx {
   float *d_c32 = nullptr, *d_lt32 = nullptr;
 
   int coarse_top = 0;  // levels min_lvl..coarse_top run in one block (k3_coarse)
+
+  // The dense multigrid (a5g3_mg.cuh): P, F, O of all levels in FP64 with the
+  // kept corrections, and P, F, O of the FP32 correction solve. dense: the
+  // level grids fit its index arithmetic and its arrays could be allocated;
+  // the box-slot phases serve otherwise.
+  bool dense = false;
+  int dtop = 0;        // levels min_lvl..dtop run in one block (k3d_coarse)
+  long long dcells = 0;
+  double *d_den = nullptr, *d_corr = nullptr;
+  float *d_den32 = nullptr;
+  DAll dall{};
+  DCoarse dco{};
+  // a level with the row divisor of T's vectors (16 bytes on levels >= 1)
+  template <class T>
+  DLv dlv(int l) const {
+    DLv L = dall.lv[li(l)];
+    L.m_nxv = magic(L.nx2 / vec_of<T>(l));
+    return L;
+  }
+  template <class T>
+  static int vec_of(int l) { return l >= 1 ? (int)(16 / sizeof(T)) : 1; }
+  static unsigned magic(long long d) { return d <= 1 ? 0u : (unsigned)(((1ULL << 32) + d - 1) / d); }
   MG3<double> mg64() const {
     const size_t n = (size_t)cap * SLOT3;
     return MG3<double>{d_cc + I_PHI * n, d_cc + I_RHS * n, d_cc + I_FLD * n, voltage};
@@ -1191,6 +1217,7 @@ struct a5g3_ctx {
     R.chl = d_chl;
     R.par = d_par;
     R.off = d_off;
+    R.org = d_org;
     R.geo = d_geo;
     R.lt = d_lt;
     R.lt32 = d_lt32;
@@ -1483,11 +1510,137 @@ static void enq_solve_mixed(a5g3_ctx *c) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// The dense solve (a5g3_mg.cuh).
+template <class T>
+struct DArr {
+  T *P, *F, *O, *corr;
+  T v2;  // twice the potential of the high-z wall
+  Sweeps3 S;
+};
+static unsigned blocks_of(long long n, int per) { return (unsigned)((n + per - 1) / per); }
+
+// gsrb_boxes (:403-426): n_cycle red-black cycles on level l; first: the
+// restriction has just reached l
+template <class T>
+static void enq_dsweeps(a5g3_ctx *c, const DArr<T> &A, int l, int n_cycle, bool first) {
+  const DLv L = c->dlv<T>(l);
+  T *P = A.P + L.off, *F = A.F + L.off;
+  const T *O = A.O + L.off;
+  constexpr int VT = 16 / sizeof(T);
+  const int V = c->vec_of<T>(l);
+  const unsigned nb = blocks_of(L.half / V, 256);
+  for (int it = 0; it < 2 * n_cycle; it++) {
+    const bool f = first && it < 2;
+    if (V == 1 && f) k3d_sweep<T, 1, true><<<nb, 256, 0, c->stream>>>(L, P, F, O, it & 1, A.v2);
+    else if (V == 1) k3d_sweep<T, 1, false><<<nb, 256, 0, c->stream>>>(L, P, F, O, it & 1, A.v2);
+    else if (f) k3d_sweep<T, VT, true><<<nb, 256, 0, c->stream>>>(L, P, F, O, it & 1, A.v2);
+    else k3d_sweep<T, VT, false><<<nb, 256, 0, c->stream>>>(L, P, F, O, it & 1, A.v2);
+  }
+}
+// residual and restriction of level l (MODE RS_*)
+template <class T, int MODE>
+static void enq_drestrict(a5g3_ctx *c, const DArr<T> &A, int l) {
+  const DLv L = c->dall.lv[c->li(l)], C = c->dall.lv[c->li(l - 1)];
+  k3d_restrict<T, MODE><<<blocks_of(2LL * C.half, 128), 128, 0, c->stream>>>(
+      L, C, A.P + L.off, A.F + L.off, A.P + C.off, A.F + C.off, A.O + C.off, A.v2);
+}
+// correct_children of level l - 1, its k-th kept correction
+template <class T>
+static void enq_dcorrect(a5g3_ctx *c, const DArr<T> &A, int l, int k) {
+  const int q = c->li(l - 1);
+  const DLv L = c->dall.lv[q + 1], C = c->dall.lv[q];
+  T *cs = A.corr && k < c->dall.ncorr[q] ? A.corr + c->dall.coff[q] + k * corr_len(C) : nullptr;
+  k3d_correct<T><<<blocks_of(2LL * C.half, 128), 128, 0, c->stream>>>(L, C, A.P + L.off, A.P + C.off, A.O + C.off, cs,
+                                                                      A.v2);
+}
+template <class T>
+static void enq_dcoarse(a5g3_ctx *c, const DArr<T> &A, int mode, int k, bool last) {
+  DCoarse D = c->dco;
+  D.down = A.S.down;
+  D.up = A.S.up;
+  D.base = A.S.base;
+  k3d_coarse<T><<<1, NTHD, 3 * D.cells * sizeof(T), c->stream>>>(D, A.P, A.F, A.O, A.corr, mode, k, last ? 1 : 0, A.v2);
+}
+// mg3_fas_vcycle (:208-255) from level top
+template <class T>
+static void enq_dvcycle(a5g3_ctx *c, const DArr<T> &A, int top) {
+  const int lo = c->min_lvl, dt = c->dtop;
+  for (int l = top; l > std::max(dt, lo); l--) {
+    enq_dsweeps(c, A, l, A.S.down, l < top);
+    enq_drestrict<T, RS_RESID>(c, A, l);
+  }
+  if (dt >= lo) enq_dcoarse(c, A, CD_VCYCLE, top - dt, top == c->max_lvl);
+  else enq_dsweeps(c, A, lo, A.S.base, lo < top);
+  for (int l = std::max(dt, lo) + 1; l <= top; l++) {
+    enq_dcorrect(c, A, l, top - l + 1);
+    enq_dsweeps(c, A, l, A.S.up, false);
+  }
+}
+// the stages of mg3_fas_fmg (:186-202) above the coarse section
+template <class T>
+static void enq_dstages(a5g3_ctx *c, const DArr<T> &A) {
+  const int lo = c->min_lvl;
+  for (int l = std::max(lo, c->dtop + 1); l <= c->max_lvl; l++) {
+    if (l > lo) enq_dcorrect(c, A, l, 0);
+    enq_dvcycle(c, A, l);
+  }
+}
+// compute_fld's FP64 solve from the stored potential: set-up from the leaves'
+// slots, set_coarse_phi_rhs level by level, the FMG, then the parents'
+// right-hand sides and every box's potential and field back into the slots
+static void enq_dsolve(a5g3_ctx *c) {
+  const int lo = c->min_lvl, hi = c->max_lvl;
+  const DArr<double> A{c->d_den, c->d_den + c->dcells, c->d_den + 2 * c->dcells, c->d_corr, 2 * c->voltage, c->sweeps64()};
+  const DLv L = c->dall.lv[c->li(hi)];
+  k3d_ingest<<<c->count(hi), NTH3, 0, c->stream>>>(c->run(), L, c->ids(hi), A.P + L.off, A.F + L.off);
+  enq_drestrict<double, RS_RESID>(c, A, hi);
+  for (int l = hi - 1; l > std::max(lo, c->dtop); l--) enq_drestrict<double, RS_SETUP>(c, A, l);
+  if (c->dtop >= lo) {
+    enq_dcoarse(c, A, CD_FMG, 0, false);
+  } else {
+    const DLv B = c->dall.lv[0];
+    k3d_add_lpl<double><<<blocks_of(2LL * B.half, 128), 128, 0, c->stream>>>(B, A.P + B.off, A.F + B.off, A.v2);
+  }
+  enq_dstages(c, A);
+  // the parents are the first boxes of the level-ordered list
+  k3d_store_rhs<<<c->n_all() - c->count(hi), NTH3, 0, c->stream>>>(c->run(), c->dall, c->all_ids(), A.F, A.corr);
+  k3d_field<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->dall, c->all_ids(), c->li(hi), A.P);
+}
+// the mixed form's solve (enq_solve_mixed) on the dense FP32 levels
+static void enq_dsolve_mixed(a5g3_ctx *c) {
+  const int lo = c->min_lvl, hi = c->max_lvl;
+  const DArr<float> A{c->d_den32, c->d_den32 + c->dcells, c->d_den32 + 2 * c->dcells, nullptr, 0.0f,
+                      Sweeps3{c->sched.n_cycle_down, c->sched.n_cycle_up, c->sched.n_cycle_base}};
+  const DLv L = c->dall.lv[c->li(hi)];
+  for (int pass = 0; pass < c->sched.n_corr; pass++) {
+    k3d_mx_resid<<<c->count(hi), NTH3, 0, c->stream>>>(c->run(), L, c->ids(hi), A.F + L.off);
+    cudaMemsetAsync(A.P, 0, c->dcells * sizeof(float), c->stream);
+    if (c->sched.fmg) {
+      cudaMemsetAsync(A.O, 0, L.off * sizeof(float), c->stream);
+      for (int l = hi; l > std::max(lo, c->dtop); l--) enq_drestrict<float, RS_F>(c, A, l);
+      if (c->dtop >= lo) enq_dcoarse(c, A, CD_FMG_ZERO, 0, false);
+      enq_dstages(c, A);
+    } else {
+      enq_dvcycle(c, A, hi);
+    }
+    k3d_mx_acc<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->dall, c->all_ids(), A.P);
+  }
+}
+
 // compute_fld (src/streamer_3d.f90:309-345) with one FMG cycle; in the mixed
-// form (not on a first call) the defect-correction solve
+// form (not on a first call) the defect-correction solve. A first call (no
+// guess: once per run) takes the box-slot phases, whose base level starts
+// from the ghost cells in memory as the reference's does.
 static void enq_compute_fld(a5g3_ctx *c, bool no_guess) {
+  const bool mixed = c->precision == A5G_MIXED && !no_guess;
+  if (!mixed && !no_guess && c->dense) {
+    enq_dsolve(c);
+    return;
+  }
   k3_set_rhs<<<c->count(c->max_lvl), NTH3, 0, c->stream>>>(c->run(), c->ids(c->max_lvl));
-  if (c->precision == A5G_MIXED && !no_guess) enq_solve_mixed(c);
+  if (mixed && c->d_den32) enq_dsolve_mixed(c);
+  else if (mixed) enq_solve_mixed(c);
   else enq_fmg(c, false, no_guess);
   // the |E| side ghosts of every level are filled by k3_fld itself
   k3_fld<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->all_ids());
@@ -1549,6 +1702,82 @@ static int ready(a5g3_ctx *c) {
   return A5G_OK;
 }
 
+// The dense levels and their arrays. Leaves c->dense false (the box-slot
+// phases serve) where a level's grid is too large for the 32-bit index
+// arithmetic or device memory for the arrays is short.
+static void setup_dense(a5g3_ctx *c) {
+  const a5g3_params &p = c->p;
+  const int lo = c->min_lvl, hi = c->max_lvl, nlev = hi - lo + 1;
+  if (nlev > MAXLV3) return;
+  std::vector<int4> org((size_t)c->cap, int4{0, 0, 0, 0});
+  for (int id = 1; id <= c->max_id; id++)
+    org[id] = int4{(c->ix[3 * id] - 1) * c->nc[id], (c->ix[3 * id + 1] - 1) * c->nc[id],
+                   (c->ix[3 * id + 2] - 1) * c->nc[id], c->lvl[id] - lo};
+  DAll &D = c->dall;
+  long long off = 0, coff = 0;
+  for (int q = 0; q < nlev; q++) {
+    const int l = lo + q, nc = c->nc_of(l), s = l >= 1 ? 1 << (l - 1) : 1;
+    const long long nx = (long long)p.n_base[0] * s * nc, ny = (long long)p.n_base[1] * s * nc,
+                    nz = (long long)p.n_base[2] * s * nc, n = nx * ny * nz;
+    // the magic division is exact while the dividend times (m d - 2^32) stays below 2^32
+    for (const long long d : {nx / 2, nx / 4, nx / 8, ny}) {
+      const long long m = a5g3_ctx::magic(d), t = d == ny ? ny * nz : n / 2;
+      if (d > 1 && (double)t * (double)(m * d - (1LL << 32)) >= 4294967296.0) return;
+    }
+    if (n >= 2147483648LL) return;
+    DLv &L = D.lv[q];
+    L = DLv{(int)(nx / 2), (int)ny, (int)nz, (int)(n / 2), a5g3_ctx::magic(nx / 2), 0u, a5g3_ctx::magic(ny), off, 0, 0};
+    const double dr = c->geo[4 * c->lv_ids[c->lv_off[q]] + 3];
+    L.dx2 = dr * dr;
+    L.inv_dx2 = 1 / (dr * dr);
+    off += n;
+    D.ncorr[q] = hi - l;
+    D.coff[q] = coff;
+    coff += D.ncorr[q] * corr_len(L);
+  }
+  c->dcells = off;
+  // the coarse section: levels of at most DCOARSE cells, never the finest
+  DCoarse &C = c->dco;
+  c->dtop = lo - 1;
+  C.cells = 0;
+  C.nwarp = 0;
+  for (int l = lo; l < hi && C.n < 8 && 2 * D.lv[c->li(l)].half <= DCOARSE; l++) {
+    const int q = c->li(l);
+    C.lv[q] = D.lv[q];
+    C.goff[q] = D.lv[q].off;
+    C.lv[q].off = C.cells;
+    C.coff[q] = D.coff[q];
+    C.ncorr[q] = D.ncorr[q];
+    C.cells += 2 * D.lv[q].half;
+    if (C.nwarp == q && D.lv[q].half <= DWARP) C.nwarp = q + 1;
+    C.n = q + 1;
+    c->dtop = l;
+  }
+  // the attribute belongs to the kernel, not to this run: the most any run's
+  // coarse section takes (levels shrink by 8 from DCOARSE cells)
+  constexpr int sm = 3 * (DCOARSE + DCOARSE / 7 + 1);
+  if (C.cells * 3 > sm) return;
+  if (C.n > 0 && (cudaFuncSetAttribute(k3d_coarse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       sm * (int)sizeof(double)) != cudaSuccess ||
+                  cudaFuncSetAttribute(k3d_coarse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       sm * (int)sizeof(float)) != cudaSuccess)) {
+    cudaGetLastError();
+    return;
+  }
+  if (upload(c->d_org, org, c->stream) != A5G_OK) {
+    cudaGetLastError();
+    return;
+  }
+  // P, F of every level, O of every level but the finest, the corrections
+  const long long nO = D.lv[nlev - 1].off, nd = 2 * off + nO + coff;
+  if (cudaMalloc((void **)&c->d_den, nd * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  c->d_corr = c->d_den + 2 * off + nO;
+  c->dense = true;
+}
+
 extern "C" {
 
 const char *a5g3_last_error(void) { return g_err3.c_str(); }
@@ -1599,6 +1828,7 @@ int a5g3_create(const a5g3_params *p, a5g3_ctx **out) {
   // COARSE_BOXES boxes each (4,096 cells), never the finest level
   c->coarse_top = c->min_lvl - 1;
   for (int l = c->min_lvl; l < c->max_lvl && c->count(l) <= COARSE_BOXES; l++) c->coarse_top = l;
+  setup_dense(c);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return bail(fail3(A5G_ECUDA, "setup failed"));
   *out = c;
   return A5G_OK;
@@ -1612,7 +1842,8 @@ int a5g3_destroy(a5g3_ctx *c) {
   for (void *ptr : {(void *)c->d_cc, (void *)c->d_fc, (void *)c->d_lt, (void *)c->d_lt32, (void *)c->d_c32,
                     (void *)c->d_scal, (void *)c->d_part,
                     (void *)c->d_nc, (void *)c->d_nbr, (void *)c->d_chl, (void *)c->d_par, (void *)c->d_off,
-                    (void *)c->d_ids, (void *)c->d_geo})
+                    (void *)c->d_ids, (void *)c->d_geo, (void *)c->d_org, (void *)c->d_den,
+                    (void *)c->d_den32})
     if (ptr) cudaFree(ptr);
   if (c->h_red) cudaFreeHost(c->h_red);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1698,7 +1929,14 @@ int a5g3_set_precision(a5g3_ctx *c, int precision, const a5g_mg_schedule *sched)
   if (s.fmg < 0 || s.fmg > 1 || s.n_cycle_down < 1 || s.n_cycle_up < 1 || s.n_cycle_base < 1 || s.n_corr < 1 ||
       s.n_cycle_down > 8 || s.n_cycle_up > 8 || s.n_cycle_base > 64 || s.n_corr > 8)
     return fail3(A5G_EINVAL, "bad schedule (fmg 0/1, cycles 1..8, base 1..64, corrections 1..8)");
-  if (precision == A5G_MIXED && !c->d_c32) {
+  if (precision == A5G_MIXED && c->dense && !c->d_den32) {
+    const long long n = 2 * c->dcells + std::max(c->dall.lv[c->li(c->max_lvl)].off, 1LL);
+    if (cudaMalloc((void **)&c->d_den32, n * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      return fail3(A5G_ENOMEM, "device allocation of the FP32 multigrid storage failed");
+    }
+  }
+  if (precision == A5G_MIXED && !c->dense && !c->d_c32) {
     const size_t n = (size_t)3 * c->cap * SLOT3;
     if (cudaMalloc((void **)&c->d_c32, n * sizeof(float)) != cudaSuccess) {
       cudaGetLastError();
