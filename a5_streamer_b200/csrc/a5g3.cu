@@ -51,6 +51,8 @@ struct Run3 {
   const double *geo;   // [cap][4] r_min[3], dr
   const double *lt;    // transport table, rows x 4, column-major
   const float *lt32;   // its FP32 copy (the mixed form's lookups)
+  const double *lt4;   // the table by rows (4 values each), so that the two
+  const float *lt4f;   // columns of a lookup come with one load per row
   double *scal;        // device scalars (S_*)
   double *part;        // per-block partial reductions
   long long cap;       // slots (max_id + 1)
@@ -109,12 +111,15 @@ template <>
 __device__ __forceinline__ const double *lt_tab<double>(const Run3 &R) { return R.lt; }
 template <>
 __device__ __forceinline__ const float *lt_tab<float>(const Run3 &R) { return R.lt32; }
+// (int)ceil(x) for |x| < 2^31 in one conversion
+__device__ __forceinline__ int ceil_int(double x) { return __double2int_ru(x); }
+__device__ __forceinline__ int ceil_int(float x) { return __float2int_ru(x); }
 template <class T>
 __device__ __forceinline__ LocT<T> lt_locT(const Run3 &R, T x) {
   const T frac = (x - T(R.lt_xmin)) * T(R.lt_inv_dx);
   LocT<T> l;
   if (frac < T(2.0e9) && frac > T(-2.0e9)) {
-    l.ix = (int)ceil(frac);
+    l.ix = ceil_int(frac);
     l.fr = T(l.ix) - frac;
   } else {
     l.ix = frac > T(0) ? R.lt_rows : 0;
@@ -134,6 +139,23 @@ __device__ __forceinline__ T lt_colT(const Run3 &R, int col, const LocT<T> &l) {
   const T *c = lt_tab<T>(R) + (size_t)R.lt_rows * col;
   return l.fr * c[l.ix - 1] + (T(1) - l.fr) * c[l.ix];
 }
+// Columns col, col + 1 (col even) at a location, from the table by rows.
+template <class T>
+__device__ __forceinline__ void lt_pairT(const Run3 &R, int col, const LocT<T> &l, T &a, T &b);
+template <>
+__device__ __forceinline__ void lt_pairT<double>(const Run3 &R, int col, const LocT<double> &l, double &a, double &b) {
+  const double2 u = *reinterpret_cast<const double2 *>(R.lt4 + 4 * (l.ix - 1) + col);
+  const double2 v = *reinterpret_cast<const double2 *>(R.lt4 + 4 * l.ix + col);
+  a = l.fr * u.x + (1.0 - l.fr) * v.x;
+  b = l.fr * u.y + (1.0 - l.fr) * v.y;
+}
+template <>
+__device__ __forceinline__ void lt_pairT<float>(const Run3 &R, int col, const LocT<float> &l, float &a, float &b) {
+  const float2 u = *reinterpret_cast<const float2 *>(R.lt4f + 4 * (l.ix - 1) + col);
+  const float2 v = *reinterpret_cast<const float2 *>(R.lt4f + 4 * l.ix + col);
+  a = l.fr * u.x + (1.0f - l.fr) * v.x;
+  b = l.fr * u.y + (1.0f - l.fr) * v.y;
+}
 template <class T>
 __device__ __forceinline__ T koren_mlimT(T a, T b) {
   const T sixth = T(1 / 6.0);
@@ -151,8 +173,11 @@ __device__ __forceinline__ T norm2_3T(const T x[3]) {
     if (x[k] != T(0)) {
       const T ax = fabs(x[k]);
       if (scale < ax) {
-        const T v = scale / ax;
-        ssq = T(1) + ssq * v * v;
+        // (the first entry: 0 / ax = 0, ssq = 1 without the division)
+        if (scale != T(0)) {
+          const T v = scale / ax;
+          ssq = T(1) + ssq * v * v;
+        }
         scale = ax;
       } else {
         const T v = ax / scale;
@@ -173,8 +198,9 @@ __device__ __forceinline__ float dscale<float>() { return 0x1p-40f; }
 // ---------------------------------------------------------------------------
 // a3_tree_copy_cc for two variable pairs at once (elec -> elec_old, pion ->
 // pion_old at the start of a step); whole slots, two doubles per thread.
-__global__ void k3_copy2(Run3 R, int a0, int b0, int a1, int b1) {
-  const size_t n2 = (size_t)R.cap * SLOT3 / 2;
+// slots: how many of the first slots.
+__global__ void k3_copy2(Run3 R, int a0, int b0, int a1, int b1, long long slots) {
+  const size_t n2 = (size_t)slots * SLOT3 / 2;
   const double2 *s0 = reinterpret_cast<const double2 *>(VAR(R, a0));
   const double2 *s1 = reinterpret_cast<const double2 *>(VAR(R, a1));
   double2 *d0 = reinterpret_cast<double2 *>(VAR(R, b0));
@@ -188,8 +214,8 @@ __global__ void k3_copy2(Run3 R, int a0, int b0, int a1, int b1) {
 
 // average_dens (src/streamer_3d.f90:557-563): x = 0.5 (x + x_old) for n_e
 // and n_i, whole slots.
-__global__ void k3_average(Run3 R) {
-  const size_t n = (size_t)R.cap * SLOT3;
+__global__ void k3_average(Run3 R, long long slots) {
+  const size_t n = (size_t)slots * SLOT3;
   double *e = VAR(R, I_ELEC), *p = VAR(R, I_PION);
   const double *eo = VAR(R, I_ELEC_OLD), *po = VAR(R, I_PION_OLD);
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
@@ -370,28 +396,29 @@ __global__ void __launch_bounds__(NTH3) k3_update(Run3 R, const int *ids) {
 // times the sum of its eight child cells in column-major order. One block per
 // child box; the child's cells land in its octant of the parent (child
 // offset), so the blocks write disjoint parent cells.
+__device__ __forceinline__ void restrict_item(const Run3 &R, int id, int nc, int u, int iv) {
+  const int g = nc + 2, hnc = nc >> 1;
+  const int p = R.par[id], pg = R.nc[p] + 2;
+  const int *o = R.off + 3 * id;
+  const int i = u % hnc + 1, j = (u / hnc) % hnc + 1, k = u / (hnc * hnc) + 1;
+  const double *c = CC(R, iv, id);
+  const int f = ix3(g, 2 * i - 1, 2 * j - 1, 2 * k - 1);
+  double s = c[f];
+  s = s + c[f + 1];
+  s = s + c[f + g];
+  s = s + c[f + g + 1];
+  s = s + c[f + g * g];
+  s = s + c[f + g * g + 1];
+  s = s + c[f + g * g + g];
+  s = s + c[f + g * g + g + 1];
+  CC(R, iv, p)[ix3(pg, o[0] + i, o[1] + j, o[2] + k)] = 0.125 * s;
+}
 __global__ void __launch_bounds__(NTH3) k3_restrict(Run3 R, const int *ids, int iv0, int iv1) {
   const int id = ids[blockIdx.x];
-  const int nc = R.nc[id], g = nc + 2, hnc = nc >> 1, nh = hnc * hnc * hnc;
-  const int p = R.par[id];
-  const int pg = R.nc[p] + 2;
-  const int *o = R.off + 3 * id;
+  const int nc = R.nc[id], hnc = nc >> 1, nh = hnc * hnc * hnc;
   for (int t = threadIdx.x; t < 2 * nh; t += NTH3) {
     const int iv = t < nh ? iv0 : iv1;
-    if (iv < 0) continue;
-    const int u = t < nh ? t : t - nh;
-    const int i = u % hnc + 1, j = (u / hnc) % hnc + 1, k = u / (hnc * hnc) + 1;
-    const double *c = CC(R, iv, id);
-    const int f = ix3(g, 2 * i - 1, 2 * j - 1, 2 * k - 1);
-    double s = c[f];
-    s = s + c[f + 1];
-    s = s + c[f + g];
-    s = s + c[f + g + 1];
-    s = s + c[f + g * g];
-    s = s + c[f + g * g + 1];
-    s = s + c[f + g * g + g];
-    s = s + c[f + g * g + g + 1];
-    CC(R, iv, p)[ix3(pg, o[0] + i, o[1] + j, o[2] + k)] = 0.125 * s;
+    if (iv >= 0) restrict_item(R, id, nc, t < nh ? t : t - nh, iv);
   }
 }
 
@@ -1159,6 +1186,8 @@ struct a5g3_ctx {
   std::vector<double> h_lt;
   double voltage = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;  // the step's second branch, forked from and joined to stream inside its graph
+  cudaEvent_t ev[5] = {};
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   double *h_red = nullptr;  // pinned, 4 doubles
@@ -1180,6 +1209,8 @@ struct a5g3_ctx {
   int dtop = 0;        // levels min_lvl..dtop run in one block (k3d_coarse)
   long long dcells = 0;
   double *d_den = nullptr, *d_corr = nullptr;
+  double *d_dens = nullptr;  // the step's dense densities (Stage3: e1, p1, e2)
+  bool eps_one = false;      // eps is 1 everywhere (set_init_cond), not since written by the caller
   float *d_den32 = nullptr;
   DAll dall{};
   DCoarse dco{};
@@ -1221,6 +1252,8 @@ struct a5g3_ctx {
     R.geo = d_geo;
     R.lt = d_lt;
     R.lt32 = d_lt32;
+    R.lt4 = d_lt + 4 * lt_rows;  // behind the columns
+    R.lt4f = d_lt32 ? d_lt32 + 4 * lt_rows : nullptr;
     R.scal = d_scal;
     R.part = d_part;
     R.cap = cap;
@@ -1586,14 +1619,14 @@ static void enq_dstages(a5g3_ctx *c, const DArr<T> &A) {
     enq_dvcycle(c, A, l);
   }
 }
-// compute_fld's FP64 solve from the stored potential: set-up from the leaves'
-// slots, set_coarse_phi_rhs level by level, the FMG, then the parents'
-// right-hand sides and every box's potential and field back into the slots
+// The FP64 solve on the dense levels from the finest level's P and F:
+// set_coarse_phi_rhs level by level, then the FMG.
+static DArr<double> darr64(const a5g3_ctx *c) {
+  return DArr<double>{c->d_den, c->d_den + c->dcells, c->d_den + 2 * c->dcells, c->d_corr, 2 * c->voltage, c->sweeps64()};
+}
 static void enq_dsolve(a5g3_ctx *c) {
   const int lo = c->min_lvl, hi = c->max_lvl;
-  const DArr<double> A{c->d_den, c->d_den + c->dcells, c->d_den + 2 * c->dcells, c->d_corr, 2 * c->voltage, c->sweeps64()};
-  const DLv L = c->dall.lv[c->li(hi)];
-  k3d_ingest<<<c->count(hi), NTH3, 0, c->stream>>>(c->run(), L, c->ids(hi), A.P + L.off, A.F + L.off);
+  const DArr<double> A = darr64(c);
   enq_drestrict<double, RS_RESID>(c, A, hi);
   for (int l = hi - 1; l > std::max(lo, c->dtop); l--) enq_drestrict<double, RS_SETUP>(c, A, l);
   if (c->dtop >= lo) {
@@ -1603,18 +1636,17 @@ static void enq_dsolve(a5g3_ctx *c) {
     k3d_add_lpl<double><<<blocks_of(2LL * B.half, 128), 128, 0, c->stream>>>(B, A.P + B.off, A.F + B.off, A.v2);
   }
   enq_dstages(c, A);
-  // the parents are the first boxes of the level-ordered list
-  k3d_store_rhs<<<c->n_all() - c->count(hi), NTH3, 0, c->stream>>>(c->run(), c->dall, c->all_ids(), A.F, A.corr);
-  k3d_field<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->dall, c->all_ids(), c->li(hi), A.P);
 }
-// the mixed form's solve (enq_solve_mixed) on the dense FP32 levels
+// The mixed form's solve (enq_solve_mixed) on the dense levels: per pass the
+// FP64 residual of P, the FP32 correction from 0 and its accumulation.
 static void enq_dsolve_mixed(a5g3_ctx *c) {
   const int lo = c->min_lvl, hi = c->max_lvl;
+  const DArr<double> B = darr64(c);
   const DArr<float> A{c->d_den32, c->d_den32 + c->dcells, c->d_den32 + 2 * c->dcells, nullptr, 0.0f,
                       Sweeps3{c->sched.n_cycle_down, c->sched.n_cycle_up, c->sched.n_cycle_base}};
-  const DLv L = c->dall.lv[c->li(hi)];
+  const DLv L = c->dlv<double>(hi);
   for (int pass = 0; pass < c->sched.n_corr; pass++) {
-    k3d_mx_resid<<<c->count(hi), NTH3, 0, c->stream>>>(c->run(), L, c->ids(hi), A.F + L.off);
+    k3d_mx_resid<<<blocks_of(L.half, 256), 256, 0, c->stream>>>(L, B.P + L.off, B.F + L.off, A.F + L.off, B.v2);
     cudaMemsetAsync(A.P, 0, c->dcells * sizeof(float), c->stream);
     if (c->sched.fmg) {
       cudaMemsetAsync(A.O, 0, L.off * sizeof(float), c->stream);
@@ -1624,8 +1656,27 @@ static void enq_dsolve_mixed(a5g3_ctx *c) {
     } else {
       enq_dvcycle(c, A, hi);
     }
-    k3d_mx_acc<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->dall, c->all_ids(), A.P);
+    k3d_mx_acc<<<grid_for(c->dcells), 256, 0, c->stream>>>(B.P, A.P, c->dcells);
   }
+}
+// the solved potential and its field into the slots of every box (leaves
+// false: of the parents, the first boxes of the level-ordered list), in FP64
+// with the parents' right-hand sides
+static void enq_dstore(a5g3_ctx *c, bool mixed, bool leaves, cudaStream_t st) {
+  const int hi = c->max_lvl, np = c->n_all() - c->count(hi), n = leaves ? c->n_all() : np;
+  const DArr<double> A = darr64(c);
+  if (!mixed && np > 0) k3d_store_rhs<<<np, NTH3, 0, st>>>(c->run(), c->dall, c->all_ids(), A.F, A.corr);
+  const int tail = mixed ? -1 : c->li(hi);
+  if (c->eps_one) k3d_field<false><<<n, NTH3, 0, st>>>(c->run(), c->dall, c->all_ids(), tail, A.P);
+  else k3d_field<true><<<n, NTH3, 0, st>>>(c->run(), c->dall, c->all_ids(), tail, A.P);
+}
+// the potential of the boxes the solve starts from: the leaves, in the mixed
+// form (whose correction is added on every level) the parents too
+static void enq_dphi_in(a5g3_ctx *c, bool leaves, bool parents) {
+  const int hi = c->max_lvl, np = c->n_all() - c->count(hi);
+  const int *ids = parents ? c->all_ids() : c->ids(hi);
+  const int n = (leaves ? c->count(hi) : 0) + (parents ? np : 0);
+  if (n > 0) k3d_ingest_phi<<<n, NTH3, 0, c->stream>>>(c->run(), c->dall, ids, c->d_den);
 }
 
 // compute_fld (src/streamer_3d.f90:309-345) with one FMG cycle; in the mixed
@@ -1634,13 +1685,18 @@ static void enq_dsolve_mixed(a5g3_ctx *c) {
 // from the ghost cells in memory as the reference's does.
 static void enq_compute_fld(a5g3_ctx *c, bool no_guess) {
   const bool mixed = c->precision == A5G_MIXED && !no_guess;
-  if (!mixed && !no_guess && c->dense) {
-    enq_dsolve(c);
+  const int hi = c->max_lvl;
+  if (c->dense && !no_guess) {
+    const DLv L = c->dall.lv[c->li(hi)];
+    k3d_ingest_rhs<<<c->count(hi), NTH3, 0, c->stream>>>(c->run(), L, c->ids(hi), c->d_den + c->dcells + L.off);
+    enq_dphi_in(c, true, mixed);
+    if (mixed) enq_dsolve_mixed(c);
+    else enq_dsolve(c);
+    enq_dstore(c, mixed, true, c->stream);
     return;
   }
-  k3_set_rhs<<<c->count(c->max_lvl), NTH3, 0, c->stream>>>(c->run(), c->ids(c->max_lvl));
-  if (mixed && c->d_den32) enq_dsolve_mixed(c);
-  else if (mixed) enq_solve_mixed(c);
+  k3_set_rhs<<<c->count(hi), NTH3, 0, c->stream>>>(c->run(), c->ids(hi));
+  if (mixed) enq_solve_mixed(c);
   else enq_fmg(c, false, no_guess);
   // the |E| side ghosts of every level are filled by k3_fld itself
   k3_fld<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->all_ids());
@@ -1656,9 +1712,64 @@ static void enq_restrict(a5g3_ctx *c, int iv0, int iv1) {
 // finest level; consistent fluxes change nothing on a uniform octree. The
 // mixed form runs the fluxes and the update in FP32 and the field solves by
 // defect correction.
+// Where the leaves' permittivity is 1 and the dense levels are there, the
+// transport runs in the fused kernels of a5g3_mg.cuh between dense solves.
+template <class T>
+static void enq_step_dense(a5g3_ctx *c) {
+  const int hi = c->max_lvl, lo = c->min_lvl, n = c->count(hi), np = c->n_all() - n;
+  const bool mixed = c->precision == A5G_MIXED;
+  const DLv L = c->dall.lv[c->li(hi)];
+  const long long nl = 2LL * L.half;
+  const Stage3 S{c->d_dens, c->d_dens + nl, c->d_dens + 2 * nl, c->d_den + L.off, c->d_den + c->dcells + L.off, L};
+  // the parents' slots, and the unused slot 0, come before the leaves'
+  const long long slots = c->lv_ids[c->lv_off[c->li(hi)]];
+  auto solve = [&] {
+    if (mixed) enq_dsolve_mixed(c);
+    else enq_dsolve(c);
+  };
+  // What concerns only the parents' slots runs beside the leaves' kernels: on
+  // a second stream, forked and joined by events (inside the capture these
+  // become graph dependencies). The parents' right-hand sides and fields
+  // after the first solve are taken from the dense levels before the second
+  // solve overwrites those.
+  cudaStream_t main = c->stream, side = c->side;
+  auto after = [](cudaStream_t first, cudaStream_t then, cudaEvent_t ev) {
+    cudaEventRecord(ev, first);
+    cudaStreamWaitEvent(then, ev, 0);
+  };
+  after(main, side, c->ev[0]);
+  k3_copy2<<<grid_for(slots * SLOT3 / 2), NTH3, 0, side>>>(c->run(), I_ELEC, I_ELEC_OLD, I_PION, I_PION_OLD, slots);
+  k3d_stage<T, 1><<<n, NTH3, stage_smem<T, 1>(), main>>>(c->run(), S, c->ids(hi));
+  if (mixed) enq_dphi_in(c, false, true);
+  solve();
+  if (!mixed) {
+    after(main, side, c->ev[1]);
+    enq_dstore(c, false, false, side);
+  }
+  k3d_stage<T, 2><<<n, NTH3, stage_smem<T, 2>(), main>>>(c->run(), S, c->ids(hi));
+  after(side, main, c->ev[2]);
+  after(main, side, c->ev[3]);
+  int l = hi - 1;
+  k3d_restrict_dens<<<c->count(l), NTH3, 0, side>>>(c->run(), S, c->ids(l));
+  for (; l > lo && c->count(l) > COARSE_BOXES; l--)
+    k3_restrict<<<c->count(l), NTH3, 0, side>>>(c->run(), c->ids(l), I_ELEC, I_PION);
+  if (l > lo) k3_restrict_low<<<1, 1024, 0, side>>>(c->run(), l);
+  k3_gc<<<np, NTH3, 0, side>>>(c->run(), c->all_ids(), I_ELEC, I_PION, 0);
+  k3_average<<<grid_for(slots * SLOT3), NTH3, 0, side>>>(c->run(), slots);
+  k3d_final<<<n, NTH3, 0, main>>>(c->run(), S, c->ids(hi));
+  solve();
+  enq_dstore(c, mixed, true, main);
+  after(side, main, c->ev[4]);
+}
+
 static void enq_step(a5g3_ctx *c) {
+  if (c->dense && c->eps_one && c->max_lvl > 1) {
+    if (c->precision == A5G_MIXED) enq_step_dense<float>(c);
+    else enq_step_dense<double>(c);
+    return;
+  }
   const long long ncell = c->cap * SLOT3;
-  k3_copy2<<<grid_for(ncell / 2), NTH3, 0, c->stream>>>(c->run(), I_ELEC, I_ELEC_OLD, I_PION, I_PION_OLD);
+  k3_copy2<<<grid_for(ncell / 2), NTH3, 0, c->stream>>>(c->run(), I_ELEC, I_ELEC_OLD, I_PION, I_PION_OLD, c->cap);
   const int hi = c->max_lvl;
   const bool mx = c->precision == A5G_MIXED;
   for (int stage = 1; stage <= 2; stage++) {
@@ -1676,7 +1787,7 @@ static void enq_step(a5g3_ctx *c) {
       k3_gc<<<c->n_all() - c->count(hi), NTH3, 0, c->stream>>>(c->run(), c->all_ids(), I_ELEC, I_PION, 0);
     if (stage == 1) enq_compute_fld(c, false);
   }
-  k3_average<<<grid_for(ncell), NTH3, 0, c->stream>>>(c->run());
+  k3_average<<<grid_for(ncell), NTH3, 0, c->stream>>>(c->run(), c->cap);
   enq_compute_fld(c, false);
 }
 
@@ -1689,6 +1800,13 @@ static void drop_graph(a5g3_ctx *c) {
     c->exec = nullptr;
     c->graph = nullptr;
   }
+}
+
+// eps has been written: by set_init_cond (1 everywhere) or by the caller. A
+// captured step holds the choice it led to.
+static void eps_written(a5g3_ctx *c, bool one) {
+  if (c->eps_one != one) drop_graph(c);
+  c->eps_one = one;
 }
 
 static int launched(a5g3_ctx *c) {
@@ -1757,10 +1875,12 @@ static void setup_dense(a5g3_ctx *c) {
   // coarse section takes (levels shrink by 8 from DCOARSE cells)
   constexpr int sm = 3 * (DCOARSE + DCOARSE / 7 + 1);
   if (C.cells * 3 > sm) return;
-  if (C.n > 0 && (cudaFuncSetAttribute(k3d_coarse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if ((cudaFuncSetAttribute(k3d_coarse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        sm * (int)sizeof(double)) != cudaSuccess ||
                   cudaFuncSetAttribute(k3d_coarse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       sm * (int)sizeof(float)) != cudaSuccess)) {
+                                       sm * (int)sizeof(float)) != cudaSuccess ||
+                  cudaFuncSetAttribute(k3d_stage<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)stage_smem<double, 2>()) != cudaSuccess)) {
     cudaGetLastError();
     return;
   }
@@ -1768,13 +1888,18 @@ static void setup_dense(a5g3_ctx *c) {
     cudaGetLastError();
     return;
   }
-  // P, F of every level, O of every level but the finest, the corrections
-  const long long nO = D.lv[nlev - 1].off, nd = 2 * off + nO + coff;
+  // P, F of every level, O of every level but the finest, the corrections,
+  // and the step's dense densities
+  const long long nO = D.lv[nlev - 1].off, nd = 2 * off + nO + coff + 6LL * D.lv[nlev - 1].half;
   if (cudaMalloc((void **)&c->d_den, nd * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
+  for (cudaEvent_t &e : c->ev)
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return;
+  if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess) return;
   c->d_corr = c->d_den + 2 * off + nO;
+  c->d_dens = c->d_corr + coff;
   c->dense = true;
 }
 
@@ -1846,6 +1971,9 @@ int a5g3_destroy(a5g3_ctx *c) {
                     (void *)c->d_den32})
     if (ptr) cudaFree(ptr);
   if (c->h_red) cudaFreeHost(c->h_red);
+  for (cudaEvent_t e : c->ev)
+    if (e) cudaEventDestroy(e);
+  if (c->side) cudaStreamDestroy(c->side);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return A5G_OK;
@@ -1903,12 +2031,18 @@ int a5g3_set_table(a5g3_ctx *c, int n_rows, int n_cols, double x_min, double inv
   if (c->d_lt) cudaFree(c->d_lt);
   c->d_lt = nullptr;
   c->h_lt.assign(rc, rc + (size_t)n_rows * n_cols);
-  CK3(cudaMalloc((void **)&c->d_lt, c->h_lt.size() * sizeof(double)));
-  CK3(cudaMemcpy(c->d_lt, rc, c->h_lt.size() * sizeof(double), cudaMemcpyHostToDevice));
+  // the columns, then the same values by rows (4 n_rows doubles before them:
+  // every row starts on a 32-byte boundary)
+  std::vector<double> both(c->h_lt);
+  both.resize(2 * c->h_lt.size());
+  for (int r = 0; r < n_rows; r++)
+    for (int q = 0; q < 4; q++) both[4 * (size_t)n_rows + 4 * (size_t)r + q] = rc[(size_t)q * n_rows + r];
+  CK3(cudaMalloc((void **)&c->d_lt, both.size() * sizeof(double)));
+  CK3(cudaMemcpy(c->d_lt, both.data(), both.size() * sizeof(double), cudaMemcpyHostToDevice));
   {
     // FP32 copy for the lookups of the mixed form
-    std::vector<float> t32(c->h_lt.size());
-    for (size_t k = 0; k < t32.size(); k++) t32[k] = (float)c->h_lt[k];
+    std::vector<float> t32(both.size());
+    for (size_t k = 0; k < t32.size(); k++) t32[k] = (float)both[k];
     if (c->d_lt32) cudaFree(c->d_lt32);
     c->d_lt32 = nullptr;
     CK3(cudaMalloc((void **)&c->d_lt32, t32.size() * sizeof(float)));
@@ -1976,11 +2110,13 @@ int a5g3_set_init_cond(a5g3_ctx *c, double bg, int n_seeds, const double *r0, co
     S.falloff[s] = falloff[s];
   }
   k3_init<<<c->n_all(), NTH3, 0, c->stream>>>(c->run(), c->all_ids(), S);
+  eps_written(c, true);
   return launched(c);
 }
 
 int a5g3_upload_cc(a5g3_ctx *c, int iv, const double *h) {
   if (!c || !h || iv < 0 || iv >= NV3) return fail3(A5G_EINVAL, "bad argument");
+  if (iv == I_EPS) eps_written(c, false);
   CK3(cudaMemcpyAsync(c->d_cc + (size_t)iv * c->cap * SLOT3, h, (size_t)c->cap * SLOT3 * sizeof(double),
                       cudaMemcpyHostToDevice, c->stream));
   CK3(cudaStreamSynchronize(c->stream));
@@ -2010,7 +2146,8 @@ int a5g3_download_fc(a5g3_ctx *c, int d, int f, double *h) {
 
 int a5g3_tree_copy_cc(a5g3_ctx *c, int a, int b) {
   if (!c || a < 0 || a >= NV3 || b < 0 || b >= NV3) return fail3(A5G_EINVAL, "bad argument");
-  k3_copy2<<<grid_for(c->cap * SLOT3 / 2), NTH3, 0, c->stream>>>(c->run(), a, b, -1, -1);
+  k3_copy2<<<grid_for(c->cap * SLOT3 / 2), NTH3, 0, c->stream>>>(c->run(), a, b, -1, -1, c->cap);
+  if (b == I_EPS) eps_written(c, false);
   return launched(c);
 }
 static int with_dt(a5g3_ctx *c, double dt) {
@@ -2042,7 +2179,7 @@ int a5g3_gc_tree(a5g3_ctx *c, int iv) {
 }
 int a5g3_average_dens(a5g3_ctx *c) {
   if (!c) return fail3(A5G_EINVAL, "null context");
-  k3_average<<<grid_for(c->cap * SLOT3), NTH3, 0, c->stream>>>(c->run());
+  k3_average<<<grid_for(c->cap * SLOT3), NTH3, 0, c->stream>>>(c->run(), c->cap);
   return launched(c);
 }
 int a5g3_compute_fld(a5g3_ctx *c, int no_guess) {

@@ -506,26 +506,36 @@ struct DAll {
   long long coff[MAXLV3];
   int ncorr[MAXLV3];
 };
+__device__ __forceinline__ double space_charge(double e, double p) { return UC_ELEM_CHARGE / UC_EPS0 * (e - p); }
 
-// compute_fld's space charge on whole slots of the leaves (k3_set_rhs), and
-// the leaves' right-hand side and potential into the finest dense level. A
-// row of 8 cells goes to two runs of 4, one per colour: 32-byte sectors.
-__global__ void __launch_bounds__(NTH3) k3d_ingest(Run3 R, DLv L, const int *ids, double *P, double *F) {
+// compute_fld's space charge on whole slots of the leaves (k3_set_rhs), into
+// the slots and the finest dense level. A row of 8 cells goes to two runs of
+// 4, one per colour: 32-byte sectors.
+__global__ void __launch_bounds__(NTH3) k3d_ingest_rhs(Run3 R, DLv L, const int *ids, double *F) {
   const int id = ids[blockIdx.x];
   constexpr int g = NC3 + 2;
-  const double fac = UC_ELEM_CHARGE / UC_EPS0;
-  const double *e = CC(R, I_ELEC, id), *p = CC(R, I_PION, id), *phi = CC(R, I_PHI, id);
+  const double *e = CC(R, I_ELEC, id), *p = CC(R, I_PION, id);
   double *rhs = CC(R, I_RHS, id);
   const int4 o = R.org[id];
   for (int c = threadIdx.x; c < SLOT3; c += NTH3) {
-    const double v = fac * (e[c] - p[c]);
+    const double v = space_charge(e[c], p[c]);
     rhs[c] = v;
     const int i = c % g, j = (c / g) % g, k = c / (g * g);
-    if (i >= 1 && i <= NC3 && j >= 1 && j <= NC3 && k >= 1 && k <= NC3) {
-      const int d = didx(L, o.x + i - 1, o.y + j - 1, o.z + k - 1);
-      F[d] = v;
-      P[d] = phi[c];
-    }
+    if (i >= 1 && i <= NC3 && j >= 1 && j <= NC3 && k >= 1 && k <= NC3)
+      F[didx(L, o.x + i - 1, o.y + j - 1, o.z + k - 1)] = v;
+  }
+}
+// the potential of the boxes in ids into their dense levels
+__global__ void __launch_bounds__(NTH3) k3d_ingest_phi(Run3 R, const __grid_constant__ DAll D, const int *ids,
+                                                       double *P) {
+  const int id = ids[blockIdx.x];
+  const int4 o = R.org[id];
+  const DLv &L = D.lv[o.w];
+  const int nc = R.nc[id], g = nc + 2;
+  const double *phi = CC(R, I_PHI, id);
+  for (int t = threadIdx.x; t < nc * nc * nc; t += NTH3) {
+    const int i = t % nc, j = (t / nc) % nc, k = t / (nc * nc);
+    P[L.off + didx(L, o.x + i, o.y + j, o.z + k)] = phi[ix3(g, i + 1, j + 1, k + 1)];
   }
 }
 
@@ -564,25 +574,46 @@ __global__ void __launch_bounds__(NTH3) k3d_store_rhs(Run3 R, const __grid_const
       x = min(max(x, 0), nx - 1);
       y = min(max(y, 0), L.ny - 1);
       z = min(max(z, 0), L.nz - 1);
-      const long long at = high ? 2LL * L.half + y * nx + x : didx(L, x, y, z);
-      for (int q = 0; q < nk; q++) {
-        const double w = cr[q * cl + at];
-        v = v + (low ? -w : w);
+      const double *w = cr + (high ? 2LL * L.half + y * nx + x : didx(L, x, y, z));
+      for (int q = 0; q < nk; q += 4) {  // four loads in flight, added in order
+        double a[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) a[m] = q + m < nk ? w[(q + m) * cl] : 0.0;
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+          if (q + m < nk) v = v + (low ? -a[m] : a[m]);
       }
     }
     rhs[c] = v;
   }
 }
 
-// The potential of every box (cells and side ghosts, sides_bc_pot on the
-// walls) from the dense levels into its slot, then fld_from_pot
-// (src/streamer_3d.f90:348-393) from the staged values, as fld_box, with
-// the |E| side ghosts pushed. Leaves: the edge and corner entries of tmp as
-// the FMG's copy leaves them (phi's).
-template <int NCT>
-__device__ __forceinline__ void field_box(const Run3 &R, const DLv &L, const int4 o, int id, bool leaf, const double *P,
-                                          double *sp, double *sfc) {
-  const int nc = NCT ? NCT : R.nc[id], g = nc + 2, gs = g * g * g, F = (nc + 1) * nc * nc, nx = 2 * L.nx2;
+// Potential at (x, y, z) of a dense level or one cell beyond a wall
+// (sides_bc_pot, src/streamer_3d.f90:693-715)
+__device__ __forceinline__ double phi_at(const DLv &L, const double *P, int x, int y, int z, double v2) {
+  const double p = dval(L, P, min(max(x, 0), 2 * L.nx2 - 1), min(max(y, 0), L.ny - 1), min(max(z, 0), L.nz - 1));
+  return z < 0 ? -p : (z >= L.nz ? v2 - p : p);
+}
+// Field of a face from the potentials beside it (fld_from_pot,
+// src/streamer_3d.f90:348-393): on box-edge faces 2 inv_dr dphi eps / (eps0 +
+// eps), whose division by 2 is exact where both eps are 1.
+__device__ __forceinline__ double face_of(double dphi, double inv_dr, bool edge, double e_own, double e_sum) {
+  if (!edge) return inv_dr * dphi;
+  if (e_own == 1.0 && e_sum == 2.0) return (2 * inv_dr * dphi) * 0.5;
+  return 2 * inv_dr * dphi * e_own / e_sum;
+}
+
+// The potential of every box (cells and side ghosts) from the dense levels
+// into its slot, then fld_from_pot from the staged values: each thread forms
+// the six faces of its cells, so no face passes through shared memory, and
+// pushes the |E| side ghosts (level 6: 568 us with staged faces and eps read
+// on every face, 468 so). EPS: read eps on the box-edge faces (else it
+// is 1 everywhere). tail: the edge and corner entries of the leaves' tmp as
+// the FP64 FMG's copy leaves them (phi's).
+template <int NCT, bool EPS>
+__device__ __forceinline__ void field_box(const Run3 &R, const DLv &L, const int4 o, int id, bool tail, const double *P,
+                                          double *sp) {
+  const int nc = NCT ? NCT : R.nc[id], g = nc + 2, gs = g * g * g;
   const double inv_dr = 1 / R.geo[4 * id + 3], v2 = 2 * R.voltage;
   const double *eps = CC(R, I_EPS, id);
   double *phi = CC(R, I_PHI, id), *fld = CC(R, I_FLD, id);
@@ -590,102 +621,396 @@ __device__ __forceinline__ void field_box(const Run3 &R, const DLv &L, const int
     const int i = c % g, j = (c / g) % g, k = c / (g * g);
     const int in = (i >= 1 && i <= nc) + (j >= 1 && j <= nc) + (k >= 1 && k <= nc);
     if (in < 2) {
-      if (leaf) fld[c] = phi[c];
+      if (tail) fld[c] = phi[c];
       continue;
     }
-    const int x = o.x + i - 1, y = o.y + j - 1, z = o.z + k - 1;
-    const double p = dval(L, P + L.off, min(max(x, 0), nx - 1), min(max(y, 0), L.ny - 1), min(max(z, 0), L.nz - 1));
-    const double v = z < 0 ? -p : (z >= L.nz ? v2 - p : p);
+    const double v = phi_at(L, P + L.off, o.x + i - 1, o.y + j - 1, o.z + k - 1, v2);
     sp[c] = v;
     phi[c] = v;
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < 3 * F; q += NTH3) {
-    const int d = q / F, r = q - d * F;
-    int i, j, k, a;
-    if (d == 0) {
-      i = r % (nc + 1) + 1;
-      j = (r / (nc + 1)) % nc + 1;
-      k = r / ((nc + 1) * nc) + 1;
-      a = i;
-    } else if (d == 1) {
-      i = r % nc + 1;
-      j = (r / nc) % (nc + 1) + 1;
-      k = r / (nc * (nc + 1)) + 1;
-      a = j;
-    } else {
-      i = r % nc + 1;
-      j = (r / nc) % nc + 1;
-      k = r / (nc * nc) + 1;
-      a = k;
-    }
-    const int st = d == 0 ? 1 : d == 1 ? g : g * g;
-    const int c0 = ix3(g, i, j, k), cm = c0 - st;
-    double v;
-    if (a == 1) {
-      v = 2 * inv_dr * (sp[cm] - sp[c0]) * eps[cm] / (eps[c0] + eps[cm]);
-    } else if (a == nc + 1) {
-      v = 2 * inv_dr * (sp[cm] - sp[c0]) * eps[c0] / (eps[c0] + eps[cm]);
-    } else {
-      v = inv_dr * (sp[cm] - sp[c0]);
-    }
-    sfc[d * FSLOT3 + r] = v;
-    FC(R, d, F_FLD, id)[r] = v;
-  }
-  __syncthreads();
   const int n = nc * nc * nc;
+  double *fx = FC(R, 0, F_FLD, id), *fy = FC(R, 1, F_FLD, id), *fz = FC(R, 2, F_FLD, id);
   for (int t = threadIdx.x; t < n; t += NTH3) {
-    const int i = t % nc + 1, j = (t / nc) % nc + 1, k = t / (nc * nc) + 1;
+    const int i = t % nc + 1, j = (t / nc) % nc + 1, k = t / (nc * nc) + 1, c = ix3(g, i, j, k);
+    const int pos[3] = {i, j, k}, st[3] = {1, g, g * g};
+    double f[3][2];
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        // face h of direction d: between cells cm and c0
+        const int c0 = c + h * st[d], cm = c0 - st[d], a = pos[d] + h;
+        const bool edge = a == 1 || a == nc + 1;
+        double eo = 1.0, es = 2.0;
+        if (EPS && edge) {
+          eo = eps[a == 1 ? cm : c0];
+          es = eps[c0] + eps[cm];
+        }
+        f[d][h] = face_of(sp[cm] - sp[c0], inv_dr, edge, eo, es);
+      }
     const int xl = (i - 1) + (nc + 1) * ((j - 1) + nc * (k - 1));
     const int yl = (i - 1) + nc * ((j - 1) + (nc + 1) * (k - 1));
     const int zl = (i - 1) + nc * ((j - 1) + nc * (k - 1));
-    const double sx = sfc[xl] + sfc[xl + 1];
-    const double sy = sfc[FSLOT3 + yl] + sfc[FSLOT3 + yl + nc];
-    const double sz = sfc[2 * FSLOT3 + zl] + sfc[2 * FSLOT3 + zl + nc * nc];
+    fx[xl] = f[0][0];
+    fy[yl] = f[1][0];
+    fz[zl] = f[2][0];
+    if (i == nc) fx[xl + 1] = f[0][1];
+    if (j == nc) fy[yl + nc] = f[1][1];
+    if (k == nc) fz[zl + nc * nc] = f[2][1];
+    const double sx = f[0][0] + f[0][1], sy = f[1][0] + f[1][1], sz = f[2][0] + f[2][1];
     const double v = 0.5 * sqrt(sx * sx + sy * sy + sz * sz);
-    fld[ix3(g, i, j, k)] = v;
+    fld[c] = v;
     push_side_ghosts(R, I_FLD, id, nc, i, j, k, v);
   }
 }
+template <bool EPS>
 __global__ void __launch_bounds__(NTH3) k3d_field(Run3 R, const __grid_constant__ DAll D, const int *ids, int hi,
                                                   const double *P) {
-  __shared__ double sp[SLOT3], sfc[3 * FSLOT3];
+  __shared__ double sp[SLOT3];
   const int id = ids[blockIdx.x];
   const int4 o = R.org[id];
   const DLv &L = D.lv[o.w];
-  if (R.nc[id] == NC3) field_box<NC3>(R, L, o, id, o.w == hi, P, sp, sfc);
-  else field_box<0>(R, L, o, id, o.w == hi, P, sp, sfc);
+  if (R.nc[id] == NC3) field_box<NC3, EPS>(R, L, o, id, o.w == hi, P, sp);
+  else field_box<0, EPS>(R, L, o, id, o.w == hi, P, sp);
 }
 
-// The mixed form: the FP64 residual of the leaves rhs - lpl(phi), ghost
-// neighbours from their sources with the applied voltage, into the FP32
-// correction's finest level; and phi += c on the cells of every box with the
-// FP64 ghost fill of phi pushed in the same pass.
-__global__ void __launch_bounds__(NTH3) k3d_mx_resid(Run3 R, DLv L, const int *ids, float *F) {
+// The mixed form: the FP64 residual F - lpl(P) of the finest level into the
+// FP32 correction's right-hand side, and P += c on every cell of every level.
+__global__ void __launch_bounds__(256) k3d_mx_resid(DLv L, const double *P, const double *F, float *F32, double v2) {
+  const unsigned t = blockIdx.x * 256u + threadIdx.x;
+  constexpr int V = 2;
+  if (t >= (unsigned)(2 * L.half / V)) return;
+  const int c = t >= (unsigned)(L.half / V), u = t - c * (L.half / V);
+  const int nv = L.nx2 / V, r = fastdiv(u, L.m_nxv), xv = (u - r * nv) * V;
+  const int z = fastdiv(r, L.m_ny), y = r - z * L.ny, b = r * L.nx2 + xv;
+  const Vec<double, V> o = ldv<double, V>(P + c * L.half + b), f = ldv<double, V>(F + c * L.half + b);
+  const Nbr<double, V> n = neighbours<double, V>(L, P + (1 - c) * L.half, o, b, xv, y, z, (c + y + z) & 1, v2);
+  Vec<float, V> w;
+#pragma unroll
+  for (int k = 0; k < V; k++) w.v[k] = (float)(f.v[k] - lpl_of<double, V>(n, k, o.v[k], L.inv_dx2));
+  *reinterpret_cast<Vec<float, V> *>(F32 + c * L.half + b) = w;
+}
+__global__ void __launch_bounds__(256) k3d_mx_acc(double *P, const float *c, long long n) {
+  for (long long k = blockIdx.x * 256LL + threadIdx.x; k < n; k += gridDim.x * 256LL) P[k] = P[k] + (double)c[k];
+}
+
+// ---------------------------------------------------------------------------
+// The transport of a time step on the leaves (eps 1 everywhere), one block
+// per box. Two kernels replace the old-density copy, the two flux and update
+// passes, the average and the space charge of the slot form; what is read
+// again only inside the step stays in dense arrays (x fastest): stage 1
+// writes n_e, n_i and the right-hand side of the first solve, stage 2 takes
+// |E| and the face fields from the dense potential, so that the first solve
+// needs no field pass. The parents' densities after stage 1 are never read,
+// so only stage 2's are restricted. At level 6 (16.8M cells, launch list):
+// copies, fluxes, updates, average and space charge 3,450 us in the slot
+// form; here stage 1 640, stage 2 903, k3d_final 311.
+struct Stage3 {
+  double *e1, *p1, *e2;  // dense densities of the finest level (p: updated in place)
+  double *P, *F;         // finest dense level: potential, right-hand side
+  DLv L;
+};
+constexpr int G12 = NC3 + 4, S12 = G12 * G12 * G12;
+__device__ __forceinline__ int ix12(int i, int j, int k) { return (i + 1) + G12 * ((j + 1) + G12 * (k + 1)); }
+__device__ __forceinline__ size_t nat(const DLv &L, int x, int y, int z) {
+  return ((size_t)z * L.ny + y) * (2 * L.nx2) + x;
+}
+// bytes of shared memory: n_e with two ghost layers, |E|, the fluxes, and in
+// stage 2 the potential
+template <class T, int STAGE>
+constexpr size_t stage_smem() {
+  return (STAGE == 2 ? sizeof(double) * S12 : 0) + sizeof(T) * (S12 + SLOT3 + 3 * FSLOT3);
+}
+
+// Electron flux through one face (src/streamer_3d.f90:396-554, as
+// k3_fluxes): em2, em1 | e0, ep1 the scaled densities along the normal, fm,
+// f0 the |E| beside it, fld the face field.
+template <class T>
+__device__ __forceinline__ double koren_flux(const Run3 &R, T em2, T em1, T e0, T ep1, T fm, T f0, T fld, T fac,
+                                             T inv_dr) {
+  const LocT<T> loc = lt_locT<T>(R, T(0.5) * (f0 + fm));
+  T mobility, diff_coeff;
+  lt_pairT<T>(R, C_MOB, loc, mobility, diff_coeff);
+  const T v_drift = -mobility * fld;
+  const T gradc = e0 - em1;
+  const bool neg = v_drift < T(0);
+  const T grad2 = neg ? ep1 - e0 : em1 - em2;
+  const T lim = koren_mlimT<T>(gradc, grad2), ff = fac * fld;
+  T out;
+  if (neg) {
+    out = v_drift * (e0 - lim);
+    if (out < ff) out = ff;
+  } else {
+    out = v_drift * (em1 + lim);
+    if (out > ff) out = ff;
+  }
+  return (double)(out - diff_coeff * gradc * inv_dr) / (double)dscale<T>();
+}
+
+// A thread owns the cells (i, j, k) and (i, j, k + 1) of the box: their low
+// faces (and, on 192 threads, one high face of the box) with the direction
+// known at compile time, six independent chains per thread. What bounds the
+// kernel is instruction issue and the latency of its FP64 chains, not HBM:
+// with faces dealt out flat (index divisions, one chain per thread) stage 1
+// took 1,621 us and stage 2 1,088 us at level 6.
+template <class T, int STAGE>
+__global__ void __launch_bounds__(NTH3, 3) k3d_stage(Run3 R, const __grid_constant__ Stage3 S, const int *ids) {
+  extern __shared__ double2 sm_d2[];
+  constexpr int nc = NC3, g = nc + 2, F = (nc + 1) * nc * nc;
+  double *sphi = reinterpret_cast<double *>(sm_d2);
+  T *se = reinterpret_cast<T *>(sphi + (STAGE == 2 ? S12 : 0)), *sf = se + S12, *sfx = sf + SLOT3;
   const int id = ids[blockIdx.x];
-  constexpr int nc = NC3, g = nc + 2;
-  const MG3<double> M{VAR(R, I_PHI), VAR(R, I_RHS), VAR(R, I_FLD), R.voltage};
-  const double dr = R.geo[4 * id + 3], inv_dr_sq = 1 / (dr * dr);
-  const double *phi = SL(M.phi, id), *rhs = SL(M.rhs, id);
   const int4 o = R.org[id];
-  for (int t = threadIdx.x; t < nc * nc * nc; t += NTH3) {
-    const int i = t % nc + 1, j = (t / nc) % nc + 1, k = t / (nc * nc) + 1, c = ix3(g, i, j, k);
-    F[didx(L, o.x + i - 1, o.y + j - 1, o.z + k - 1)] =
-        (float)(rhs[c] - lpl3_src(R, M, id, nc, phi, c, i, j, k, inv_dr_sq));
+  const DLv &L = S.L;
+  const int nx = 2 * L.nx2, tid = threadIdx.x;
+  const int i = tid & 7, j = (tid >> 3) & 7, k0 = (tid >> 6) * 2;
+  const T ds = dscale<T>();
+  const double inv64 = 1 / R.geo[4 * id + 3];
+  const T inv_dr = T(inv64);
+  const double dt = R.scal[S_DT];
+  const double *e = CC(R, I_ELEC, id), *p = CC(R, I_PION, id);
+  const int xf0 = i + (nc + 1) * (j + nc * k0), yf0 = i + nc * (j + (nc + 1) * k0), zf0 = i + nc * (j + nc * k0);
+  // the box's high face of this thread (tid < 192): direction bd, at (i, j)
+  const int bd = tid >> 6;
+  const int bq = bd == 0 ? nc + (nc + 1) * (i + nc * j) : bd == 1 ? i + nc * (nc + (nc + 1) * j) : i + nc * (j + nc * nc);
+  double fl[2][3], fb = 0;  // face fields
+  if (STAGE == 1) {
+    // densities saved whole; n_e, |E| and the second ghost layer staged
+    double *eo = CC(R, I_ELEC_OLD, id), *po = CC(R, I_PION_OLD, id);
+    const double *f = CC(R, I_FLD, id), *phi = CC(R, I_PHI, id);
+    double ve[4], vp[4], vf[4], vh[4], vn[2];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int c = tid + m * NTH3;
+      if (c < SLOT3) {
+        ve[m] = e[c];
+        vf[m] = f[c];
+        vp[m] = p[c];
+        vh[m] = phi[c];
+      }
+    }
+    const int *nb = R.nbr + 6 * id;
+    int dst[2];
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      const int t = tid + m * NTH3;
+      if (t < 6 * nc * nc) {
+        const int s = t >> 6, a = (t & 7) + 1, b = ((t >> 3) & 7) + 1, d = s >> 1;
+        const bool hi = s & 1;
+        const int n = nb[s];
+        // a3_gc2_box: the neighbour's second cell from the shared side, or the own one
+        const int q = n > 0 ? (hi ? 2 : nc - 1) : (hi ? nc - 1 : 2), w = hi ? nc + 2 : -1;
+        const double *x = n > 0 ? CC(R, I_ELEC, n) : e;
+        vn[m] = x[d == 0 ? ix3(g, q, a, b) : d == 1 ? ix3(g, a, q, b) : ix3(g, a, b, q)];
+        dst[m] = d == 0 ? ix12(w, a, b) : d == 1 ? ix12(a, w, b) : ix12(a, b, w);
+      }
+    }
+    const double *fx = FC(R, 0, F_FLD, id), *fy = FC(R, 1, F_FLD, id), *fz = FC(R, 2, F_FLD, id);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      fl[u][0] = fx[xf0 + u * (nc + 1) * nc];
+      fl[u][1] = fy[yf0 + u * (nc + 1) * nc];
+      fl[u][2] = fz[zf0 + u * nc * nc];
+    }
+    if (tid < 192) fb = (bd == 0 ? fx : bd == 1 ? fy : fz)[bq];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      const int c = tid + m * NTH3;
+      if (c < SLOT3) {
+        eo[c] = ve[m];
+        po[c] = vp[m];
+        const int ci = c % g, cj = (c / g) % g, ck = c / (g * g);
+        se[ix12(ci, cj, ck)] = T(ve[m]) * ds;
+        sf[c] = T(vf[m]);
+        if (ci >= 1 && ci <= nc && cj >= 1 && cj <= nc && ck >= 1 && ck <= nc)
+          S.P[didx(L, o.x + ci - 1, o.y + cj - 1, o.z + ck - 1)] = vh[m];
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+      if (tid + m * NTH3 < 6 * nc * nc) se[dst[m]] = T(vn[m]) * ds;
+  } else {
+    // n_e with two layers and the potential around the box from the dense
+    // arrays; beyond a wall n_e mirrors (a3_gc_neumann, a3_gc2_neumann)
+    const double v2 = 2 * R.voltage;
+#pragma unroll
+    for (int m = 0; m < 7; m++) {
+      const int c = tid + m * NTH3;
+      if (c >= S12) continue;
+      const int ci = c % G12 - 1, cj = (c / G12) % G12 - 1, ck = c / (G12 * G12) - 1;
+      const int out = (ci < 1 || ci > nc) + (cj < 1 || cj > nc) + (ck < 1 || ck > nc);
+      if (out > 2) continue;
+      const int x = o.x + ci - 1, y = o.y + cj - 1, z = o.z + ck - 1;
+      if (out <= 1) {
+        const int mx = x < 0 ? -1 - x : (x >= nx ? 2 * nx - 1 - x : x);
+        const int my = y < 0 ? -1 - y : (y >= L.ny ? 2 * L.ny - 1 - y : y);
+        const int mz = z < 0 ? -1 - z : (z >= L.nz ? 2 * L.nz - 1 - z : z);
+        se[c] = T(S.e1[nat(L, mx, my, mz)]) * ds;
+      }
+      sphi[c] = phi_at(L, S.P, x, y, z, v2);
+    }
+    __syncthreads();
+    // |E| of the cells and of the facing cells of the neighbours (a wall's
+    // ghost mirrors the cell); faces at multiples of nc are box-edge faces
+    auto fields = [&](int ci, int cj, int ck, double lo[3]) {
+      const int c = ix12(ci, cj, ck);
+      const int pos[3] = {ci, cj, ck}, st[3] = {1, G12, G12 * G12};
+      const double v = sphi[c];
+      double s3[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const int m = pos[d] & (nc - 1);  // 1: low face, 0: high face on the box edge
+        lo[d] = face_of(sphi[c - st[d]] - v, inv64, m == 1, 1.0, 2.0);
+        s3[d] = lo[d] + face_of(v - sphi[c + st[d]], inv64, m == 0, 1.0, 2.0);
+      }
+      return T(0.5 * sqrt(s3[0] * s3[0] + s3[1] * s3[1] + s3[2] * s3[2]));
+    };
+#pragma unroll
+    for (int u = 0; u < 2; u++) sf[ix3(g, i + 1, j + 1, k0 + u + 1)] = fields(i + 1, j + 1, k0 + u + 1, fl[u]);
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      const int t = tid + m * NTH3;
+      if (t >= 6 * nc * nc) continue;
+      const int s = t >> 6, a = (t & 7) + 1, b = ((t >> 3) & 7) + 1, d = s >> 1;
+      const bool hi = s & 1;
+      const int org = d == 0 ? o.x : d == 1 ? o.y : o.z, end = d == 0 ? nx : d == 1 ? L.ny : L.nz;
+      const bool wall = hi ? org + nc >= end : org == 0;
+      const int q = hi ? nc + 1 : 0, w = wall ? (hi ? nc : 1) : q;
+      double lo[3];
+      const T v = d == 0 ? fields(w, a, b, lo) : d == 1 ? fields(a, w, b, lo) : fields(a, b, w, lo);
+      sf[d == 0 ? ix3(g, q, a, b) : d == 1 ? ix3(g, a, q, b) : ix3(g, a, b, q)] = v;
+    }
+    if (tid < 192) {
+      const int c = bd == 0 ? ix12(nc + 1, i + 1, j + 1) : bd == 1 ? ix12(i + 1, nc + 1, j + 1) : ix12(i + 1, j + 1, nc + 1);
+      fb = face_of(sphi[c - (bd == 0 ? 1 : bd == 1 ? G12 : G12 * G12)] - sphi[c], inv64, true, 1.0, 2.0);
+    }
+  }
+  __syncthreads();
+  const T fac = T(-0.8 * UC_EPS0 / (UC_ELEM_CHARGE * dt)) * ds;
+  double *ex = FC(R, 0, F_ELEC, id), *ey = FC(R, 1, F_ELEC, id), *ez = FC(R, 2, F_ELEC, id);
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int c = ix12(i + 1, j + 1, k0 + u + 1), f = ix3(g, i + 1, j + 1, k0 + u + 1);
+    const T e0 = se[c], f0 = sf[f];
+    const int q[3] = {xf0 + u * (nc + 1) * nc, yf0 + u * (nc + 1) * nc, zf0 + u * nc * nc};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const int st = d == 0 ? 1 : d == 1 ? G12 : G12 * G12, gt = d == 0 ? 1 : d == 1 ? g : g * g;
+      const double v = koren_flux<T>(R, se[c - 2 * st], se[c - st], e0, se[c + st], sf[f - gt], f0, T(fl[u][d]), fac, inv_dr);
+      if (STAGE == 2) (d == 0 ? ex : d == 1 ? ey : ez)[q[d]] = v;
+      sfx[d * F + q[d]] = T(v);
+    }
+  }
+  if (tid < 192) {
+    const int c = bd == 0 ? ix12(nc + 1, i + 1, j + 1) : bd == 1 ? ix12(i + 1, nc + 1, j + 1) : ix12(i + 1, j + 1, nc + 1);
+    const int f = bd == 0 ? ix3(g, nc + 1, i + 1, j + 1) : bd == 1 ? ix3(g, i + 1, nc + 1, j + 1) : ix3(g, i + 1, j + 1, nc + 1);
+    const int st = bd == 0 ? 1 : bd == 1 ? G12 : G12 * G12, gt = bd == 0 ? 1 : bd == 1 ? g : g * g;
+    const double v = koren_flux<T>(R, se[c - 2 * st], se[c - st], se[c], se[c + st], sf[f - gt], sf[f], T(fb), fac, inv_dr);
+    if (STAGE == 2) (bd == 0 ? ex : bd == 1 ? ey : ez)[bq] = v;
+    sfx[bd * F + bq] = T(v);
+  }
+  __syncthreads();
+  // update_solution (src/streamer_3d.f90:566-615), as k3_update
+  const T tdt = T(dt);
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int x = o.x + i, y = o.y + j, z = o.z + k0 + u, c = ix3(g, i + 1, j + 1, k0 + u + 1);
+    const size_t n = nat(L, x, y, z);
+    const double e_in = STAGE == 1 ? e[c] : S.e1[n], p_in = STAGE == 1 ? p[c] : S.p1[n];
+    const LocT<T> loc = lt_locT<T>(R, sf[c]);
+    T alpha, eta;
+    lt_pairT<T>(R, C_ALPHA, loc, alpha, eta);
+    const T *xf = sfx + xf0 + u * (nc + 1) * nc, *yf = sfx + F + yf0 + u * (nc + 1) * nc, *zf = sfx + 2 * F + zf0 + u * nc * nc;
+    const T x0 = xf[0], x1 = xf[1], y0 = yf[0], y1 = yf[nc], z0 = zf[0], z1 = zf[nc * nc];
+    T dflux[3];
+    dflux[0] = x0 + x1;
+    dflux[1] = y0 + y1;
+    dflux[2] = z0 + z1;
+    const T src = T(0.5) * norm2_3T<T>(dflux) * (alpha - eta);
+    T sflux = x0 - x1;
+    sflux = sflux + y0;
+    sflux = sflux - y1;
+    sflux = sflux + z0;
+    sflux = sflux - z1;
+    sflux = sflux * inv_dr;
+    const double ev = e_in + (double)((src + sflux) * tdt);
+    const double pv = p_in + (double)(src * tdt);
+    if (STAGE == 1) {
+      S.e1[n] = ev;
+      S.F[didx(L, x, y, z)] = space_charge(ev, pv);
+    } else {
+      S.e2[n] = ev;
+    }
+    S.p1[n] = pv;
   }
 }
-__global__ void __launch_bounds__(NTH3) k3d_mx_acc(Run3 R, const __grid_constant__ DAll D, const int *ids,
-                                                   const float *P) {
+
+// The end of the transport on the leaves: average_dens
+// (src/streamer_3d.f90:557-563) on whole slots, the ghost cells of the
+// updated densities from their sources (a3_gc_tree with Neumann sides), and
+// the space charge of the second solve. Edge and corner entries are never
+// updated: their average is the saved value.
+__global__ void __launch_bounds__(NTH3) k3d_final(Run3 R, const __grid_constant__ Stage3 S, const int *ids) {
   const int id = ids[blockIdx.x];
-  const int nc = R.nc[id], g = nc + 2, n = nc * nc * nc;
+  constexpr int nc = NC3, g = nc + 2;
   const int4 o = R.org[id];
-  const DLv &L = D.lv[o.w];
-  double *phi = CC(R, I_PHI, id);
-  for (int t = threadIdx.x; t < n; t += NTH3) {
-    const int i = t % nc + 1, j = (t / nc) % nc + 1, k = t / (nc * nc) + 1;
-    const int c = ix3(g, i, j, k);
-    const double v = phi[c] + (double)dval(L, P + L.off, o.x + i - 1, o.y + j - 1, o.z + k - 1);
-    phi[c] = v;
-    push_side_ghosts(R, I_PHI, id, nc, i, j, k, v, 1);
+  const DLv &L = S.L;
+  double *e = CC(R, I_ELEC, id), *p = CC(R, I_PION, id), *rhs = CC(R, I_RHS, id);
+  const double *eo = CC(R, I_ELEC_OLD, id), *po = CC(R, I_PION_OLD, id);
+  for (int c = threadIdx.x; c < SLOT3; c += NTH3) {
+    const int i = c % g, j = (c / g) % g, k = c / (g * g);
+    const int in = (i >= 1 && i <= nc) + (j >= 1 && j <= nc) + (k >= 1 && k <= nc);
+    const int x = o.x + i - 1, y = o.y + j - 1, z = o.z + k - 1;
+    const double a = eo[c], b = po[c];
+    double ev = a, pv = b;
+    if (in >= 2) {
+      const size_t n = nat(L, min(max(x, 0), 2 * L.nx2 - 1), min(max(y, 0), L.ny - 1), min(max(z, 0), L.nz - 1));
+      ev = S.e2[n];
+      pv = S.p1[n];
+    }
+    ev = 0.5 * (ev + a);
+    pv = 0.5 * (pv + b);
+    const double v = space_charge(ev, pv);
+    e[c] = ev;
+    p[c] = pv;
+    rhs[c] = v;
+    if (in == 3) S.F[didx(L, x, y, z)] = v;
+  }
+}
+
+// a3_restrict_box (afivo/src/m_aX_restrict.f90:67-142) of the dense leaf
+// densities into the parents' slots, one block per parent
+__global__ void __launch_bounds__(NTH3) k3d_restrict_dens(Run3 R, const __grid_constant__ Stage3 S, const int *ids) {
+  const int id = ids[blockIdx.x];
+  constexpr int nc = NC3;
+  const int4 o = R.org[id];
+  const DLv &L = S.L;
+  const size_t nx = 2 * L.nx2, pl = nx * L.ny;
+  for (int t = threadIdx.x; t < 2 * nc * nc * nc; t += NTH3) {
+    const int w = t / (nc * nc * nc), u = t % (nc * nc * nc), i = u % nc, j = (u / nc) % nc, k = u / (nc * nc);
+    const double *c = (w ? S.p1 : S.e2) + nat(L, 2 * (o.x + i), 2 * (o.y + j), 2 * (o.z + k));
+    double s = c[0];
+    s = s + c[1];
+    s = s + c[nx];
+    s = s + c[nx + 1];
+    s = s + c[pl];
+    s = s + c[pl + 1];
+    s = s + c[pl + nx];
+    s = s + c[pl + nx + 1];
+    CC(R, w ? I_PION : I_ELEC, id)[ix3(nc + 2, i + 1, j + 1, k + 1)] = 0.125 * s;
+  }
+}
+// The restriction of both densities from level top down to the coarsest,
+// all levels' few boxes in one block.
+__global__ void __launch_bounds__(1024) k3_restrict_low(Run3 R, int top) {
+  for (int l = top; l > R.lo; l--) {
+    const Lv v = lv_of(R, l);
+    const int hnc = v.nc >> 1, nh = hnc * hnc * hnc;
+    for (int t = threadIdx.x; t < 2 * nh * v.n; t += 1024) {
+      const int id = v.first + t / (2 * nh), u = t % (2 * nh);
+      restrict_item(R, id, v.nc, u % nh, u < nh ? I_ELEC : I_PION);
+    }
+    __syncthreads();
   }
 }
