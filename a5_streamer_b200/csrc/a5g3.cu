@@ -1864,6 +1864,7 @@ static void setup_dense(a5g3_ctx *c) {
     C.lv[q] = D.lv[q];
     C.goff[q] = D.lv[q].off;
     C.lv[q].off = C.cells;
+    C.lv[q].m_nxv = a5g3_ctx::magic(D.lv[q].nx2 / 2);
     C.coff[q] = D.coff[q];
     C.ncorr[q] = D.ncorr[q];
     C.cells += 2 * D.lv[q].half;

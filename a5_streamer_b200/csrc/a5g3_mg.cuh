@@ -54,33 +54,47 @@ struct alignas(sizeof(T) * V) Vec {
 template <class T, int V>
 __device__ __forceinline__ Vec<T, V> ldv(const T *p) { return *reinterpret_cast<const Vec<T, V> *>(p); }
 
-// The six neighbours of V consecutive cells of one colour in row (y, z),
-// from the other colour's array a (own: their own values, which the walls
-// mirror: Neumann on x and y, -own at low z, 2 V - own at high z,
-// src/streamer_3d.f90:693-715). b: index of the first cell; q: x parity of
-// the row's cells of this colour.
+// V consecutive cells of one colour: index of the first within the colour,
+// parity of the row's y + z, and which of the group's sides are walls.
+struct Group {
+  int b;
+  unsigned fl;
+};
+enum { GF_ODD = 1, GF_XL = 2, GF_XH = 4, GF_YL = 8, GF_YH = 16, GF_ZL = 32, GF_ZH = 64 };
+template <int V>
+__device__ __forceinline__ Group group_of(const DLv &L, int xv, int r) {
+  const int z = fastdiv(r, L.m_ny), y = r - z * L.ny;
+  return Group{r * L.nx2 + xv, (unsigned)((y + z) & 1) | (xv == 0 ? GF_XL : 0) | (xv + V == L.nx2 ? GF_XH : 0) |
+                                   (y == 0 ? GF_YL : 0) | (y == L.ny - 1 ? GF_YH : 0) | (z == 0 ? GF_ZL : 0) |
+                                   (z == L.nz - 1 ? GF_ZH : 0)};
+}
+
+// The six neighbours of group g of colour c from the arrays P (both
+// colours). Beyond a wall the group's own values are mirrored (Neumann on x
+// and y, -own at low z, 2 V - own at high z, src/streamer_3d.f90:693-715):
+// the address is selected, not the branch, so the loads go out together.
 template <class T, int V>
 struct Nbr {
   Vec<T, V> xm, xp, ym, yp, zm, zp;
 };
 template <class T, int V>
-__device__ __forceinline__ Nbr<T, V> neighbours(const DLv &L, const T *a, const Vec<T, V> &own, int b, int xv, int y,
-                                                int z, int q, T v2) {
+__device__ __forceinline__ Nbr<T, V> neighbours(const DLv &L, const T *P, int c, const Group &g, T v2) {
   Nbr<T, V> n;
-  const Vec<T, V> m = ldv<T, V>(a + b);
+  const T *own = P + c * L.half + g.b, *a = P + (1 - c) * L.half + g.b;
   const int pl = L.nx2 * L.ny;
-  const bool wl = q == 0 && xv == 0, wh = q == 1 && xv + V == L.nx2;
-  const T e = (wl || wh) ? (wl ? own.v[0] : own.v[V - 1]) : (q ? a[b + V] : a[b - 1]);
-  n.ym = y > 0 ? ldv<T, V>(a + b - L.nx2) : own;
-  n.yp = y < L.ny - 1 ? ldv<T, V>(a + b + L.nx2) : own;
-  if (z > 0) n.zm = ldv<T, V>(a + b - pl);
-  if (z < L.nz - 1) n.zp = ldv<T, V>(a + b + pl);
+  const bool q = ((g.fl ^ c) & GF_ODD) != 0;  // x parity of the group's cells
+  const Vec<T, V> m = ldv<T, V>(a);
+  const T e = *(q ? ((g.fl & GF_XH) ? own + V - 1 : a + V) : ((g.fl & GF_XL) ? own : a - 1));
+  n.ym = ldv<T, V>((g.fl & GF_YL) ? own : a - L.nx2);
+  n.yp = ldv<T, V>((g.fl & GF_YH) ? own : a + L.nx2);
+  n.zm = ldv<T, V>((g.fl & GF_ZL) ? own : a - pl);
+  n.zp = ldv<T, V>((g.fl & GF_ZH) ? own : a + pl);
 #pragma unroll
   for (int k = 0; k < V; k++) {
     n.xm.v[k] = q ? m.v[k] : (k == 0 ? e : m.v[k > 0 ? k - 1 : 0]);
     n.xp.v[k] = q ? (k == V - 1 ? e : m.v[k < V - 1 ? k + 1 : 0]) : m.v[k];
-    if (z == 0) n.zm.v[k] = -own.v[k];
-    if (z == L.nz - 1) n.zp.v[k] = v2 - own.v[k];
+    if (g.fl & GF_ZL) n.zm.v[k] = -n.zm.v[k];
+    if (g.fl & GF_ZH) n.zp.v[k] = v2 - n.zp.v[k];
   }
   return n;
 }
@@ -106,39 +120,34 @@ __device__ __forceinline__ T gsrb_of(const Nbr<T, V> &n, int k, T dx2f) {
   return sixth * (s - dx2f);
 }
 
-// V cells of one half-sweep of colour c (colour 0 on odd half-sweeps: the
+// One group of a half-sweep of colour c (colour 0 on odd half-sweeps: the
 // reference's cells with i + j + k + it even, 1-based). FIRST: the level's
 // first visit in a cycle, F = lpl(O) + F before it is used; O holds P's
 // values from before the visit, so the second colour's operator does not see
 // the first colour's update.
 template <class T, int V, bool FIRST>
-__device__ __forceinline__ void sweep_cells(const DLv &L, T *P, T *F, const T *O, int c, int xv, int r, T v2) {
-  const int z = fastdiv(r, L.m_ny), y = r - z * L.ny;
-  const int q = (c + y + z) & 1, b = r * L.nx2 + xv;
-  T *own = P + c * L.half;
-  const T *oth = P + (1 - c) * L.half;
-  const bool wall = y == 0 || y == L.ny - 1 || z == 0 || z == L.nz - 1 || xv == 0 || xv + V == L.nx2;
-  Vec<T, V> o{};
-  if (wall || FIRST) o = ldv<T, V>(own + b);
-  Vec<T, V> f = ldv<T, V>(F + c * L.half + b);
-  const Nbr<T, V> n = neighbours<T, V>(L, oth, o, b, xv, y, z, q, v2);
+__device__ __forceinline__ void sweep_group(const DLv &L, T *P, T *F, const T *O, int c, const Group &g, T v2) {
+  T *own = P + c * L.half + g.b, *fp = F + c * L.half + g.b;
+  Vec<T, V> f = ldv<T, V>(fp);
+  const Nbr<T, V> n = neighbours<T, V>(L, P, c, g, v2);
   if (FIRST) {
     const T inv = T(L.inv_dx2);
+    const Vec<T, V> o = ldv<T, V>(own);
     if (c == 0) {
 #pragma unroll
       for (int k = 0; k < V; k++) f.v[k] = lpl_of<T, V>(n, k, o.v[k], inv) + f.v[k];
     } else {
-      const Nbr<T, V> n0 = neighbours<T, V>(L, O + (1 - c) * L.half, o, b, xv, y, z, q, v2);
+      const Nbr<T, V> n0 = neighbours<T, V>(L, O, c, g, v2);
 #pragma unroll
       for (int k = 0; k < V; k++) f.v[k] = lpl_of<T, V>(n0, k, o.v[k], inv) + f.v[k];
     }
-    *reinterpret_cast<Vec<T, V> *>(F + c * L.half + b) = f;
+    *reinterpret_cast<Vec<T, V> *>(fp) = f;
   }
   const T dx2 = T(L.dx2);
   Vec<T, V> w;
 #pragma unroll
   for (int k = 0; k < V; k++) w.v[k] = gsrb_of<T, V>(n, k, dx2 * f.v[k]);
-  *reinterpret_cast<Vec<T, V> *>(own + b) = w;
+  *reinterpret_cast<Vec<T, V> *>(own) = w;
 }
 
 template <class T, int V, bool FIRST>
@@ -146,7 +155,7 @@ __global__ void __launch_bounds__(256) k3d_sweep(DLv L, T *P, T *F, const T *O, 
   const unsigned t = blockIdx.x * 256u + threadIdx.x;
   if (t >= (unsigned)(L.half / V)) return;
   const int nv = L.nx2 / V, r = fastdiv(t, L.m_nxv);
-  sweep_cells<T, V, FIRST>(L, P, F, O, c, (t - r * nv) * V, r, v2);
+  sweep_group<T, V, FIRST>(L, P, F, O, c, group_of<V>(L, (t - r * nv) * V, r), v2);
 }
 
 // Value of cell (x, y, z) of a level
@@ -292,6 +301,31 @@ __device__ __forceinline__ void correct_cell(const DLv &L, const DLv &C, T *P, c
     *p = *p + T(0.25) * s;
   }
 }
+// The same for one fine cell (x, y, z), where there are more threads than
+// coarse cells to spread them over; the first cell of each block of eight
+// keeps the correction.
+template <class T>
+__device__ __forceinline__ void correct_fine(const DLv &L, const DLv &C, T *P, const T *Pc, const T *Oc, T *corr,
+                                             unsigned t, T v2) {
+  const int c = t >= (unsigned)L.half, b = (int)t - c * L.half, r = fastdiv(b, L.m_nx), z = fastdiv(r, L.m_ny),
+            y = r - z * L.ny, x = 2 * (b - r * L.nx2) + ((c + y + z) & 1);
+  const int X = x >> 1, Y = y >> 1, Z = z >> 1, nx = 2 * C.nx2;
+  const int X2 = X + (x & 1 ? 1 : -1), Y2 = Y + (y & 1 ? 1 : -1), Z2 = Z + (z & 1 ? 1 : -1);
+  const int i0 = didx(C, X, Y, Z);
+  const T p0 = Pc[i0], o0 = Oc[i0], c1 = p0 - o0;
+  const bool wx = X2 < 0 || X2 >= nx, wy = Y2 < 0 || Y2 >= C.ny, zl = Z2 < 0, zh = Z2 >= C.nz;
+  const int ix = wx ? i0 : didx(C, X2, Y, Z), iy = wy ? i0 : didx(C, X, Y2, Z), iz = (zl || zh) ? i0 : didx(C, X, Y, Z2);
+  T pz = Pc[iz], oz = Oc[iz];
+  if (zl) pz = -pz, oz = -oz;
+  if (zh) pz = v2 - pz, oz = v2 - oz;
+  const T cz = pz - oz;
+  T s = c1 + (Pc[ix] - Oc[ix]);
+  s = s + (Pc[iy] - Oc[iy]);
+  s = s + cz;
+  P[t] = P[t] + T(0.25) * s;
+  if (corr && !(x & 1) && !(y & 1) && !(z & 1)) corr[i0] = c1;
+  if (corr && zh && !(x & 1) && !(y & 1)) corr[2 * C.half + Y * nx + X] = cz;
+}
 template <class T>
 __device__ __forceinline__ void correct_at(const DLv &L, const DLv &C, T *P, const T *Pc, const T *Oc, T *corr,
                                            unsigned t, T v2) {
@@ -310,11 +344,9 @@ __global__ void __launch_bounds__(128) k3d_correct(DLv L, DLv C, T *P, const T *
 // side in the FMG's set-up)
 template <class T>
 __device__ __forceinline__ void add_lpl_at(const DLv &L, const T *P, T *F, unsigned t, T v2) {
-  const int c = t >= (unsigned)L.half, b = (int)t - c * L.half;
-  const int r = fastdiv(b, L.m_nx), xv = b - r * L.nx2, z = fastdiv(r, L.m_ny), y = r - z * L.ny;
-  const Vec<T, 1> o{{P[t]}};
-  const Nbr<T, 1> n = neighbours<T, 1>(L, P + (1 - c) * L.half, o, b, xv, y, z, (c + y + z) & 1, v2);
-  F[t] = lpl_of<T, 1>(n, 0, o.v[0], T(L.inv_dx2)) + F[t];
+  const int c = t >= (unsigned)L.half, b = (int)t - c * L.half, r = fastdiv(b, L.m_nx);
+  const Nbr<T, 1> n = neighbours<T, 1>(L, P, c, group_of<1>(L, b - r * L.nx2, r), v2);
+  F[t] = lpl_of<T, 1>(n, 0, P[t], T(L.inv_dx2)) + F[t];
 }
 template <class T>
 __global__ void __launch_bounds__(128) k3d_add_lpl(DLv L, const T *P, T *F, T v2) {
@@ -328,7 +360,11 @@ __global__ void __launch_bounds__(128) k3d_add_lpl(DLv L, const T *P, T *F, T v2
 // of the level above. What bounds it is the chain of some 60 dependent
 // phases per V-cycle, each a shared-memory round trip and a barrier, so the
 // levels of at most 64 cells per colour run in one warp behind warp barriers
-// while the other warps wait once.
+// while the other warps wait once, a level visit keeps its addresses in
+// registers, and the phases are out of line: inlined copies overran the
+// instruction cache. Per launch on the level-4 cube 64 us with inlined
+// phases and addresses formed in every sweep, 41 so (FP64); 38 -> 22 in the
+// mixed form on 2 x 1 x 3 base boxes.
 constexpr int DCOARSE = 4096, NTHD = 512, DWARP = 64, MAXLV3 = 16;
 struct DCoarse {
   DLv lv[8];       // the levels, coarsest first; off: first cell in shared memory
@@ -356,32 +392,135 @@ struct Team {
   }
 };
 
-template <class T, bool FIRST>
-__device__ __forceinline__ void cd_sweep(const DLv &L, T *P, T *F, const T *O, int c, T v2, const Team &g) {
-  for (int t = g.tid; t < L.half; t += g.n) {
-    const int r = fastdiv(t, L.m_nx);
-    sweep_cells<T, 1, FIRST>(L, P, F, O, c, t - r * L.nx2, r, v2);
-  }
-  g.sync();
+// The half-sweeps of a level visit. A thread's groups (at most K of each
+// colour, V cells each) keep their neighbours' places, their wall flags and
+// dx^2 F in registers through the visit: with one block the phases are bound
+// by instruction issue and latency, not by shared memory.
+struct Places {
+  int own, m, e, ym, yp, zm, zp;  // as neighbours(), from the start of the level
+  unsigned fl;
+};
+template <int V>
+__device__ __forceinline__ Places places_of(const DLv &L, int c, const Group &g) {
+  const int own = c * L.half + g.b, a = (1 - c) * L.half + g.b, pl = L.nx2 * L.ny;
+  const bool q = ((g.fl ^ c) & GF_ODD) != 0;
+  Places w;
+  w.own = own;
+  w.m = a;
+  w.e = q ? ((g.fl & GF_XH) ? own + V - 1 : a + V) : ((g.fl & GF_XL) ? own : a - 1);
+  w.ym = (g.fl & GF_YL) ? own : a - L.nx2;
+  w.yp = (g.fl & GF_YH) ? own : a + L.nx2;
+  w.zm = (g.fl & GF_ZL) ? own : a - pl;
+  w.zp = (g.fl & GF_ZH) ? own : a + pl;
+  w.fl = (g.fl & ~(unsigned)GF_ODD) | (q ? GF_ODD : 0);
+  return w;
 }
-template <class T>
-__device__ __forceinline__ void cd_gsrb(const DLv &L, T *P, T *F, const T *O, int cycles, bool first, T v2,
-                                        const Team &g) {
-  int it = 0;
-  if (first) {
-    cd_sweep<T, true>(L, P, F, O, 0, v2, g);
-    cd_sweep<T, true>(L, P, F, O, 1, v2, g);
-    it = 2;
+template <class T, int V>
+__device__ __forceinline__ Nbr<T, V> neighbours_at(const T *P, const Places &w, T v2) {
+  Nbr<T, V> n;
+  const Vec<T, V> m = ldv<T, V>(P + w.m);
+  const T e = P[w.e];
+  n.ym = ldv<T, V>(P + w.ym);
+  n.yp = ldv<T, V>(P + w.yp);
+  n.zm = ldv<T, V>(P + w.zm);
+  n.zp = ldv<T, V>(P + w.zp);
+  const bool q = w.fl & GF_ODD;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    n.xm.v[k] = q ? m.v[k] : (k == 0 ? e : m.v[k > 0 ? k - 1 : 0]);
+    n.xp.v[k] = q ? (k == V - 1 ? e : m.v[k < V - 1 ? k + 1 : 0]) : m.v[k];
+    if (w.fl & GF_ZL) n.zm.v[k] = -n.zm.v[k];
+    if (w.fl & GF_ZH) n.zp.v[k] = v2 - n.zp.v[k];
   }
+  return n;
+}
+template <class T, int V, int K>
+__device__ __forceinline__ void cd_visit(const DLv &L, T *P, T *F, int cycles, bool first, T v2, const Team &g) {
+  const int n = L.half / V, nv = L.nx2 / V;
+  const T dx2 = T(L.dx2), inv = T(L.inv_dx2);
+  Places w[2][K];
+  Vec<T, V> df[2][K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int t = g.tid + k * g.n;
+    if (t < n) {
+      const int r = fastdiv(t, V == 1 ? L.m_nx : L.m_nxv);
+      const Group gr = group_of<V>(L, (t - r * nv) * V, r);
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        w[c][k] = places_of<V>(L, c, gr);
+        Vec<T, V> f = ldv<T, V>(F + w[c][k].own);
+        if (first) {  // F = lpl(P) + F, before any cell of P changes
+          const Nbr<T, V> nb = neighbours_at<T, V>(P, w[c][k], v2);
+          const Vec<T, V> o = ldv<T, V>(P + w[c][k].own);
+#pragma unroll
+          for (int v = 0; v < V; v++) f.v[v] = lpl_of<T, V>(nb, v, o.v[v], inv) + f.v[v];
+          *reinterpret_cast<Vec<T, V> *>(F + w[c][k].own) = f;
+        }
+#pragma unroll
+        for (int v = 0; v < V; v++) df[c][k].v[v] = dx2 * f.v[v];
+      }
+    }
+  }
+  if (first) g.sync();
 #pragma unroll 1
-  for (; it < 2 * cycles; it++) cd_sweep<T, false>(L, P, F, O, it & 1, v2, g);
+  for (int it = 0; it < cycles; it++) {
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        if (g.tid + k * g.n < n) {
+          const Nbr<T, V> nb = neighbours_at<T, V>(P, w[c][k], v2);
+          Vec<T, V> o;
+#pragma unroll
+          for (int v = 0; v < V; v++) o.v[v] = gsrb_of<T, V>(nb, v, df[c][k].v[v]);
+          *reinterpret_cast<Vec<T, V> *>(P + w[c][k].own) = o;
+        }
+      }
+      g.sync();
+    }
+  }
+}
+// V = 2 where rows allow it. The block form takes at most DCOARSE / 2 cells
+// per colour, the warp form DWARP.
+// Out of line: its copies would not fit the instruction cache together.
+template <class T>
+__device__ __noinline__ void cd_gsrb(const DLv &L, T *P, T *F, int cycles, bool first, T v2, const Team &g) {
+  if (g.warp) {
+    if (L.half <= 32) cd_visit<T, 1, 1>(L, P, F, cycles, first, v2, g);
+    else cd_visit<T, 1, DWARP / 32>(L, P, F, cycles, first, v2, g);
+  } else if (L.nx2 & 1) {
+    // (rows of odd length: coarse levels of odd base grids only)
+    if (first) {
+      for (int t = g.tid; t < 2 * L.half; t += g.n) add_lpl_at<T>(L, P, F, t, v2);
+      g.sync();
+    }
+    for (int it = 0; it < 2 * cycles; it++) {
+      for (int t = g.tid; t < L.half; t += g.n) {
+        const int r = fastdiv(t, L.m_nx);
+        sweep_group<T, 1, false>(L, P, F, P, it & 1, group_of<1>(L, t - r * L.nx2, r), v2);
+      }
+      g.sync();
+    }
+  } else {
+    cd_visit<T, 2, DCOARSE / 4 / NTHD>(L, P, F, cycles, first, v2, g);
+  }
+}
+
+template <class T>
+__device__ __noinline__ void cd_correct(const DLv &L, const DLv &C, T *P, const T *Pc, const T *Oc, T *cs, T v2) {
+  if (2 * L.half <= 2 * NTHD) {
+    for (int t = threadIdx.x; t < 2 * L.half; t += NTHD) correct_fine<T>(L, C, P, Pc, Oc, cs, t, v2);
+  } else {
+    for (int t = threadIdx.x; t < 2 * C.half; t += NTHD) correct_at<T>(L, C, P, Pc, Oc, cs, t, v2);
+  }
 }
 
 // A V-cycle over levels 0..q (mg3_fas_vcycle, :208-255); first: level q has
 // just been reached by the restriction. k: which of a level's kept
 // corrections this cycle's are (k + q - l).
 template <class T>
-__device__ void cd_vcycle(const DCoarse &D, T *P, T *F, T *O, int q, bool first, T *corr, int k, T v2) {
+__device__ __noinline__ void cd_vcycle(const DCoarse &D, T *P, T *F, T *O, int q, bool first, T *corr, int k, T v2) {
   Team g{(int)threadIdx.x, NTHD, false};
   int l = q;
   bool fst = first;
@@ -390,7 +529,7 @@ __device__ void cd_vcycle(const DCoarse &D, T *P, T *F, T *O, int q, bool first,
   for (; l >= 1; l--) {
     if (l < D.nwarp) break;
     const DLv &L = D.lv[l], &C = D.lv[l - 1];
-    cd_gsrb<T>(L, P + L.off, F + L.off, O + L.off, D.down, fst, v2, g);
+    cd_gsrb<T>(L, P + L.off, F + L.off, D.down, fst, v2, g);
     for (int t = g.tid; t < 2 * C.half; t += g.n)
       restrict_at<T, RS_RESID>(L, C, P + L.off, F + L.off, P + C.off, F + C.off, O + C.off, t, v2);
     g.sync();
@@ -402,35 +541,35 @@ __device__ void cd_vcycle(const DCoarse &D, T *P, T *F, T *O, int q, bool first,
       const Team w{(int)threadIdx.x, 32, true};
       for (; l >= 1; l--) {
         const DLv &L = D.lv[l], &C = D.lv[l - 1];
-        cd_gsrb<T>(L, P + L.off, F + L.off, O + L.off, D.down, fst, v2, w);
+        cd_gsrb<T>(L, P + L.off, F + L.off, D.down, fst, v2, w);
         for (int t = w.tid; t < 2 * C.half; t += 32)
           restrict_at<T, RS_RESID>(L, C, P + L.off, F + L.off, P + C.off, F + C.off, O + C.off, t, v2);
         w.sync();
         fst = true;
       }
-      cd_gsrb<T>(D.lv[0], P + D.lv[0].off, F + D.lv[0].off, O + D.lv[0].off, D.base, fst, v2, w);
+      cd_gsrb<T>(D.lv[0], P + D.lv[0].off, F + D.lv[0].off, D.base, fst, v2, w);
       for (l = 1; l <= lw; l++) {
         const DLv &L = D.lv[l], &C = D.lv[l - 1];
         const int kk = k + q - l;
         T *cs = corr && kk + 1 < D.ncorr[l - 1] ? corr + D.coff[l - 1] + (kk + 1) * corr_len(C) : nullptr;
-        for (int t = w.tid; t < 2 * C.half; t += 32)
-          correct_at<T>(L, C, P + L.off, P + C.off, O + C.off, cs, t, v2);
+        for (int t = w.tid; t < 2 * L.half; t += 32)
+          correct_fine<T>(L, C, P + L.off, P + C.off, O + C.off, cs, t, v2);
         w.sync();
-        cd_gsrb<T>(L, P + L.off, F + L.off, O + L.off, D.up, false, v2, w);
+        cd_gsrb<T>(L, P + L.off, F + L.off, D.up, false, v2, w);
       }
     }
     __syncthreads();
   } else {
-    cd_gsrb<T>(D.lv[0], P + D.lv[0].off, F + D.lv[0].off, O + D.lv[0].off, D.base, fst, v2, g);
+    cd_gsrb<T>(D.lv[0], P + D.lv[0].off, F + D.lv[0].off, D.base, fst, v2, g);
   }
   // up
   for (l = lw + 1; l <= q; l++) {
     const DLv &L = D.lv[l], &C = D.lv[l - 1];
     const int kk = k + q - l;
     T *cs = corr && kk + 1 < D.ncorr[l - 1] ? corr + D.coff[l - 1] + (kk + 1) * corr_len(C) : nullptr;
-    for (int t = g.tid; t < 2 * C.half; t += g.n) correct_at<T>(L, C, P + L.off, P + C.off, O + C.off, cs, t, v2);
+    cd_correct<T>(L, C, P + L.off, P + C.off, O + C.off, cs, v2);
     g.sync();
-    cd_gsrb<T>(L, P + L.off, F + L.off, O + L.off, D.up, false, v2, g);
+    cd_gsrb<T>(L, P + L.off, F + L.off, D.up, false, v2, g);
   }
 }
 
@@ -441,9 +580,14 @@ __device__ void cd_vcycle(const DCoarse &D, T *P, T *F, T *O, int q, bool first,
 // and F back (else only the top level's P, which the level above corrects
 // from).
 template <class T>
-__global__ void __launch_bounds__(NTHD) k3d_coarse(const __grid_constant__ DCoarse D, T *gP, T *gF, T *gO, T *corr,
-                                                   int mode, int k, int last, T v2) {
+__global__ void __launch_bounds__(NTHD, 1) k3d_coarse(const __grid_constant__ DCoarse gD, T *gP, T *gF, T *gO, T *corr,
+                                                      int mode, int k, int last, T v2) {
   extern __shared__ double2 sm_d2[];
+  // the levels are indexed at run time: their description in shared memory
+  __shared__ DCoarse D;
+  for (int t = threadIdx.x; t < (int)(sizeof(DCoarse) / sizeof(int)); t += NTHD)
+    reinterpret_cast<int *>(&D)[t] = reinterpret_cast<const int *>(&gD)[t];
+  __syncthreads();
   T *P = reinterpret_cast<T *>(sm_d2), *F = P + D.cells, *O = F + D.cells;
   const int top = D.n - 1;
   {
@@ -480,8 +624,7 @@ __global__ void __launch_bounds__(NTHD) k3d_coarse(const __grid_constant__ DCoar
       if (l > 0) {
         const DLv &L = D.lv[l], &C = D.lv[l - 1];
         T *cs = corr && D.ncorr[l - 1] > 0 ? corr + D.coff[l - 1] : nullptr;
-        for (int t = threadIdx.x; t < 2 * C.half; t += NTHD)
-          correct_at<T>(L, C, P + L.off, P + C.off, O + C.off, cs, t, v2);
+        cd_correct<T>(L, C, P + L.off, P + C.off, O + C.off, cs, v2);
         __syncthreads();
       }
       cd_vcycle<T>(D, P, F, O, l, false, corr, 0, v2);
@@ -683,9 +826,10 @@ __global__ void __launch_bounds__(256) k3d_mx_resid(DLv L, const double *P, cons
   if (t >= (unsigned)(2 * L.half / V)) return;
   const int c = t >= (unsigned)(L.half / V), u = t - c * (L.half / V);
   const int nv = L.nx2 / V, r = fastdiv(u, L.m_nxv), xv = (u - r * nv) * V;
-  const int z = fastdiv(r, L.m_ny), y = r - z * L.ny, b = r * L.nx2 + xv;
+  const Group g = group_of<V>(L, xv, r);
+  const int b = g.b;
   const Vec<double, V> o = ldv<double, V>(P + c * L.half + b), f = ldv<double, V>(F + c * L.half + b);
-  const Nbr<double, V> n = neighbours<double, V>(L, P + (1 - c) * L.half, o, b, xv, y, z, (c + y + z) & 1, v2);
+  const Nbr<double, V> n = neighbours<double, V>(L, P, c, g, v2);
   Vec<float, V> w;
 #pragma unroll
   for (int k = 0; k < V; k++) w.v[k] = (float)(f.v[k] - lpl_of<double, V>(n, k, o.v[k], L.inv_dx2));
