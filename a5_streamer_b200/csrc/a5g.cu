@@ -103,11 +103,13 @@ struct RunDev {
   int bx_off[MAXLEV + 1], pb_off[MAXLEV + 1];
   int lv_nc[MAXLEV], pad3;
   double lv_dr[MAXLEV];
+  double lv_dx2[MAXLEV], lv_inv2[MAXLEV];  // dr^2, 1 / dr^2
   const BoxRec *boxes;
   const BoxRec *sboxes;        // records addressing the shared-memory copy
   // cell plans and cylindrical weights of the shared-memory solve, built on
   // the host per topology: level index li uses block cplan_blk[li] (2 NTHR
   // entries), -1 where the level's colours do not fit one cell per thread
+  // (or an address does not fit 16 bits)
   const int4 *cplan;
   const double2 *cwts;
   int cplan_blk[MAXLEV];
@@ -290,11 +292,16 @@ constexpr int WTS_DOUBLES = 2 * NTHR * 2;      // doubles taken by the weights
 // applied potential (2 V - own); sides_bc_pot (src/streamer_2d.f90:620-638).
 enum { GK_COPY = 0, GK_RB = 1, GK_NEG = 2, GK_TOP = 3 };
 
-// A cell plan as an int4: x = cell address (-1: none), y / z = first source
-// of the x / y ghost neighbour, w = i | j << 8 | x kind << 16 | y kind << 18.
+// A cell plan as an int4 of 16-bit addresses in the shared-memory arrays:
+// x = cell | lx source << 16, y = hx source | ly source << 16, z = hy source |
+// VF_ flags << 16, w = parent cell of the 2 x 2 block the cell's thread
+// restricts (p_visit). The source of a neighbour is the neighbour's cell, or
+// for a ghost neighbour the first source of its recipe.
+enum { VF_ON = 1, VF_RBX = 2, VF_XL = 4, VF_RBY = 8, VF_YL = 16, VF_NEG = 32, VF_TOP = 64, VF_ODDI = 128, VF_ODDJ = 256,
+       VF_PARENT = 512 };
 
 // First source and kind of side ghost (side, k) of box B (as phi_ghost).
-__host__ __device__ __forceinline__ void ghost_src(const BoxRec &B, int nc, int ncg, int side, int k, int &s0,
+inline void ghost_src(const BoxRec &B, int nc, int ncg, int side, int k, int &s0,
                                           int &kind) {
   const int dim = side >> 1;
   const bool low = (side & 1) == 0;
@@ -314,14 +321,20 @@ __host__ __device__ __forceinline__ void ghost_src(const BoxRec &B, int nc, int 
   }
 }
 
-__host__ __device__ __forceinline__ int4 make_plan(const BoxRec &B, int nc, int ncg, int i, int j) {
-  int4 c;
-  c.x = B.base + i + ncg * j;
-  int xk, yk;
-  ghost_src(B, nc, ncg, i == 1 ? 0 : 1, j, c.y, xk);
-  ghost_src(B, nc, ncg, j == 1 ? 2 : 3, i, c.z, yk);
-  c.w = i | (j << 8) | (xk << 16) | (yk << 18);
-  return c;
+inline int4 make_plan(const BoxRec &B, int nc, int ncg, int i, int j, int parent_cell) {
+  const int g = B.base + i + ncg * j;
+  int gx, gy, xk, yk;
+  ghost_src(B, nc, ncg, i == 1 ? 0 : 1, j, gx, xk);
+  ghost_src(B, nc, ncg, j == 1 ? 2 : 3, i, gy, yk);
+  const int lx = i > 1 ? g - 1 : gx, hx = i < nc ? g + 1 : gx, ly = j > 1 ? g - ncg : gy, hy = j < nc ? g + ncg : gy;
+  const bool ex = i == 1 || i == nc, ey = j == 1 || j == nc;  // has an x / y ghost neighbour
+  int fl = VF_ON | (i & 1 ? VF_ODDI : 0) | (j & 1 ? VF_ODDJ : 0) | (i == 1 ? VF_XL : 0) | (j == 1 ? VF_YL : 0) |
+           (B.flags & CF_PARENT ? VF_PARENT : 0);
+  if (ex && xk == GK_RB) fl |= VF_RBX;
+  if (ey && yk == GK_RB) fl |= VF_RBY;
+  if (ey && yk == GK_NEG) fl |= VF_NEG;
+  if (ey && yk == GK_TOP) fl |= VF_TOP;
+  return make_int4(g | (lx << 16), hx | (ly << 16), hy | (fl << 16), parent_cell);
 }
 
 // box_gsrb_clpl weights (i+ioff-1)/(i+ioff-1/2) and (i+ioff)/(i+ioff-1/2)
@@ -617,19 +630,22 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
     const int nc = P.lv_nc[li], ncg = nc + 2, half = (nc * nc) >> 1, hn = nc >> 1;
     const int sh = __builtin_ctz(nc), hsh = 2 * sh - 1;
     const int b0 = P.bx_off[li], nb = P.bx_off[li + 1] - b0;
-    if (nb * half > NTHR) continue;
+    if (nb * half > NTHR || P.smem_doubles > 65535) continue;
     P.cplan_blk[li] = (int)(P.cplan.size() / (2 * NTHR));
     for (int k = 0; k < NTHR; k++) {
       int4 c[2];
-      c[0] = c[1] = make_int4(-1, 0, 0, 0);
+      c[0] = c[1] = make_int4(0, 0, 0, 0);
       double2 w[2] = {make_double2(0, 0), make_double2(0, 0)};
       if (k < nb * half) {
         const BoxRec &B = P.sboxes[b0 + (k >> hsh)];
         const int item = k & (half - 1);
         const int j = (item >> (sh - 1)) + 1, m = item & (hn - 1);
+        const int pncg = li > 0 ? P.lv_nc[li - 1] + 2 : 0;
+        const int pc = li > 0 ? B.pbase + (B.o0 + m + 1) + pncg * (B.o1 + ((j - 1) >> 1) + 1) : 0;
         for (int p = 0; p < 2; p++) {
-          c[p] = make_plan(B, nc, ncg, 2 * m + 2 - ((p + j) & 1), j);
-          cyl_weights(B.gi0 + (c[p].w & 255), w[p].x, w[p].y);
+          const int i = 2 * m + 2 - ((p + j) & 1);
+          c[p] = make_plan(B, nc, ncg, i, j, pc);
+          cyl_weights(B.gi0 + i, w[p].x, w[p].y);
         }
       }
       P.cplan.push_back(c[0]);
@@ -1428,6 +1444,10 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
   std::memcpy(h.pb_off, P.pb_off, sizeof(P.pb_off));
   std::memcpy(h.lv_nc, P.lv_nc, sizeof(P.lv_nc));
   std::memcpy(h.lv_dr, P.lv_dr, sizeof(P.lv_dr));
+  for (int li = 0; li < nlev; li++) {
+    h.lv_dx2[li] = P.lv_dr[li] * P.lv_dr[li];
+    h.lv_inv2[li] = 1 / (P.lv_dr[li] * P.lv_dr[li]);
+  }
   h.boxes = c->p_boxes;
   h.pbx = c->p_pbx;
   h.cplan = c->p_cplan;

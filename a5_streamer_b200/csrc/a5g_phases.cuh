@@ -716,7 +716,7 @@ __device__ __forceinline__ T lap_at(const RunDev &R, double V, const T *phi, con
 
 struct LvlInfo {
   int nc, ncg, sh, b0, nb, li;
-  double dr;
+  double dx2, inv2;  // dr^2, 1 / dr^2 (formed on the host: no division in a phase)
 };
 __device__ __forceinline__ LvlInfo lvl_info(const RunDev &R, int lvl) {
   const int li = lvl - R.min_lvl;
@@ -727,7 +727,8 @@ __device__ __forceinline__ LvlInfo lvl_info(const RunDev &R, int lvl) {
   L.b0 = R.bx_off[li];
   L.nb = R.bx_off[li + 1] - L.b0;
   L.li = li;
-  L.dr = R.lv_dr[li];
+  L.dx2 = R.lv_dx2[li];
+  L.inv2 = R.lv_inv2[li];
   return L;
 }
 
@@ -771,7 +772,7 @@ __device__ __noinline__ void p_sweep(const RunDev &R, const MGV<T> &M, int lvl, 
   const LvlInfo L = lvl_info(R, lvl);
   T *phi = M.phi;
   const T *rhs = M.rhs;
-  const T dx2 = T(L.dr * L.dr);
+  const T dx2 = T(L.dx2);
   const int half = (L.nc * L.nc) >> 1, hsh = 2 * L.sh - 1, hn = L.nc >> 1;
   const int p = it & 1;  // parity (i + j) & 1 of the updated cells
   const bool cyl = R.coord == 1;
@@ -868,16 +869,16 @@ __device__ void p_fill(const RunDev &R, const MGV<T> &M, int lvl) {
 // parent's phi (box_rstr_lpl, :683-705); fill: the ghosts of level lvl are
 // filled in the same phase (the residual evaluates ghost neighbours from
 // their sources). leaf_rhs: first set the space charge e/eps0 (n_e - n_i) on
-// leaf cells (src/streamer_2d.f90:317-329). store_res: keep the residual in
-// the box's own tmp (set_coarse_phi_rhs); otherwise tmp is left as it was
-// (update_coarse saves and restores it).
+// leaf cells (src/streamer_2d.f90:317-329). The box's own tmp is left as it
+// was (update_coarse saves and restores it; what set_coarse_phi_rhs leaves
+// there is overwritten by the FMG's copy before any read).
 template <class T>
-__device__ __noinline__ void p_fr(const RunDev &R, const MGV<T> &M, int lvl, bool fill, bool leaf_rhs, bool store_res) {
+__device__ __noinline__ void p_fr(const RunDev &R, const MGV<T> &M, int lvl, bool fill, bool leaf_rhs) {
   const LvlInfo L = lvl_info(R, lvl);
   const int pncg = R.lv_nc[lvl - 1 - R.min_lvl] + 2;
   T *phi = M.phi, *tmp = M.tmp, *rhs = M.rhs;
   const double *e = VAR(R, I_ELEC), *pi = VAR(R, I_PION);
-  const T inv_dr_sq = T(1 / (L.dr * L.dr));
+  const T inv_dr_sq = T(L.inv2);
   const double fac = UC_ELEM_CHARGE / UC_EPS0;
   // one cell per thread, whole warps per iteration: the 2x2 block of a
   // parent cell is gathered by shuffles (cells of a box are consecutive
@@ -899,7 +900,6 @@ __device__ __noinline__ void p_fr(const RunDev &R, const MGV<T> &M, int lvl, boo
         rh = rhs[g];
       }
       res = rh - lap_at(R, M.V, phi, B, L.nc, L.ncg, i, j, inv_dr_sq);
-      if (store_res) tmp[g] = res;
       ph = phi[g];
     }
     const unsigned FULL = 0xffffffffu;
@@ -927,7 +927,7 @@ __device__ void p_fc(const RunDev &R, const MGV<T> &M, int lvl, bool copy_tmp) {
   const int *pb = M.pbx + R.pb_off[li];
   const int npb = R.pb_off[li + 1] - R.pb_off[li];
   T *phi = M.phi, *tmp = M.tmp, *rhs = M.rhs;
-  const T inv_dr_sq = T(1 / (L.dr * L.dr));
+  const T inv_dr_sq = T(L.inv2);
   const int per = L.nc * L.nc, n = npb * per;
   for (int k = TID(), nt_ = NTH(); k < n; k += nt_) {
     const BoxRec &B = M.boxes[pb[k >> (2 * L.sh)]];
@@ -1048,7 +1048,7 @@ __device__ __noinline__ void p_residual_all(const RunDev &R, const MGV<T> &M, in
   const T *rhs = M.rhs;
   for (int lvl = R.min_lvl; lvl <= max_lvl; lvl++) {
     const LvlInfo L = lvl_info(R, lvl);
-    const T inv_dr_sq = T(1 / (L.dr * L.dr));
+    const T inv_dr_sq = T(L.inv2);
     const int per = L.nc * L.nc, n = L.nb * per;
     for (int k = TID(), nt_ = NTH(); k < n; k += nt_) {
       const BoxRec &B = M.boxes[L.b0 + (k >> (2 * L.sh))];
@@ -1061,54 +1061,35 @@ __device__ __noinline__ void p_residual_all(const RunDev &R, const MGV<T> &M, in
 }
 
 // ---------------------------------------------------------------------------
-// Cell plans of a level visit. When the multigrid variables are in shared
-// memory and every colour of a level has at most one cell per thread, each
-// thread forms once per visit, for its red and its black cell, the cell
-// address and the first source and kind of each ghost neighbour, and keeps
-// them in its two shared-memory plan slots through the half-sweeps (and the
-// residual/restriction) of that visit. The values computed are those of
-// p_sweep / p_fr; only the address work moves out of the phases.
+// Level visits of the shared-memory solve. Where every colour of a level has
+// at most one cell per thread, the host forms for each thread's red and black
+// cell the addresses of the cell's four neighbours (or of their ghost
+// recipes' first sources) and the kinds of those recipes; a visit takes them
+// into registers once and runs the level's half-sweeps, and on the way down
+// the residual and restriction, from there. The values are those of p_sweep /
+// p_fr. A visit's phases are a chain of short dependent steps on one SM, so
+// what counts is the latency of one step: four shared-memory loads and the
+// sum, no address work, no branch where no recipe but a copy occurs.
 
-// Value of a ghost neighbour from its first source v0 and the cell's own
-// value vo, its neighbour across the box va and along the side vb.
+// The multigrid arrays of the shared-memory solve, from the dynamic shared
+// memory itself: derived from g_dsmem they are known to be shared.
 template <class T>
-__device__ __forceinline__ T ghost_eval(T v0, int kind, T vo, T va, T vb, double V) {
-  const T vrb = T(0.5) * v0 + vo - T(0.25) * (va + vb);
-  const T vw = kind == GK_NEG ? -vo : T(2 * V) - vo;
-  return kind == GK_COPY ? v0 : (kind == GK_RB ? vrb : vw);
-}
-
-// The four neighbours of the plan's cell (as phi_nbrs; mem: read the ghost
-// cells stored in memory instead). The across and along neighbours a ghost
-// recipe reads are among the cell's direct neighbours.
+struct SmArr {
+  T *phi, *rhs, *tmp;
+  const BoxRec *boxes;
+  T v2;  // twice the potential of the applied-voltage wall
+};
 template <class T>
-__device__ __forceinline__ void plan_nbrs(double V, const T *phi, const int4 &c, int nc, int ncg,
-                                          bool mem, T &lx, T &hx, T &ly, T &hy) {
-  const int g = c.x, i = c.w & 255, j = (c.w >> 8) & 255;
-  const T dlx = phi[g - 1], dhx = phi[g + 1], dly = phi[g - ncg], dhy = phi[g + ncg];
-  if (mem) {
-    lx = dlx;
-    hx = dhx;
-    ly = dly;
-    hy = dhy;
-    return;
-  }
-  const T vo = phi[g], x0 = phi[c.y], y0 = phi[c.z];
-  const T gx = ghost_eval(x0, (c.w >> 16) & 3, vo, i == 1 ? dhx : dlx, (j & 1) ? dhy : dly, V);
-  const T gy = ghost_eval(y0, (c.w >> 18) & 3, vo, j == 1 ? dhy : dly, (i & 1) ? dhx : dlx, V);
-  lx = i > 1 ? dlx : gx;
-  hx = i < nc ? dhx : gx;
-  ly = j > 1 ? dly : gy;
-  hy = j < nc ? dhy : gy;
+__device__ __forceinline__ SmArr<T> sm_arrays(const RunDev &R) {
+  double *base = g_dsmem + PLAN_DOUBLES + (R.coord == 1 ? WTS_DOUBLES : 0);
+  T *b = reinterpret_cast<T *>(base);
+  const int S = std::is_same<T, double>::value ? R.smem_doubles : R.mx_smem;
+  return SmArr<T>{b, b + S, b + 2 * S, reinterpret_cast<const BoxRec *>(b + 3 * S),
+                  std::is_same<T, double>::value ? T(2 * R.applied_voltage) : T(0)};
 }
 
 __device__ __forceinline__ int4 *plan_slots() { return reinterpret_cast<int4 *>(g_dsmem); }
 __device__ __forceinline__ double2 *wts_slots() { return reinterpret_cast<double2 *>(g_dsmem + PLAN_DOUBLES); }
-
-struct LevelPlan {
-  int bx;    // index of the box record of the thread's cells (-1: none)
-  int item;  // cell index within each colour of the box (row-major, nc/2 per row)
-};
 
 // Asynchronous 16-byte copies global -> shared (cp.async), used to fetch the
 // host-built plans of the next level while the current level's phases run.
@@ -1120,83 +1101,25 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// The level index whose plans are being fetched into the slots (-1: none).
+// The level index whose plans are in the slots or on their way (-1: none).
 // Every thread tracks the same value: the control flow of the multigrid is
-// uniform over the block.
+// uniform over the block. Each thread copies and reads its own slots only.
 struct PlanFetch {
   int li = -1;
 };
 
 template <class T>
-__device__ __forceinline__ bool plan_fits(const MGV<T> &M, const LvlInfo &L) {
-  return M.plans && L.nb * ((L.nc * L.nc) >> 1) <= NTHR;
+__device__ __forceinline__ bool plan_fits(const RunDev &R, const MGV<T> &M, const LvlInfo &L) {
+  return M.plans && R.cplan_blk[L.li] >= 0;
 }
 
-// Forms the thread's two cell plans (colour p = (i + j) & 1). Each thread
-// reads only its own slots afterwards, so no barrier is needed.
-template <class T>
-__device__ __forceinline__ LevelPlan make_level_plan(const RunDev &R, const MGV<T> &M, const LvlInfo &L,
-                                                     bool cyl, PlanFetch &pf) {
-  LevelPlan P;
-  const int half = (L.nc * L.nc) >> 1, hsh = 2 * L.sh - 1, hn = L.nc >> 1;
-  const int k = threadIdx.x;
-  P.bx = -1;
-  P.item = k & (half - 1);
-  if (k < L.nb * half) P.bx = L.b0 + (k >> hsh);
-  const int blk = R.cplan_blk[L.li];
-  if (pf.li >= 0) {
-    // a fetch is in flight: let it land (it is this level's plans, or slots
-    // about to be overwritten)
-    cp_async_wait_all();
-    const bool mine = pf.li == L.li;
-    pf.li = -1;
-    if (mine) return P;
-  }
-  if (blk >= 0) {
-    // plans of this level built on the host at the topology upload
-    const size_t o = (size_t)blk * 2 * NTHR + 2 * threadIdx.x;
-    plan_slots()[2 * threadIdx.x] = R.cplan[o];
-    plan_slots()[2 * threadIdx.x + 1] = R.cplan[o + 1];
-    if (cyl) {
-      wts_slots()[2 * threadIdx.x] = R.cwts[o];
-      wts_slots()[2 * threadIdx.x + 1] = R.cwts[o + 1];
-    }
-    return P;
-  }
-  int4 c[2];
-  c[0].x = c[1].x = -1;
-  if (k < L.nb * half) {
-    P.bx = L.b0 + (k >> hsh);
-    const BoxRec &B = M.boxes[P.bx];
-    const int j = (P.item >> (L.sh - 1)) + 1, m = P.item & (hn - 1);
-#pragma unroll
-    for (int p = 0; p < 2; p++) c[p] = make_plan(B, L.nc, L.ncg, 2 * m + 2 - ((p + j) & 1), j);
-  }
-  plan_slots()[2 * threadIdx.x] = c[0];
-  plan_slots()[2 * threadIdx.x + 1] = c[1];
-  if (cyl && P.bx >= 0) {
-    const int gi0 = M.boxes[P.bx].gi0;
-#pragma unroll
-    for (int p = 0; p < 2; p++) {
-      double2 w;
-      cyl_weights(gi0 + (c[p].w & 255), w.x, w.y);
-      wts_slots()[2 * threadIdx.x + p] = w;
-    }
-  }
-  return P;
-}
-
-// Start fetching the host-built plans of level lvl into the slots (each
-// thread its own four 16-byte slots), to be taken by make_level_plan. Only
-// after the last read of the slots by the current level, which a barrier
-// separates from this call.
-template <class T>
-__device__ __forceinline__ void fetch_level_plan(const RunDev &R, const MGV<T> &M, int lvl, bool cyl,
-                                                 PlanFetch &pf) {
-  if (lvl < R.min_lvl || lvl > R.max_lvl || pf.li >= 0) return;
-  const LvlInfo L = lvl_info(R, lvl);
-  const int blk = R.cplan_blk[L.li];
-  if (!plan_fits(M, L) || blk < 0) return;
+// Start fetching the plans of level index li into the slots, unless they are
+// there or the level has none. Only after this thread's last read of them.
+__device__ __forceinline__ void fetch_plan(const RunDev &R, int li, bool cyl, PlanFetch &pf) {
+  if (li < 0 || li >= R.nlev || pf.li == li) return;
+  const int blk = R.cplan_blk[li];
+  if (blk < 0) return;
+  if (pf.li >= 0) cp_async_wait_all();
   const size_t o = (size_t)blk * 2 * NTHR + 2 * threadIdx.x;
   cp_async16(&plan_slots()[2 * threadIdx.x], &R.cplan[o]);
   cp_async16(&plan_slots()[2 * threadIdx.x + 1], &R.cplan[o + 1]);
@@ -1205,75 +1128,173 @@ __device__ __forceinline__ void fetch_level_plan(const RunDev &R, const MGV<T> &
     cp_async16(&wts_slots()[2 * threadIdx.x + 1], &R.cwts[o + 1]);
   }
   cp_async_commit();
-  pf.li = L.li;
+  pf.li = li;
 }
 
-// One red-black half-sweep `it` from the cell plans (p_sweep).
+// One cell of a visit.
 template <class T>
-__device__ __forceinline__ void plan_sweep(const RunDev &R, const MGV<T> &M, const LvlInfo &L,
-                                           const LevelPlan &P, int it, bool mem) {
-  const int4 c = plan_slots()[2 * threadIdx.x + (it & 1)];
-  if (c.x >= 0) {
-    T *phi = M.phi;
-    T lx, hx, ly, hy;
-    plan_nbrs(M.V, phi, c, L.nc, L.ncg, mem, lx, hx, ly, hy);
-    const T r = M.rhs[c.x], dx2 = T(L.dr * L.dr);
-    if (R.coord == 1) {
-      const double2 w = wts_slots()[2 * threadIdx.x + (it & 1)];
-      phi[c.x] = T(0.25) * (T(w.x) * lx + T(w.y) * hx + hy + ly - dx2 * r);
-    } else {
-      phi[c.x] = T(0.25) * (hx + lx + hy + ly - dx2 * r);
+struct VCell {
+  int own, lx, hx, ly, hy;
+  unsigned fl;
+  T wx, wy;  // cylindrical weights of lx, hx
+};
+template <class T>
+__device__ __forceinline__ VCell<T> vcell(int p, bool cyl) {
+  const int4 c = plan_slots()[2 * threadIdx.x + p];
+  VCell<T> v;
+  v.own = c.x & 0xffff;
+  v.lx = (unsigned)c.x >> 16;
+  v.hx = c.y & 0xffff;
+  v.ly = (unsigned)c.y >> 16;
+  v.hy = c.z & 0xffff;
+  v.fl = (unsigned)c.z >> 16;
+  v.wx = v.wy = T(1);
+  if (cyl) {
+    const double2 w = wts_slots()[2 * threadIdx.x + p];
+    v.wx = T(w.x);
+    v.wy = T(w.y);
+  }
+  return v;
+}
+// The four neighbours of a cell (as phi_nbrs). The across and along
+// neighbours that a refinement-boundary recipe reads are among the cell's
+// direct neighbours; a wall's source is the cell itself.
+template <class T>
+__device__ __forceinline__ void vnbrs(const T *phi, const VCell<T> &v, T v2, T &lx, T &hx, T &ly, T &hy) {
+  lx = phi[v.lx];
+  hx = phi[v.hx];
+  ly = phi[v.ly];
+  hy = phi[v.hy];
+  if (v.fl & (VF_RBX | VF_RBY | VF_NEG | VF_TOP)) {
+    const T vo = phi[v.own];
+    const T bx = (v.fl & VF_ODDJ) ? hy : ly, by = (v.fl & VF_ODDI) ? hx : lx;
+    const T gx = T(0.5) * ((v.fl & VF_XL) ? lx : hx) + vo - T(0.25) * (((v.fl & VF_XL) ? hx : lx) + bx);
+    const T gy = T(0.5) * ((v.fl & VF_YL) ? ly : hy) + vo - T(0.25) * (((v.fl & VF_YL) ? hy : ly) + by);
+    if (v.fl & VF_RBX) {
+      if (v.fl & VF_XL) lx = gx;
+      else hx = gx;
     }
+    if (v.fl & VF_RBY) {
+      if (v.fl & VF_YL) ly = gy;
+      else hy = gy;
+    }
+    if (v.fl & VF_NEG) ly = -vo;
+    if (v.fl & VF_TOP) hy = v2 - vo;
+  }
+}
+// box_gsrb_lpl (m_aX_mg.f90:636-659) / box_gsrb_clpl (:998-1024); dr: dx^2 rhs
+template <class T>
+__device__ __forceinline__ T vgsrb(const VCell<T> &v, bool cyl, T lx, T hx, T ly, T hy, T dr) {
+  if (cyl) return T(0.25) * (v.wx * lx + v.wy * hx + hy + ly - dr);
+  return T(0.25) * (hx + lx + hy + ly - dr);
+}
+template <class T>
+__device__ __forceinline__ T vlap(const VCell<T> &v, bool cyl, T lx, T hx, T ly, T hy, T own, T inv) {
+  if (cyl) return (v.wx * lx + v.wy * hx + ly + hy - T(4) * own) * inv;
+  return inv * (lx + hx + ly + hy - T(4) * own);
+}
+
+// One visit of level index li: n half-sweeps (stale: the first reads the ghost
+// cells in memory, as p_sweep's mem), then with down the residual of both
+// cells, restricted with phi into the parent (p_fr without the ghost fill: on
+// the way down no later phase reads this level's ghost cells before p_fill
+// refills them). The 2x2 block of cells (2ii-1..2ii, 2jj-1..2jj) belongs to
+// the threads of items (2jj-2) hn + ii-1 (cells (2ii-1, 2jj-1) and (2ii,
+// 2jj-1)) and that item + hn (cells (2ii, 2jj) and (2ii-1, 2jj)), which are in
+// the same warp; the first adds the four in the order of box_rstr_lpl. The
+// plans of level index next are fetched meanwhile. Out of line: the kernels
+// hold several copies of the cycle, which share this one.
+template <class T>
+__device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, bool stale, bool down, int next, PlanFetch pf) {
+  const SmArr<T> A = sm_arrays<T>(R);
+  const bool cyl = R.coord == 1;
+  T *phi = A.phi;
+  fetch_plan(R, li, cyl, pf);
+  cp_async_wait_all();
+  const VCell<T> c0 = vcell<T>(0, cyl), c1 = vcell<T>(1, cyl);
+  const int pc = plan_slots()[2 * threadIdx.x].w;
+  fetch_plan(R, next, cyl, pf);
+  const bool on = c0.fl & VF_ON;
+  const T dx2 = T(R.lv_dx2[li]);
+  T r0 = 0, r1 = 0;
+  if (on) {
+    r0 = A.rhs[c0.own];
+    r1 = A.rhs[c1.own];
+  }
+  const T d0 = dx2 * r0, d1 = dx2 * r1;
+  T lx, hx, ly, hy;
+  int it = 1;
+  if (stale) {
+    if (on) {
+      const int ncg = R.lv_nc[li] + 2;
+      lx = phi[c1.own - 1];
+      hx = phi[c1.own + 1];
+      ly = phi[c1.own - ncg];
+      hy = phi[c1.own + ncg];
+      phi[c1.own] = vgsrb<T>(c1, cyl, lx, hx, ly, hy, d1);
+    }
+    __syncthreads();
+    it = 2;
+  }
+#pragma unroll 1
+  for (; it <= n; it++) {
+    if (on) {
+      if (it & 1) {
+        vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
+        phi[c1.own] = vgsrb<T>(c1, cyl, lx, hx, ly, hy, d1);
+      } else {
+        vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
+        phi[c0.own] = vgsrb<T>(c0, cyl, lx, hx, ly, hy, d0);
+      }
+    }
+    __syncthreads();
+  }
+  if (!down) return pf;
+  const T inv = T(R.lv_inv2[li]);
+  T e0 = 0, e1 = 0, p0 = 0, p1 = 0;
+  if (on) {
+    p0 = phi[c0.own];
+    p1 = phi[c1.own];
+    vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
+    e0 = r0 - vlap<T>(c0, cyl, lx, hx, ly, hy, p0, inv);
+    vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
+    e1 = r1 - vlap<T>(c1, cyl, lx, hx, ly, hy, p1, inv);
+  }
+  const int nc = R.lv_nc[li], hn = nc >> 1, sh = 31 - __clz(nc);
+  // from the item one row up: its even cell (2ii, 2jj) and odd cell (2ii-1, 2jj)
+  const T e11 = __shfl_down_sync(0xffffffffu, e0, hn), e01 = __shfl_down_sync(0xffffffffu, e1, hn);
+  const T p11 = __shfl_down_sync(0xffffffffu, p0, hn), p01 = __shfl_down_sync(0xffffffffu, p1, hn);
+  const int row = (threadIdx.x & (((nc * nc) >> 1) - 1)) >> (sh - 1);
+  if (on && (row & 1) == 0) {
+    A.tmp[pc] = T(0.25) * (e0 + e1 + e01 + e11);
+    phi[pc] = T(0.25) * (p0 + p1 + p01 + p11);
   }
   __syncthreads();
+  return pf;
 }
 
-// Residual of both cells of the plan, restricted with phi into the parent
-// (p_fr with fill, without leaf_rhs and store_res). The 2x2 block of cells
-// (2ii-1..2ii, 2jj-1..2jj) belongs to the threads of items (2jj-2) hn + ii-1
-// (cells (2ii-1, 2jj-1) and (2ii, 2jj-1)) and that item + hn (cells
-// (2ii, 2jj) and (2ii-1, 2jj)), which are in the same warp; the first adds
-// the four in the order of box_rstr_lpl.
+// p_fc with copy_tmp from the cell plans of level index li: the right-hand
+// side of the parent boxes and their tmp = phi, and the level's ghost fill.
 template <class T>
-__device__ __forceinline__ void plan_fr(const RunDev &R, const MGV<T> &M, const LvlInfo &L,
-                                        const LevelPlan &P, int lvl) {
-  T *phi = M.phi, *tmp = M.tmp;
-  const T inv_dr_sq = T(1 / (L.dr * L.dr));
-  T res[2] = {0, 0}, ph[2] = {0, 0};
+__device__ __noinline__ PlanFetch p_fc_visit(const RunDev &R, const MGV<T> &M, int li, PlanFetch pf) {
+  const SmArr<T> A = sm_arrays<T>(R);
+  const bool cyl = R.coord == 1;
+  fetch_plan(R, li, cyl, pf);
+  cp_async_wait_all();
+  const T inv = T(R.lv_inv2[li]);
 #pragma unroll
   for (int p = 0; p < 2; p++) {
-    const int4 c = plan_slots()[2 * threadIdx.x + p];
-    if (c.x < 0) continue;
+    const VCell<T> c = vcell<T>(p, cyl);
+    if ((c.fl & (VF_ON | VF_PARENT)) != (VF_ON | VF_PARENT)) continue;
     T lx, hx, ly, hy;
-    plan_nbrs(M.V, phi, c, L.nc, L.ncg, false, lx, hx, ly, hy);
-    const T v = phi[c.x];
-    T lap;
-    if (R.coord == 1) {
-      const double2 w = wts_slots()[2 * threadIdx.x + p];
-      lap = (T(w.x) * lx + T(w.y) * hx + ly + hy - T(4) * v) * inv_dr_sq;
-    } else {
-      lap = inv_dr_sq * (lx + hx + ly + hy - T(4) * v);
-    }
-    res[p] = M.rhs[c.x] - lap;
-    ph[p] = v;
+    vnbrs<T>(A.phi, c, A.v2, lx, hx, ly, hy);
+    const T v = A.phi[c.own];
+    A.rhs[c.own] = vlap<T>(c, cyl, lx, hx, ly, hy, v, inv) + A.tmp[c.own];
+    A.tmp[c.own] = v;
   }
-  const int hn = L.nc >> 1;
-  // from the item one row up: its even cell (2ii, 2jj) and odd cell (2ii-1, 2jj)
-  const T r11 = __shfl_down_sync(0xffffffffu, res[0], hn);
-  const T r01 = __shfl_down_sync(0xffffffffu, res[1], hn);
-  const T p11 = __shfl_down_sync(0xffffffffu, ph[0], hn);
-  const T p01 = __shfl_down_sync(0xffffffffu, ph[1], hn);
-  const int row = P.item >> (L.sh - 1);  // j - 1
-  if (P.bx >= 0 && (row & 1) == 0) {
-    const BoxRec &B = M.boxes[P.bx];
-    const int ii = (P.item & (hn - 1)) + 1, jj = (row >> 1) + 1;
-    const int pncg = R.lv_nc[lvl - 1 - R.min_lvl] + 2;
-    const int d = B.pbase + (B.o0 + ii) + pncg * (B.o1 + jj);
-    tmp[d] = T(0.25) * (res[0] + res[1] + r01 + r11);
-    phi[d] = T(0.25) * (ph[0] + ph[1] + p01 + p11);
-  }
-  fill_phi_loop(R, M, L, false);
+  fill_phi_loop(R, M, lvl_info(R, R.min_lvl + li), true);
   __syncthreads();
+  return pf;
 }
 
 // Grid mode: levels with few cells would spend more time in grid barriers
@@ -1325,12 +1346,12 @@ __device__ __forceinline__ void local_end(int size) {
 // coarse ghost fill + rhs; base: 2 n_cycle_base half-sweeps + ghost fill;
 // up: correction, 4 half-sweeps, ghost fill. In grid mode the levels up to
 // local_top run on one block (the down, base and up phases of those levels
-// are consecutive).
+// are consecutive). after: the level index whose plans the caller's next
+// visit takes (out of range: none).
 template <class T>
 __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, int max_lvl, bool stale_base,
                                             PlanFetch &pf, int after) {
   const int min_lvl = R.min_lvl;
-  const bool cyl = R.coord == 1;
   // grid mode: the levels min_lvl..lc run on block 0 alone (the others wait
   // at the barrier of local_end); each level's code appears once
   const int lc = local_top(R, max_lvl);
@@ -1340,29 +1361,25 @@ __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, in
     if (lvl == lc) work = local_begin();
     if (!work) continue;
     const LvlInfo L = lvl_info(R, lvl);
-    if (plan_fits(M, L)) {
-      const LevelPlan P = make_level_plan(R, M, L, cyl, pf);
-      #pragma unroll 1
-      for (int it = 1; it <= M.sw_down; it++) plan_sweep(R, M, L, P, it, false);
-      plan_fr(R, M, L, P, lvl);
+    if (plan_fits(R, M, L)) {
+      pf = p_visit<T>(R, L.li, M.sw_down, false, true, L.li - 1, pf);
     } else {
       for (int it = 1; it <= M.sw_down; it++) p_sweep(R, M, lvl, it, false);
-      p_fr(R, M, lvl, true, false, false);
+      // no ghost fill of this level (update_coarse, :399-407): its ghost
+      // cells are next read after p_fill on the way up
+      p_fr(R, M, lvl, false, false);
     }
-    fetch_level_plan(R, M, lvl - 1, cyl, pf);
-    p_fc(R, M, lvl - 1, true);
+    if (plan_fits(R, M, lvl_info(R, lvl - 1))) pf = p_fc_visit<T>(R, M, L.li - 1, pf);
+    else p_fc(R, M, lvl - 1, true);
   }
   if (lc == min_lvl) work = local_begin();
   if (work) {
     const LvlInfo L = lvl_info(R, min_lvl);
-    if (plan_fits(M, L)) {
-      const LevelPlan P = make_level_plan(R, M, L, cyl, pf);
-      #pragma unroll 1
-      for (int it = 1; it <= M.sw_base; it++) plan_sweep(R, M, L, P, it, stale_base && it == 1);
+    if (plan_fits(R, M, L)) {
+      pf = p_visit<T>(R, 0, M.sw_base, stale_base, false, min_lvl < max_lvl ? 1 : after, pf);
     } else {
       for (int it = 1; it <= M.sw_base; it++) p_sweep(R, M, min_lvl, it, stale_base && it == 1);
     }
-    fetch_level_plan(R, M, min_lvl < max_lvl ? min_lvl + 1 : after, cyl, pf);
     p_fill(R, M, min_lvl);
   }
   for (int lvl = min_lvl + 1; lvl <= max_lvl; lvl++) {
@@ -1372,16 +1389,12 @@ __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, in
     }
     if (!work) continue;
     const LvlInfo L = lvl_info(R, lvl);
-    if (plan_fits(M, L)) {
-      const LevelPlan P = make_level_plan(R, M, L, cyl, pf);
-      p_correct(R, M, lvl, false, true);
-      #pragma unroll 1
-      for (int it = 1; it <= M.sw_up; it++) plan_sweep(R, M, L, P, it, false);
+    p_correct(R, M, lvl, false, true);
+    if (plan_fits(R, M, L)) {
+      pf = p_visit<T>(R, L.li, M.sw_up, false, false, lvl < max_lvl ? L.li + 1 : after, pf);
     } else {
-      p_correct(R, M, lvl, false, true);
       for (int it = 1; it <= M.sw_up; it++) p_sweep(R, M, lvl, it, false);
     }
-    fetch_level_plan(R, M, lvl < max_lvl ? lvl + 1 : after, cyl, pf);
     p_fill(R, M, lvl);
   }
   if (lc == max_lvl && lc >= min_lvl) local_end(size);
@@ -1414,7 +1427,7 @@ __device__ __forceinline__ void p_fmg_in(const RunDev &R, const MGV<T> &M, bool 
   } else {
     // set_coarse_phi_rhs for lvl = max..min+1 (:414-447)
     for (int lvl = max_lvl; lvl >= min_lvl + 1; lvl--) {
-      p_fr(R, M, lvl, lvl == max_lvl, leaf_rhs, true);
+      p_fr(R, M, lvl, lvl == max_lvl, leaf_rhs);
       p_fc(R, M, lvl - 1, false);
     }
   }
@@ -1432,7 +1445,7 @@ __device__ __forceinline__ void p_fmg_in(const RunDev &R, const MGV<T> &M, bool 
     }
     if (!work) continue;
     p_correct(R, M, lvl, true, lvl > min_lvl);
-    p_vcycle(R, M, lvl, first_call && lvl == min_lvl, pf, lvl + 1);
+    p_vcycle(R, M, lvl, first_call && lvl == min_lvl, pf, lvl + 1 - min_lvl);
     if (set_residual && lvl == max_lvl) p_residual_all(R, M, lvl);
   }
   if (lc == max_lvl && lc >= min_lvl) local_end(size);
@@ -1441,47 +1454,66 @@ __device__ __forceinline__ void p_fmg_in(const RunDev &R, const MGV<T> &M, bool 
 
 // Copy the multigrid variables of every box between device memory and the
 // compact shared-memory arrays (in: to shared memory). All slots of all
-// levels form one flat range; a thread moves two slots (three variables
-// each) per round, loading all six values before storing any.
+// levels form one flat range; a thread moves two slots per round, loading
+// both before storing either. fresh: a solve of compute_fld. Its right-hand
+// side is the space charge e/eps0 (n_e - n_i) of the leaves
+// (src/streamer_2d.f90:317-329), formed here; parents' are formed by the
+// solve, so only a box in neither list brings its stored one; tmp is written
+// before it is read, and what it holds after the solve is overwritten by the
+// field, so it moves in neither direction; the ghost entries of the stored
+// right-hand side are left alone. (Three variables whole each way took 8.7 us
+// in and 6.9 us out of the 8 mm tree's solve.)
 template <class T>
-__device__ void stage_mg(const RunDev &R, const MGV<T> &M, T *g0, T *g1, T *g2, bool in) {
-  T *g[3] = {g0, g1, g2};
-  T *s[3] = {M.phi, M.rhs, M.tmp};
+__device__ void stage_mg(const RunDev &R, const MGV<T> &M, T *g0, T *g1, T *g2, bool in, bool fresh) {
   auto level_slots = [&](int li) {
     const int ncg = R.lv_nc[li] + 2;
     return (R.bx_off[li + 1] - R.bx_off[li]) * ncg * ncg;
   };
+  const double *e = VAR(R, I_ELEC), *pi = VAR(R, I_PION);
+  const double fac = UC_ELEM_CHARGE / UC_EPS0;
   int li = 0, lo = 0, hi = level_slots(0);
-  // slot k (not below the previous call's k): source and destination index
-  auto slot_at = [&](int k, int &src, int &dst) {
+  // slot k (not below the previous call's k): device and shared index; kind
+  // of its right-hand side: 0 as stored, 1 the space charge, 2 not moved
+  auto slot_at = [&](int k, int &gi, int &si, int &kind) {
     while (k >= hi) {
       if (++li >= R.nlev) return false;
       lo = hi;
       hi = lo + level_slots(li);
     }
-    const int ncg = R.lv_nc[li] + 2, per = ncg * ncg, t = k - lo;
-    const BoxRec &B = M.boxes[R.bx_off[li] + t / per];
-    const int c = t % per;
-    src = in ? B.gbase + c : B.base + c;
-    dst = in ? B.base + c : B.gbase + c;
+    const int ncg = R.lv_nc[li] + 2, per = ncg * ncg, t = k - lo, b = t / per;
+    const BoxRec &B = M.boxes[R.bx_off[li] + b];
+    const int c = t - b * per, j = c / ncg, i = c - j * ncg;
+    gi = B.gbase + c;
+    si = B.base + c;
+    kind = 0;
+    if (fresh) {
+      const bool inner = i >= 1 && i <= ncg - 2 && j >= 1 && j <= ncg - 2;
+      if (!inner) kind = 2;
+      else if (in) kind = (B.flags & CF_LEAF) && li > 0 ? 1 : ((B.flags & CF_PARENT) ? 2 : 0);
+    }
     return true;
   };
-  T *const *from = in ? g : s;
-  T *const *to = in ? s : g;
   for (int k = threadIdx.x;; k += 2 * NTHR) {
-    int a0, d0, a1 = 0, d1 = 0;
-    if (!slot_at(k, a0, d0)) break;
-    const bool two = slot_at(k + NTHR, a1, d1);
-    T v0[3], v1[3];
+    int g[2] = {0, 0}, s[2] = {0, 0}, kind[2] = {2, 2};
+    bool ok[2];
+    ok[0] = slot_at(k, g[0], s[0], kind[0]);
+    if (!ok[0]) break;
+    ok[1] = slot_at(k + NTHR, g[1], s[1], kind[1]);
+    T v0[2], v1[2], v2[2];
 #pragma unroll
-    for (int v = 0; v < 3; v++) {
-      v0[v] = from[v][a0];
-      if (two) v1[v] = from[v][a1];
+    for (int u = 0; u < 2; u++) {
+      if (!ok[u]) continue;
+      v0[u] = in ? g0[g[u]] : M.phi[s[u]];
+      if (kind[u] == 0) v1[u] = in ? g1[g[u]] : M.rhs[s[u]];
+      if (kind[u] == 1) v1[u] = T(fac * (e[g[u]] - pi[g[u]]));
+      if (!fresh) v2[u] = in ? g2[g[u]] : M.tmp[s[u]];
     }
 #pragma unroll
-    for (int v = 0; v < 3; v++) {
-      to[v][d0] = v0[v];
-      if (two) to[v][d1] = v1[v];
+    for (int u = 0; u < 2; u++) {
+      if (!ok[u]) continue;
+      (in ? M.phi[s[u]] : g0[g[u]]) = v0[u];
+      if (kind[u] != 2) (in ? M.rhs[s[u]] : g1[g[u]]) = v1[u];
+      if (!fresh) (in ? M.tmp[s[u]] : g2[g[u]]) = v2[u];
     }
   }
   __syncthreads();
@@ -1544,8 +1576,10 @@ __device__ __forceinline__ void mg_staged(const RunDev &R, const F &body);
 // each copy sees its descriptor M as constants.
 struct FmgBody {
   bool set_residual, first_call, leaf_rhs;
+  __device__ __forceinline__ bool fresh() const { return leaf_rhs; }
   __device__ __forceinline__ void operator()(const RunDev &R, const MGV<double> &M) const {
-    p_fmg_in(R, M, set_residual, first_call, leaf_rhs);
+    // in shared memory the staging has formed the leaves' right-hand side
+    p_fmg_in(R, M, set_residual, first_call, leaf_rhs && !M.plans);
   }
 };
 // mg$D_fas_vcycle(tree, mg, max_lvl, set_residual) on its own
@@ -1554,9 +1588,10 @@ struct FmgBody {
 struct VcycleBody {
   int max_lvl;
   bool set_residual;
+  __device__ __forceinline__ bool fresh() const { return false; }
   __device__ __forceinline__ void operator()(const RunDev &R, const MGV<double> &M) const {
     PlanFetch pf;
-    p_vcycle(R, M, max_lvl, false, pf, R.max_lvl + 1);
+    p_vcycle(R, M, max_lvl, false, pf, R.nlev);
     if (set_residual) p_residual_all(R, M, max_lvl);
     if (pf.li >= 0) cp_async_wait_all();
   }
@@ -1590,9 +1625,9 @@ __device__ __forceinline__ void mg_staged(const RunDev &R, const F &body) {
     __syncthreads();
     MGV<double> M{base, base + S, base + 2 * S, sb, spb, true, R.applied_voltage,
                   4, 4, 2 * R.n_cycle_base};
-    stage_mg(R, M, VAR(R, MP), VAR(R, MR), VAR(R, MT), true);
+    stage_mg(R, M, VAR(R, MP), VAR(R, MR), VAR(R, MT), true, body.fresh());
     body(R, M);
-    stage_mg(R, M, VAR(R, MP), VAR(R, MR), VAR(R, MT), false);
+    stage_mg(R, M, VAR(R, MP), VAR(R, MR), VAR(R, MT), false, body.fresh());
   } else {
     MGV<double> M{VAR(R, MP), VAR(R, MR), VAR(R, MT), R.boxes, R.pbx, false, R.applied_voltage,
                   4, 4, 2 * R.n_cycle_base};
@@ -1631,7 +1666,7 @@ __device__ __noinline__ void p_mx_residual(const RunDev &R, const MGV<float> &M,
   double *phi = VAR(R, I_PHI), *rhs = VAR(R, I_RHS);
   const double *e = VAR(R, I_ELEC), *pi = VAR(R, I_PION);
   float *ce = M.phi, *cr = M.rhs, *ct = M.tmp;
-  const double inv_dr_sq = 1 / (L.dr * L.dr);
+  const double inv_dr_sq = L.inv2;
   const double fac = UC_ELEM_CHARGE / UC_EPS0;
   const int per = L.nc * L.nc, n = L.nb * per, nw = (n + 31) & ~31;
   for (int k = TID(), nt_ = NTH(); k < nw; k += nt_) {
@@ -1752,11 +1787,11 @@ __device__ void p_solve_mixed(const RunDev &R) {
     for (int lvl = R.max_lvl; lvl >= R.min_lvl; lvl--) p_mx_residual(R, M, lvl);
     // the plans that follow the last V-cycle of a pass: those of the next
     // pass's first V-cycle (fetched while the FP64 phases run), or none
-    const int next = pass + 1 < R.mx_n_corr ? (R.mx_fmg ? R.min_lvl : R.max_lvl) : R.max_lvl + 1;
+    const int next = pass + 1 < R.mx_n_corr ? (R.mx_fmg ? 0 : R.nlev - 1) : R.nlev;
     if (R.mx_fmg) {
       for (int lvl = R.min_lvl; lvl <= R.max_lvl; lvl++) {
         p_correct(R, M, lvl, true, lvl > R.min_lvl);
-        p_vcycle(R, M, lvl, false, pf, lvl < R.max_lvl ? lvl + 1 : next);
+        p_vcycle(R, M, lvl, false, pf, lvl < R.max_lvl ? lvl + 1 - R.min_lvl : next);
       }
     } else {
       p_vcycle(R, M, R.max_lvl, false, pf, next);
