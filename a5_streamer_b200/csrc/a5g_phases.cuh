@@ -1194,18 +1194,30 @@ __device__ __forceinline__ T vlap(const VCell<T> &v, bool cyl, T lx, T hx, T ly,
   return inv * (lx + hx + ly + hy - T(4) * own);
 }
 
-// One visit of level index li: n half-sweeps (stale: the first reads the ghost
-// cells in memory, as p_sweep's mem), then with down the residual of both
-// cells, restricted with phi into the parent (p_fr without the ghost fill: on
-// the way down no later phase reads this level's ghost cells before p_fill
-// refills them). The 2x2 block of cells (2ii-1..2ii, 2jj-1..2jj) belongs to
-// the threads of items (2jj-2) hn + ii-1 (cells (2ii-1, 2jj-1) and (2ii,
-// 2jj-1)) and that item + hn (cells (2ii, 2jj) and (2ii-1, 2jj)), which are in
-// the same warp; the first adds the four in the order of box_rstr_lpl. The
-// plans of level index next are fetched meanwhile. Out of line: the kernels
-// hold several copies of the cycle, which share this one.
+// One visit of level index li: what flags ask for around n half-sweeps.
+//  PV_FC: the level has just been reached by the restriction: the parent
+//    boxes' right-hand side lpl(phi) + tmp, tmp = phi, and the level's ghost
+//    fill (p_fc with copy_tmp);
+//  PV_COPY: tmp = phi (the FMG's stage copy), PV_CORRECT: the parent's
+//    correction added (p_correct);
+//  PV_STALE: the first half-sweep reads the ghost cells in memory (p_sweep's
+//    mem);
+//  PV_DOWN: after the half-sweeps the residual of both cells, restricted with
+//    phi into the parent (p_fr without the ghost fill: on the way down no
+//    later phase reads this level's ghost cells before they are refilled).
+//    The 2x2 block of cells (2ii-1..2ii, 2jj-1..2jj) belongs to the threads of
+//    items (2jj-2) hn + ii-1 (cells (2ii-1, 2jj-1) and (2ii, 2jj-1)) and that
+//    item + hn (cells (2ii, 2jj) and (2ii-1, 2jj)), which are in the same
+//    warp; the first adds the four in the order of box_rstr_lpl;
+//  PV_FILL: the level's ghost fill after the half-sweeps (p_fill).
+// The plans of level index next are fetched meanwhile. One out-of-line
+// function for all of it: the cycle calls it for every level in turn, and
+// inlined or separate pieces cost more in instruction fetch and set-up than
+// the half-sweeps themselves (8 mm tree: set-up, right-hand side, correction
+// and fills as calls of their own 121 us of a step, its half-sweeps 115 us).
+enum { PV_FC = 1, PV_COPY = 2, PV_CORRECT = 4, PV_STALE = 8, PV_DOWN = 16, PV_FILL = 32 };
 template <class T>
-__device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, bool stale, bool down, int next, PlanFetch pf) {
+__device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int flags, int next, PlanFetch pf) {
   const SmArr<T> A = sm_arrays<T>(R);
   const bool cyl = R.coord == 1;
   T *phi = A.phi;
@@ -1215,18 +1227,62 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, bool s
   const int pc = plan_slots()[2 * threadIdx.x].w;
   fetch_plan(R, next, cyl, pf);
   const bool on = c0.fl & VF_ON;
-  const T dx2 = T(R.lv_dx2[li]);
-  T r0 = 0, r1 = 0;
-  if (on) {
+  const T dx2 = T(R.lv_dx2[li]), inv = T(R.lv_inv2[li]);
+  const int nc = R.lv_nc[li], ncg = nc + 2, sh = 31 - __clz(nc);
+  T r0 = 0, r1 = 0, lx, hx, ly, hy;
+  if (on && (flags & PV_FC) && (c0.fl & VF_PARENT)) {
+    const T v0 = phi[c0.own], v1 = phi[c1.own];
+    vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
+    r0 = vlap<T>(c0, cyl, lx, hx, ly, hy, v0, inv) + A.tmp[c0.own];
+    vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
+    r1 = vlap<T>(c1, cyl, lx, hx, ly, hy, v1, inv) + A.tmp[c1.own];
+    A.rhs[c0.own] = r0;
+    A.rhs[c1.own] = r1;
+    A.tmp[c0.own] = v0;
+    A.tmp[c1.own] = v1;
+  } else if (on) {
     r0 = A.rhs[c0.own];
     r1 = A.rhs[c1.own];
   }
+  if (on && (flags & (PV_COPY | PV_CORRECT))) {
+    const T v0 = phi[c0.own], v1 = phi[c1.own];
+    if (flags & PV_COPY) {
+      A.tmp[c0.own] = v0;
+      A.tmp[c1.own] = v1;
+    }
+    if (flags & PV_CORRECT) {
+      // both cells lie under parent cell pc; the neighbours away from the
+      // cell in x (by the cell's column parity) and y (by the row's)
+      const int pncg = R.lv_nc[li - 1] + 2, ps = (c0.fl & VF_ODDJ) ? pc - pncg : pc + pncg;
+      const T q = phi[pc] - A.tmp[pc], qy = phi[ps] - A.tmp[ps];
+      const T ql = phi[pc - 1] - A.tmp[pc - 1], qh = phi[pc + 1] - A.tmp[pc + 1];
+      phi[c0.own] = v0 + T(0.5) * q + T(0.25) * (((c0.fl & VF_ODDI) ? ql : qh) + qy);
+      phi[c1.own] = v1 + T(0.5) * q + T(0.25) * (((c1.fl & VF_ODDI) ? ql : qh) + qy);
+    }
+  }
+  // ghost cells: fill (PV_FC, and tmp of parent boxes) or copy to tmp
+  const double V = std::is_same<T, double>::value ? R.applied_voltage : 0.0;
+  auto ghosts = [&](bool fill, bool copy_parents, bool copy_all) {
+    const int b0 = R.bx_off[li], per = 4 * nc, ng = (R.bx_off[li + 1] - b0) * per;
+    for (int k = threadIdx.x; k < ng; k += NTHR) {
+      const BoxRec &B = A.boxes[b0 + (k >> (sh + 2))];
+      const int r = k & (per - 1), side = r >> sh, kk = (r & (nc - 1)) + 1;
+      const int dim = side >> 1, gx = (side & 1) ? nc + 1 : 0;
+      const int d = B.base + (dim == 0 ? gx + ncg * kk : kk + ncg * gx);
+      if (fill) {
+        const T v = phi_ghost_sl(V, (const T *)phi, B, nc, ncg, side, kk);
+        phi[d] = v;
+        if (copy_parents && (B.flags & CF_PARENT)) A.tmp[d] = v;
+      }
+      if (copy_all) A.tmp[d] = phi[d];
+    }
+  };
+  if (flags & (PV_FC | PV_COPY)) ghosts(flags & PV_FC, flags & PV_FC, flags & PV_COPY);
+  if (flags & (PV_FC | PV_COPY | PV_CORRECT)) __syncthreads();
   const T d0 = dx2 * r0, d1 = dx2 * r1;
-  T lx, hx, ly, hy;
   int it = 1;
-  if (stale) {
+  if (flags & PV_STALE) {
     if (on) {
-      const int ncg = R.lv_nc[li] + 2;
       lx = phi[c1.own - 1];
       hx = phi[c1.own + 1];
       ly = phi[c1.own - ncg];
@@ -1249,51 +1305,30 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, bool s
     }
     __syncthreads();
   }
-  if (!down) return pf;
-  const T inv = T(R.lv_inv2[li]);
-  T e0 = 0, e1 = 0, p0 = 0, p1 = 0;
-  if (on) {
-    p0 = phi[c0.own];
-    p1 = phi[c1.own];
-    vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
-    e0 = r0 - vlap<T>(c0, cyl, lx, hx, ly, hy, p0, inv);
-    vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
-    e1 = r1 - vlap<T>(c1, cyl, lx, hx, ly, hy, p1, inv);
+  if (flags & PV_DOWN) {
+    T e0 = 0, e1 = 0, p0 = 0, p1 = 0;
+    if (on) {
+      p0 = phi[c0.own];
+      p1 = phi[c1.own];
+      vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
+      e0 = r0 - vlap<T>(c0, cyl, lx, hx, ly, hy, p0, inv);
+      vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
+      e1 = r1 - vlap<T>(c1, cyl, lx, hx, ly, hy, p1, inv);
+    }
+    // from the item one row up: its even cell (2ii, 2jj) and odd cell (2ii-1, 2jj)
+    const int hn = nc >> 1;
+    const T e11 = __shfl_down_sync(0xffffffffu, e0, hn), e01 = __shfl_down_sync(0xffffffffu, e1, hn);
+    const T p11 = __shfl_down_sync(0xffffffffu, p0, hn), p01 = __shfl_down_sync(0xffffffffu, p1, hn);
+    if (on && (c0.fl & VF_ODDJ)) {
+      A.tmp[pc] = T(0.25) * (e0 + e1 + e01 + e11);
+      phi[pc] = T(0.25) * (p0 + p1 + p01 + p11);
+    }
+    __syncthreads();
   }
-  const int nc = R.lv_nc[li], hn = nc >> 1, sh = 31 - __clz(nc);
-  // from the item one row up: its even cell (2ii, 2jj) and odd cell (2ii-1, 2jj)
-  const T e11 = __shfl_down_sync(0xffffffffu, e0, hn), e01 = __shfl_down_sync(0xffffffffu, e1, hn);
-  const T p11 = __shfl_down_sync(0xffffffffu, p0, hn), p01 = __shfl_down_sync(0xffffffffu, p1, hn);
-  const int row = (threadIdx.x & (((nc * nc) >> 1) - 1)) >> (sh - 1);
-  if (on && (row & 1) == 0) {
-    A.tmp[pc] = T(0.25) * (e0 + e1 + e01 + e11);
-    phi[pc] = T(0.25) * (p0 + p1 + p01 + p11);
+  if (flags & PV_FILL) {
+    ghosts(true, false, false);
+    __syncthreads();
   }
-  __syncthreads();
-  return pf;
-}
-
-// p_fc with copy_tmp from the cell plans of level index li: the right-hand
-// side of the parent boxes and their tmp = phi, and the level's ghost fill.
-template <class T>
-__device__ __noinline__ PlanFetch p_fc_visit(const RunDev &R, const MGV<T> &M, int li, PlanFetch pf) {
-  const SmArr<T> A = sm_arrays<T>(R);
-  const bool cyl = R.coord == 1;
-  fetch_plan(R, li, cyl, pf);
-  cp_async_wait_all();
-  const T inv = T(R.lv_inv2[li]);
-#pragma unroll
-  for (int p = 0; p < 2; p++) {
-    const VCell<T> c = vcell<T>(p, cyl);
-    if ((c.fl & (VF_ON | VF_PARENT)) != (VF_ON | VF_PARENT)) continue;
-    T lx, hx, ly, hy;
-    vnbrs<T>(A.phi, c, A.v2, lx, hx, ly, hy);
-    const T v = A.phi[c.own];
-    A.rhs[c.own] = vlap<T>(c, cyl, lx, hx, ly, hy, v, inv) + A.tmp[c.own];
-    A.tmp[c.own] = v;
-  }
-  fill_phi_loop(R, M, lvl_info(R, R.min_lvl + li), true);
-  __syncthreads();
   return pf;
 }
 
@@ -1346,11 +1381,11 @@ __device__ __forceinline__ void local_end(int size) {
 // coarse ghost fill + rhs; base: 2 n_cycle_base half-sweeps + ghost fill;
 // up: correction, 4 half-sweeps, ghost fill. In grid mode the levels up to
 // local_top run on one block (the down, base and up phases of those levels
-// are consecutive). after: the level index whose plans the caller's next
+// are consecutive). enter: flags of the first visit (p_enter); after: the level index whose plans the caller's next
 // visit takes (out of range: none).
 template <class T>
 __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, int max_lvl, bool stale_base,
-                                            PlanFetch &pf, int after) {
+                                            PlanFetch &pf, int after, int enter) {
   const int min_lvl = R.min_lvl;
   // grid mode: the levels min_lvl..lc run on block 0 alone (the others wait
   // at the barrier of local_end); each level's code appears once
@@ -1362,25 +1397,25 @@ __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, in
     if (!work) continue;
     const LvlInfo L = lvl_info(R, lvl);
     if (plan_fits(R, M, L)) {
-      pf = p_visit<T>(R, L.li, M.sw_down, false, true, L.li - 1, pf);
+      pf = p_visit<T>(R, L.li, M.sw_down, PV_DOWN | (lvl < max_lvl ? PV_FC : enter), L.li - 1, pf);
     } else {
       for (int it = 1; it <= M.sw_down; it++) p_sweep(R, M, lvl, it, false);
       // no ghost fill of this level (update_coarse, :399-407): its ghost
       // cells are next read after p_fill on the way up
       p_fr(R, M, lvl, false, false);
     }
-    if (plan_fits(R, M, lvl_info(R, lvl - 1))) pf = p_fc_visit<T>(R, M, L.li - 1, pf);
-    else p_fc(R, M, lvl - 1, true);
+    if (!plan_fits(R, M, lvl_info(R, lvl - 1))) p_fc(R, M, lvl - 1, true);
   }
   if (lc == min_lvl) work = local_begin();
   if (work) {
     const LvlInfo L = lvl_info(R, min_lvl);
     if (plan_fits(R, M, L)) {
-      pf = p_visit<T>(R, 0, M.sw_base, stale_base, false, min_lvl < max_lvl ? 1 : after, pf);
+      pf = p_visit<T>(R, 0, M.sw_base, PV_FILL | (stale_base ? PV_STALE : 0) | (min_lvl < max_lvl ? PV_FC : enter),
+                      min_lvl < max_lvl ? 1 : after, pf);
     } else {
       for (int it = 1; it <= M.sw_base; it++) p_sweep(R, M, min_lvl, it, stale_base && it == 1);
+      p_fill(R, M, min_lvl);
     }
-    p_fill(R, M, min_lvl);
   }
   for (int lvl = min_lvl + 1; lvl <= max_lvl; lvl++) {
     if (lvl == lc + 1 && lc >= min_lvl) {
@@ -1389,15 +1424,25 @@ __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, in
     }
     if (!work) continue;
     const LvlInfo L = lvl_info(R, lvl);
-    p_correct(R, M, lvl, false, true);
     if (plan_fits(R, M, L)) {
-      pf = p_visit<T>(R, L.li, M.sw_up, false, false, lvl < max_lvl ? L.li + 1 : after, pf);
+      pf = p_visit<T>(R, L.li, M.sw_up, PV_CORRECT | PV_FILL, lvl < max_lvl ? L.li + 1 : after, pf);
     } else {
+      p_correct(R, M, lvl, false, true);
       for (int it = 1; it <= M.sw_up; it++) p_sweep(R, M, lvl, it, false);
+      p_fill(R, M, lvl);
     }
-    p_fill(R, M, lvl);
   }
   if (lc == max_lvl && lc >= min_lvl) local_end(size);
+}
+
+// The FMG's step to level lvl (mg$D_fas_fmg, m_aX_mg.f90:186-196) before its
+// V-cycle, tmp = phi and the correction from the coarser level: by the
+// V-cycle's first visit (the flags returned) or here.
+template <class T>
+__device__ __forceinline__ int p_enter(const RunDev &R, const MGV<T> &M, int lvl) {
+  if (plan_fits(R, M, lvl_info(R, lvl))) return PV_COPY | (lvl > R.min_lvl ? PV_CORRECT : 0);
+  p_correct(R, M, lvl, true, lvl > R.min_lvl);
+  return 0;
 }
 
 // The FP64 V-cycle is inlined into its caller; the FP32 one (mixed form) is
@@ -1406,13 +1451,13 @@ __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, in
 // of line the FP64 step was 5% slower.
 template <class T>
 __device__ __forceinline__ void p_vcycle(const RunDev &R, const MGV<T> &M, int max_lvl, bool stale_base,
-                                         PlanFetch &pf, int after) {
-  vcycle_body<T>(R, M, max_lvl, stale_base, pf, after);
+                                         PlanFetch &pf, int after, int enter) {
+  vcycle_body<T>(R, M, max_lvl, stale_base, pf, after, enter);
 }
 template <>
 __device__ __noinline__ void p_vcycle<float>(const RunDev &R, const MGV<float> &M, int max_lvl, bool stale_base,
-                                             PlanFetch &pf, int after) {
-  vcycle_body<float>(R, M, max_lvl, stale_base, pf, after);
+                                             PlanFetch &pf, int after, int enter) {
+  vcycle_body<float>(R, M, max_lvl, stale_base, pf, after, enter);
 }
 
 // mg$D_fas_fmg, m_aX_mg.f90:163-202. leaf_rhs: compute the space charge of
@@ -1444,8 +1489,8 @@ __device__ __forceinline__ void p_fmg_in(const RunDev &R, const MGV<T> &M, bool 
       work = true;
     }
     if (!work) continue;
-    p_correct(R, M, lvl, true, lvl > min_lvl);
-    p_vcycle(R, M, lvl, first_call && lvl == min_lvl, pf, lvl + 1 - min_lvl);
+    const int enter = p_enter(R, M, lvl);
+    p_vcycle(R, M, lvl, first_call && lvl == min_lvl, pf, lvl + 1 - min_lvl, enter);
     if (set_residual && lvl == max_lvl) p_residual_all(R, M, lvl);
   }
   if (lc == max_lvl && lc >= min_lvl) local_end(size);
@@ -1591,7 +1636,7 @@ struct VcycleBody {
   __device__ __forceinline__ bool fresh() const { return false; }
   __device__ __forceinline__ void operator()(const RunDev &R, const MGV<double> &M) const {
     PlanFetch pf;
-    p_vcycle(R, M, max_lvl, false, pf, R.nlev);
+    p_vcycle(R, M, max_lvl, false, pf, R.nlev, 0);
     if (set_residual) p_residual_all(R, M, max_lvl);
     if (pf.li >= 0) cp_async_wait_all();
   }
@@ -1790,11 +1835,11 @@ __device__ void p_solve_mixed(const RunDev &R) {
     const int next = pass + 1 < R.mx_n_corr ? (R.mx_fmg ? 0 : R.nlev - 1) : R.nlev;
     if (R.mx_fmg) {
       for (int lvl = R.min_lvl; lvl <= R.max_lvl; lvl++) {
-        p_correct(R, M, lvl, true, lvl > R.min_lvl);
-        p_vcycle(R, M, lvl, false, pf, lvl < R.max_lvl ? lvl + 1 - R.min_lvl : next);
+        const int enter = p_enter(R, M, lvl);
+        p_vcycle(R, M, lvl, false, pf, lvl < R.max_lvl ? lvl + 1 - R.min_lvl : next, enter);
       }
     } else {
-      p_vcycle(R, M, R.max_lvl, false, pf, next);
+      p_vcycle(R, M, R.max_lvl, false, pf, next, 0);
     }
     p_mx_accumulate(R, M);
   }
