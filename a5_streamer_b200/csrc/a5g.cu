@@ -353,12 +353,15 @@ struct BatchSlot {
   Op op;
 };
 
-// The phases, operations and kernels, compiled twice: `blk` for a run on one
-// thread block (the group is the block; thread index, stride and barrier are
-// compile-time; no level-set branches), `grd` for a run on a group of
-// blocks or with level-set boxes (group state in s_grp, grid barriers, the
-// one-block sections of coarse levels, the level-set operators). The host
-// launches the blk kernels unless a run needs grd.
+// The phases, operations and kernels, compiled three times: `blk` for a run
+// on one thread block (the group is the block; thread index, stride and
+// barrier are compile-time; no level-set branches), `clu` for a run on one
+// cluster of blocks (the transport, the field and the staging of a solve on
+// all of them, the shared-memory multigrid on the first), `grd` for a run on
+// a group of blocks or with level-set boxes (group state in s_grp, grid
+// barriers, the one-block sections of coarse levels, the level-set
+// operators). The host launches grd where a run needs it, blk for batches
+// and where many runs share the GPU, clu otherwise (cluster_run).
 namespace blk {
 #define A5G_GRID 0
 #include "a5g_phases.cuh"
@@ -369,6 +372,11 @@ namespace grd {
 #include "a5g_phases.cuh"
 #undef A5G_GRID
 }  // namespace grd
+namespace clu {
+#define A5G_GRID 2
+#include "a5g_phases.cuh"
+#undef A5G_GRID
+}  // namespace clu
 
 // Descriptors of one launch of a5g_step_batch_static passed by value (as
 // kernel parameters, at most SLOT_FILL per launch; 96 x 40 bytes stays under
@@ -405,6 +413,7 @@ constexpr Form kBlockForm = {blk::a5g_run_kernel, blk::a5g_step_kernel, blk::a5g
                              blk::a5g_run_kernel_slots};
 constexpr Form kGroupForm = {grd::a5g_run_kernel, grd::a5g_step_kernel, grd::a5g_step_mixed_kernel,
                              grd::a5g_run_kernel_slots};
+constexpr Form kClusterForm = {clu::a5g_run_kernel, clu::a5g_step_kernel, clu::a5g_step_mixed_kernel, nullptr};
 // Photon absorption does not depend on the form.
 constexpr auto a5g_photon_kernel = blk::a5g_photon_kernel;
 constexpr auto a5g_batch_map_kernel = grd::a5g_batch_map_kernel;
@@ -436,6 +445,7 @@ static int fail(int code, const std::string &msg) {
 
 struct a5g_ctx {
   a5g_params p{};
+  int device = -1;       // counted in g_alive
   cudaStream_t stream = nullptr;
   RunDev h{};
   RunDev *d_run = nullptr;
@@ -732,12 +742,14 @@ static size_t dyn_smem_limit() {
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     size_t stat = 0;
-    constexpr int NF = 10;
+    constexpr int NF = 13;
     cudaFuncAttributes fa[NF];
     const void *fns[NF] = {(const void *)kBlockForm.run,        (const void *)kBlockForm.step,
                            (const void *)kBlockForm.step_mixed, (const void *)kBlockForm.slots,
                            (const void *)kGroupForm.run,        (const void *)kGroupForm.step,
                            (const void *)kGroupForm.step_mixed, (const void *)kGroupForm.slots,
+                           (const void *)kClusterForm.run,      (const void *)kClusterForm.step,
+                           (const void *)kClusterForm.step_mixed,
                            (const void *)a5g_photon_kernel,     (const void *)a5g_batch_map_kernel};
     for (int k = 0; k < NF; k++)
       if (cudaFuncGetAttributes(&fa[k], fns[k]) == cudaSuccess)
@@ -797,6 +809,47 @@ static const Form &batch_form(a5g_ctx *const *ctxs, int n) {
   return kBlockForm;
 }
 
+// A run outside a batch takes a cluster of CLUSTER blocks while the clusters
+// of all runs alive on the device fit its SMs together, one block otherwise.
+// The transport, the field and the staging of a solve spread over the
+// cluster; the shared-memory multigrid stays on its first block, so more
+// blocks gain less and less (8 mm tree, ten steps: 5.64 ms on one block,
+// 5.28, 4.77 and 4.58 on 2, 4 and 8; axisymmetric tree with photons 8.46 and
+// 8.45, 8.13, 7.93). Many runs on streams of their own use the SMs better
+// with one block each: 48 field solves 0.89 ms, as clusters 1.9 ms.
+constexpr int CLUSTER = 8;
+static std::mutex g_alive_mu;
+static int g_alive[256], g_sms[256];  // contexts and SMs per device
+static void count_alive(int dev, int d) {
+  if (dev < 0 || dev >= 256) return;
+  std::lock_guard<std::mutex> lock(g_alive_mu);
+  g_alive[dev] += d;
+  if (!g_sms[dev] && cudaDeviceGetAttribute(&g_sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    g_sms[dev] = 0;
+  }
+}
+static bool cluster_run(const a5g_ctx *c, int code) {
+  if (c->n_cta > 1 || c->h.has_lsf || !grid_op(code) || c->device < 0 || c->device >= 256) return false;
+  std::lock_guard<std::mutex> lock(g_alive_mu);
+  return CLUSTER * g_alive[c->device] <= g_sms[c->device];
+}
+template <class... P, class... A>
+static cudaError_t launch_cluster(void (*fn)(P...), size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(CLUSTER);
+  cfg.blockDim = dim3(NTHR);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = CLUSTER;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
+
 static int launch_smem(a5g_ctx *c, const Op &op, size_t smem) {
   if (!c) return fail(A5G_EINVAL, "null context");
   if (!c->has_tree) return fail(A5G_ESTATE, "no tree uploaded");
@@ -810,6 +863,10 @@ static int launch_smem(a5g_ctx *c, const Op &op, size_t smem) {
     const Op *ops = nullptr;
     void *args[] = {(void *)&run, (void *)&o, (void *)&runs, (void *)&ops};
     CK(cudaLaunchCooperativeKernel((const void *)F.run, dim3(c->n_cta), dim3(NTHR), args, 0, c->stream));
+    return A5G_OK;
+  }
+  if (cluster_run(c, op.code)) {
+    CK(launch_cluster(kClusterForm.run, smem, c->stream, c->d_run, op, nullptr, nullptr));
     return A5G_OK;
   }
   F.run<<<1, NTHR, smem, c->stream>>>(c->d_run, op, nullptr, nullptr);
@@ -959,8 +1016,11 @@ int a5g_create(const a5g_params *p, a5g_ctx **out) {
   }
   a5g_ctx *c = new a5g_ctx();
   c->p = *p;
+  if (cudaGetDevice(&c->device) != cudaSuccess) c->device = -1;
+  count_alive(c->device, 1);
   cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
+    count_alive(c->device, -1);
     delete c;
     return fail(A5G_ECUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
   }
@@ -1078,6 +1138,7 @@ int a5g_destroy(a5g_ctx *c) {
   cudaFree(c->bval);
   if (c->ev_order) cudaEventDestroy(c->ev_order);
   if (c->stream) cudaStreamDestroy(c->stream);
+  count_alive(c->device, -1);
   delete c;
   return A5G_OK;
 }
@@ -1742,6 +1803,13 @@ int a5g_step(a5g_ctx *c, double dt) {
     const RunDev *run = c->d_run;
     void *args[] = {(void *)&run, (void *)&dt, (void *)&deposit};
     CK(cudaLaunchCooperativeKernel(fn, dim3(c->n_cta), dim3(NTHR), args, 0, c->stream));
+    return A5G_OK;
+  }
+  if (cluster_run(c, OP_STEP)) {
+    if (c->precision == A5G_MIXED)
+      CK(launch_cluster(kClusterForm.step_mixed, c->dyn_smem32, c->stream, c->d_run, dt, deposit));
+    else
+      CK(launch_cluster(kClusterForm.step, c->dyn_smem, c->stream, c->d_run, dt, deposit));
     return A5G_OK;
   }
   if (c->precision == A5G_MIXED)

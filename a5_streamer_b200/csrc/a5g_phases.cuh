@@ -1,26 +1,21 @@
 // Phases, operations and kernels of the device path, included by a5g.cu
 // once per execution form, inside namespace blk (A5G_GRID 0: a run on one
-// thread block) and namespace grd (A5G_GRID 1: a run on a group of blocks,
-// and runs with level-set boxes). Everything a phase needs from the group
-// goes through TID(), NTH(), LEAD(), PSYNC() and the one-block sections
-// below, which the block form reduces to threadIdx.x, NTHR and
-// __syncthreads at compile time.
+// thread block), namespace grd (A5G_GRID 1: a run on a group of blocks, and
+// runs with level-set boxes) and namespace clu (A5G_GRID 2: a run on one
+// cluster). Everything a phase needs from the group goes through TID(),
+// NTH(), LEAD(), PSYNC() and the one-block sections below, which the block
+// form reduces to threadIdx.x, NTHR and __syncthreads at compile time (with
+// the group read at run time its steps took 2-4 % longer).
 #ifndef A5G_GRID
 #error "a5g_phases.cuh is included by a5g.cu with A5G_GRID set"
 #endif
 
-constexpr bool kGrid = A5G_GRID != 0;
+constexpr bool kGrid = A5G_GRID == 1, kClu = A5G_GRID == 2, kOne = A5G_GRID == 0;
 
-#if A5G_GRID
-__device__ __forceinline__ int TID() { return s_grp.tid0 + (int)threadIdx.x; }
-__device__ __forceinline__ int NTH() { return s_grp.nth; }
+__device__ __forceinline__ int TID() { return (kOne ? 0 : s_grp.tid0) + (int)threadIdx.x; }
+__device__ __forceinline__ int NTH() { return kOne ? NTHR : s_grp.nth; }
 // the one thread of the group that writes a run's scalars
-__device__ __forceinline__ bool LEAD() { return s_grp.tid0 == 0 && threadIdx.x == 0; }
-#else
-__device__ __forceinline__ int TID() { return (int)threadIdx.x; }
-__device__ __forceinline__ int NTH() { return NTHR; }
-__device__ __forceinline__ bool LEAD() { return threadIdx.x == 0; }
-#endif
+__device__ __forceinline__ bool LEAD() { return (kOne || s_grp.tid0 == 0) && threadIdx.x == 0; }
 
 // Barrier of the run's block group. One thread per block arrives on the
 // group's counter; the last arrival resets it and advances the generation;
@@ -61,10 +56,46 @@ __device__ __noinline__ void grid_sync() {
   __syncthreads();
 }
 
-// Barrier between two phases of a run.
+// Barrier between two phases of a run: of the block, of the cluster, or of
+// the grid's blocks.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 __device__ __forceinline__ void PSYNC() {
-  if (kGrid && s_grp.size > 1) grid_sync();
-  else __syncthreads();
+  if (kOne || s_grp.size == 1) __syncthreads();
+  else if (kGrid) grid_sync();
+  else cluster_sync();
+}
+
+// Cluster form: the shared-memory multigrid is the first block's. The other blocks reach its arrays by their addresses in that block's
+// window (cluster_map), to stage the potential in and out together.
+template <class T>
+__device__ __forceinline__ T *cluster_map(T *p, int rank) {
+  unsigned long long a = reinterpret_cast<unsigned long long>(p), r;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(a), "r"(rank));
+  return reinterpret_cast<T *>(r);
+}
+// A section of the first block alone: true there, where it runs as a group
+// of one; the others wait at the PSYNC that follows alone_end.
+__device__ __forceinline__ bool alone_begin() {
+  if (!kClu) return true;
+  if (s_grp.rank != 0) return false;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_grp.size = 1;
+    s_grp.nth = NTHR;
+  }
+  __syncthreads();
+  return true;
+}
+__device__ __forceinline__ void alone_end(int size) {
+  if (!kClu || s_grp.rank != 0) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_grp.size = size;
+    s_grp.nth = size * NTHR;
+  }
+  __syncthreads();
 }
 
 template <class F>
@@ -1538,12 +1569,13 @@ __device__ void stage_mg(const RunDev &R, const MGV<T> &M, T *g0, T *g1, T *g2, 
     }
     return true;
   };
-  for (int k = threadIdx.x;; k += 2 * NTHR) {
+  const int nth = NTH();
+  for (int k = TID();; k += 2 * nth) {
     int g[2] = {0, 0}, s[2] = {0, 0}, kind[2] = {2, 2};
     bool ok[2];
     ok[0] = slot_at(k, g[0], s[0], kind[0]);
     if (!ok[0]) break;
-    ok[1] = slot_at(k + NTHR, g[1], s[1], kind[1]);
+    ok[1] = slot_at(k + nth, g[1], s[1], kind[1]);
     T v0[2], v1[2], v2[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
@@ -1561,7 +1593,7 @@ __device__ void stage_mg(const RunDev &R, const MGV<T> &M, T *g0, T *g1, T *g2, 
       if (!fresh) (in ? M.tmp[s[u]] : g2[g[u]]) = v2[u];
     }
   }
-  __syncthreads();
+  PSYNC();
 }
 
 
@@ -1660,19 +1692,33 @@ __device__ __forceinline__ void mg_staged(const RunDev &R, const F &body) {
     double *base = g_dsmem + PLAN_DOUBLES + (R.coord == 1 ? WTS_DOUBLES : 0);
     BoxRec *sb = reinterpret_cast<BoxRec *>(base + 3 * S);
     int *spb = reinterpret_cast<int *>(sb + nbx);
-    {
+    const int size = kClu ? s_grp.size : 1;
+    const bool first = !kClu || s_grp.rank == 0;
+    if (first) {
       const int4 *src = reinterpret_cast<const int4 *>(R.sboxes);
       int4 *dst = reinterpret_cast<int4 *>(sb);
       const int n4 = nbx * (int)(sizeof(BoxRec) / sizeof(int4));
       for (int k = threadIdx.x; k < n4; k += NTHR) dst[k] = src[k];
       for (int k = threadIdx.x; k < npb; k += NTHR) spb[k] = R.pbx[k];
     }
-    __syncthreads();
+    PSYNC();  // (and every block of a cluster runs before its window is used)
     MGV<double> M{base, base + S, base + 2 * S, sb, spb, true, R.applied_voltage,
                   4, 4, 2 * R.n_cycle_base};
-    stage_mg(R, M, VAR(R, MP), VAR(R, MR), VAR(R, MT), true, body.fresh());
-    body(R, M);
-    stage_mg(R, M, VAR(R, MP), VAR(R, MR), VAR(R, MT), false, body.fresh());
+    // staged by all blocks of the cluster into the first one's arrays
+    MGV<double> X = M;
+    if (!first) {
+      X.phi = cluster_map(M.phi, 0);
+      X.rhs = cluster_map(M.rhs, 0);
+      X.tmp = cluster_map(M.tmp, 0);
+      X.boxes = R.sboxes;
+    }
+    stage_mg(R, X, VAR(R, MP), VAR(R, MR), VAR(R, MT), true, body.fresh());
+    if (alone_begin()) {
+      body(R, M);
+      alone_end(size);
+    }
+    if (kClu) PSYNC();
+    stage_mg(R, X, VAR(R, MP), VAR(R, MR), VAR(R, MT), false, body.fresh());
   } else {
     MGV<double> M{VAR(R, MP), VAR(R, MR), VAR(R, MT), R.boxes, R.pbx, false, R.applied_voltage,
                   4, 4, 2 * R.n_cycle_base};
@@ -1808,7 +1854,9 @@ __device__ void p_mx_accumulate(const RunDev &R, const MGV<float> &M) {
 // memory: staging them too (with the FP32 arrays) was measured slower, the
 // copies in and out costing more than the residual and accumulation save.
 __device__ void p_solve_mixed(const RunDev &R) {
-  MGV<float> M;
+  MGV<float> M, X;  // X: as the other blocks of a cluster reach M
+  const int size = kClu ? s_grp.size : 1;
+  const bool local = kClu && R.mx_smem > 0;  // the FP32 cycles on the first block
   if (R.mx_smem > 0) {
     const int S = R.mx_smem, nbx = R.bx_off[R.nlev], npb = R.pb_off[R.nlev];
     float *base = reinterpret_cast<float *>(g_dsmem + PLAN_DOUBLES + (R.coord == 1 ? WTS_DOUBLES : 0));
@@ -1822,26 +1870,40 @@ __device__ void p_solve_mixed(const RunDev &R) {
     __syncthreads();
     M = MGV<float>{base, base + S, base + 2 * S, sb, spb, true, 0.0, R.mx_sw_down, R.mx_sw_up,
                    R.mx_sw_base};
+    X = M;
+    if (local) {
+      if (s_grp.rank != 0) {
+        X.phi = cluster_map(M.phi, 0);
+        X.rhs = cluster_map(M.rhs, 0);
+        X.tmp = cluster_map(M.tmp, 0);
+      }
+      PSYNC();  // every block of the cluster runs before its window is used
+    }
   } else {
     const size_t n = (size_t)R.capacity * SLOT;
     M = MGV<float>{R.cc32, R.cc32 + n, R.cc32 + 2 * n, R.boxes, R.pbx, false, 0.0, R.mx_sw_down,
                    R.mx_sw_up, R.mx_sw_base};
+    X = M;
   }
   PlanFetch pf;
   for (int pass = 0; pass < R.mx_n_corr; pass++) {
-    for (int lvl = R.max_lvl; lvl >= R.min_lvl; lvl--) p_mx_residual(R, M, lvl);
+    for (int lvl = R.max_lvl; lvl >= R.min_lvl; lvl--) p_mx_residual(R, X, lvl);
     // the plans that follow the last V-cycle of a pass: those of the next
     // pass's first V-cycle (fetched while the FP64 phases run), or none
     const int next = pass + 1 < R.mx_n_corr ? (R.mx_fmg ? 0 : R.nlev - 1) : R.nlev;
-    if (R.mx_fmg) {
-      for (int lvl = R.min_lvl; lvl <= R.max_lvl; lvl++) {
-        const int enter = p_enter(R, M, lvl);
-        p_vcycle(R, M, lvl, false, pf, lvl < R.max_lvl ? lvl + 1 - R.min_lvl : next, enter);
+    if (!local || alone_begin()) {
+      if (R.mx_fmg) {
+        for (int lvl = R.min_lvl; lvl <= R.max_lvl; lvl++) {
+          const int enter = p_enter(R, M, lvl);
+          p_vcycle(R, M, lvl, false, pf, lvl < R.max_lvl ? lvl + 1 - R.min_lvl : next, enter);
+        }
+      } else {
+        p_vcycle(R, M, R.max_lvl, false, pf, next, 0);
       }
-    } else {
-      p_vcycle(R, M, R.max_lvl, false, pf, next, 0);
+      if (local) alone_end(size);
     }
-    p_mx_accumulate(R, M);
+    if (local) PSYNC();
+    p_mx_accumulate(R, X);
   }
   if (pf.li >= 0) cp_async_wait_all();
 }
@@ -2105,8 +2167,8 @@ __device__ void dt_reductions(const RunDev &R) {
     mx = dmax(red[0][0], mx);
     mn = dmin(red[1][0], mn);
     me = dmax(red[2][0], me);
-    if (kGrid && s_grp.size > 1) {
-      // grid mode: each block's values, combined by the lead after a barrier
+    if (!kOne && s_grp.size > 1) {
+      // several blocks: each block's values, combined by the lead after a barrier
       // (max and min are exact: any order gives the same result)
       double *g = s_grp.red + 4 * s_grp.rank;
       g[0] = mx;
@@ -2114,8 +2176,8 @@ __device__ void dt_reductions(const RunDev &R) {
       g[2] = me;
     }
   }
-  if (kGrid && s_grp.size > 1) {
-    grid_sync();
+  if (!kOne && s_grp.size > 1) {
+    PSYNC();
     if (LEAD()) {
       for (int r = 1; r < s_grp.size; r++) {
         const double *g = s_grp.red + 4 * r;
@@ -2926,12 +2988,22 @@ __device__ __forceinline__ void stage_run(const RunDev *src, RunDev &sR, int siz
   __syncthreads();
 }
 
+// The group of this block in a launch: in the group form all blocks of a
+// single-run launch, in the cluster form the cluster.
+struct Launch {
+  int size, rank;
+};
+__device__ __forceinline__ Launch launch_of(bool batch) {
+  if (kOne || (kGrid && batch)) return Launch{1, 0};
+  return Launch{(int)gridDim.x, (int)blockIdx.x};  // (a cluster launch is one cluster)
+}
+
 // One block per run of a batch, or one run on all blocks of the launch.
 __global__ void __launch_bounds__(NTHR, 1)
 a5g_run_kernel(const RunDev *single, Op single_op, const RunDev *const *runs, const Op *ops) {
   __shared__ RunDev sR;
-  if (runs) stage_run(runs[blockIdx.x], sR, 1, 0);
-  else stage_run(single, sR, (int)gridDim.x, (int)blockIdx.x);
+  const Launch w = launch_of(runs != nullptr);
+  stage_run(runs ? runs[blockIdx.x] : single, sR, w.size, w.rank);
   Op op = runs ? ops[blockIdx.x] : single_op;
   run_op(sR, op);
 }
@@ -2940,7 +3012,8 @@ a5g_run_kernel(const RunDev *single, Op single_op, const RunDev *const *runs, co
 // of its own so that profilers can select the hot launch by name.
 __global__ void __launch_bounds__(NTHR, 1) a5g_step_kernel(const RunDev *run, double dt, int deposit) {
   __shared__ RunDev sR;
-  stage_run(run, sR, (int)gridDim.x, (int)blockIdx.x);
+  const Launch w = launch_of(false);
+  stage_run(run, sR, w.size, w.rank);
   step<false>(sR, dt, deposit != 0);
 }
 
@@ -2948,10 +3021,12 @@ __global__ void __launch_bounds__(NTHR, 1) a5g_step_kernel(const RunDev *run, do
 __global__ void __launch_bounds__(NTHR, 1) a5g_step_mixed_kernel(const RunDev *run, double dt,
                                                                  int deposit) {
   __shared__ RunDev sR;
-  stage_run(run, sR, (int)gridDim.x, (int)blockIdx.x);
+  const Launch w = launch_of(false);
+  stage_run(run, sR, w.size, w.rank);
   step<true>(sR, dt, deposit != 0);
 }
 
+#if A5G_GRID != 2
 // Same work as a5g_run_kernel, with each block's run and operation read from
 // a descriptor table (the fixed array below).
 __global__ void __launch_bounds__(NTHR, 1) a5g_run_kernel_slots(const BatchSlot *slots) {
@@ -2960,8 +3035,9 @@ __global__ void __launch_bounds__(NTHR, 1) a5g_run_kernel_slots(const BatchSlot 
   Op op = slots[blockIdx.x].op;
   run_op(sR, op);
 }
+#endif
 
-#if A5G_GRID
+#if A5G_GRID == 1
 // A device-driven batch whose members take several blocks each (the
 // members' a5g_set_ctas): block b runs operation ops[k] of run k as rank r of
 // its run's group of m blocks, gmap[3 b ..] = {k, r, m}; one cooperative
