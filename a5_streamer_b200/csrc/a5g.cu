@@ -446,6 +446,8 @@ static int fail(int code, const std::string &msg) {
 struct a5g_ctx {
   a5g_params p{};
   int device = -1;       // counted in g_alive
+  BatchSlot *batch_tbl = nullptr;  // descriptors of a5g_step_batch with this run first: 2 batch_cap entries
+  int batch_cap = 0;
   cudaStream_t stream = nullptr;
   RunDev h{};
   RunDev *d_run = nullptr;
@@ -1102,6 +1104,7 @@ int a5g_create(const a5g_params *p, a5g_ctx **out) {
 int a5g_destroy(a5g_ctx *c) {
   if (!c) return A5G_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
+  cudaFree(c->batch_tbl);
   cudaFree(c->d_run);
   cudaFree(c->cc);
   cudaFree(c->fx);
@@ -1922,6 +1925,18 @@ static int batch_order_out(a5g_ctx *const *ctxs, int n, cudaStream_t s, cudaEven
   return A5G_OK;
 }
 
+// The descriptors of a launch into a table on the device, by kernel parameters.
+static int static_fill(BatchSlot *table, const BatchSlot *slots, int n, cudaStream_t s) {
+  for (int k0 = 0; k0 < n; k0 += SLOT_FILL) {
+    const int m = std::min(SLOT_FILL, n - k0);
+    SlotChunk chunk;
+    std::memset(&chunk, 0, sizeof(chunk));
+    std::memcpy(chunk.s, slots + k0, (size_t)m * sizeof(BatchSlot));
+    a5g_fill_slots_kernel<<<1, 128, 0, s>>>(table + k0, chunk, m);
+    CK(cudaGetLastError());
+  }
+  return A5G_OK;
+}
 int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts) {
   if (!ctxs || !dts || n < 1) return fail(A5G_EINVAL, "bad batch");
   for (int k = 0; k < n; k++) {
@@ -1930,13 +1945,12 @@ int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts) {
     if (!(dts[k] > 0)) return fail(A5G_EINVAL, "dt must be > 0");
   }
   a5g_ctx *c0 = ctxs[0];
-  std::vector<const RunDev *> rp(n);
-  std::vector<Op> ops(2 * n);
+  std::vector<BatchSlot> slots(2 * (size_t)n);  // the steps, then the photon sources
   bool any_ph = false;
   int max_team = 0;
   size_t ph_smem = 0;
   for (int k = 0; k < n; k++) {
-    rp[k] = ctxs[k]->d_run;
+    slots[k].run = slots[n + k].run = ctxs[k]->d_run;
     const bool ph = ctxs[k]->p.photoi_enabled != 0;
     if (ph) {
       int r = ph_ready(ctxs[k]);
@@ -1949,34 +1963,41 @@ int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts) {
       int r = mx_ready(ctxs[k]);
       if (r) return r;
     }
-    ops[k] = mkop(ctxs[k]->precision == A5G_MIXED ? OP_STEP_MIXED : OP_STEP, ph ? 1 : 0, 0, dts[k]);
-    ops[n + k] = ph ? mkop(OP_PH_SOURCE, 1, 0, dts[k]) : mkop(OP_NOP);
+    slots[k].op = mkop(ctxs[k]->precision == A5G_MIXED ? OP_STEP_MIXED : OP_STEP, ph ? 1 : 0, 0, dts[k]);
+    slots[n + k].op = ph ? mkop(OP_PH_SOURCE, 1, 0, dts[k]) : mkop(OP_NOP);
   }
   // the batch runs on c0's stream after the other members' queued work
   int ro = batch_order_in(ctxs, n, c0->stream);
   if (ro) return ro;
-  const RunDev **d_rp = nullptr;
-  Op *d_ops = nullptr;
-  CK(cudaMallocAsync((void **)&d_rp, n * sizeof(void *), c0->stream));
-  CK(cudaMallocAsync((void **)&d_ops, 2 * n * sizeof(Op), c0->stream));
-  CK(cudaMemcpyAsync(d_rp, rp.data(), n * sizeof(void *), cudaMemcpyHostToDevice, c0->stream));
-  CK(cudaMemcpyAsync(d_ops, ops.data(), 2 * n * sizeof(Op), cudaMemcpyHostToDevice, c0->stream));
+  // The descriptors go as kernel parameters into a table that c0 keeps: the
+  // launches of later calls on c0's stream come after this call's, so the
+  // table can be written again, and a call neither allocates nor copies (two
+  // stream-ordered allocations a call, given back to the system at every
+  // synchronisation, made single calls tens of milliseconds long).
+  if (c0->batch_cap < n) {
+    CK(cudaStreamSynchronize(c0->stream));
+    cudaFree(c0->batch_tbl);
+    c0->batch_tbl = nullptr;
+    c0->batch_cap = 0;
+    CK(cudaMalloc((void **)&c0->batch_tbl, 2 * (size_t)n * sizeof(BatchSlot)));
+    c0->batch_cap = n;
+  }
+  const int rf = static_fill(c0->batch_tbl, slots.data(), any_ph ? 2 * n : n, c0->stream);
+  if (rf) return rf;
   size_t dyn = 0;
   for (int k = 0; k < n; k++) dyn = std::max(dyn, std::max(ctxs[k]->dyn_smem, step_smem(ctxs[k])));
   const Form &F = batch_form(ctxs, n);
   if (any_ph) {
     // photon sources of every member with photoionization (the others run
     // an operation that does nothing here), then the absorption
-    F.run<<<n, NTHR, dyn, c0->stream>>>(nullptr, Op{}, d_rp, d_ops + n);
+    F.slots<<<n, NTHR, dyn, c0->stream>>>(c0->batch_tbl + n);
     CK(cudaGetLastError());
     dim3 grid((unsigned)((max_team + PH_THREADS - 1) / PH_THREADS), (unsigned)n);
-    a5g_photon_kernel<<<grid, PH_THREADS, ph_smem, c0->stream>>>(nullptr, d_rp, nullptr, (int)ph_smem);
+    a5g_photon_kernel<<<grid, PH_THREADS, ph_smem, c0->stream>>>(nullptr, nullptr, c0->batch_tbl, (int)ph_smem);
     CK(cudaGetLastError());
   }
-  F.run<<<n, NTHR, dyn, c0->stream>>>(nullptr, Op{}, d_rp, d_ops);
+  F.slots<<<n, NTHR, dyn, c0->stream>>>(c0->batch_tbl);
   CK(cudaGetLastError());
-  CK(cudaFreeAsync(d_rp, c0->stream));
-  CK(cudaFreeAsync(d_ops, c0->stream));
   // the members' own streams continue after the batch
   return batch_order_out(ctxs, n, c0->stream, c0->ev_order);
 }
@@ -1989,17 +2010,6 @@ static BatchSlot *g_static_dev[256] = {};
 // Writes the n descriptors of one launch into the fixed table on stream s,
 // as kernel parameters of fill launches (ordered with the launch that reads
 // them like any other work of the stream).
-static int static_fill(BatchSlot *table, const BatchSlot *slots, int n, cudaStream_t s) {
-  for (int k0 = 0; k0 < n; k0 += SLOT_FILL) {
-    const int m = std::min(SLOT_FILL, n - k0);
-    SlotChunk chunk;
-    std::memset(&chunk, 0, sizeof(chunk));
-    std::memcpy(chunk.s, slots + k0, (size_t)m * sizeof(BatchSlot));
-    a5g_fill_slots_kernel<<<1, 128, 0, s>>>(table + k0, chunk, m);
-    CK(cudaGetLastError());
-  }
-  return A5G_OK;
-}
 
 int a5g_step_batch_static(a5g_ctx **ctxs, int n, const double *dts) {
   if (!ctxs || !dts || n < 1) return fail(A5G_EINVAL, "bad batch");
