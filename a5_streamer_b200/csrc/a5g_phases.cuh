@@ -2879,38 +2879,45 @@ __device__ void tree_reduce(const RunDev &R, int iv, int kind, int team) {
 // field solves by defect correction around an FP32 multigrid (p_solve_mixed);
 // densities, the space charge, the potential, the field and the step size
 // stay in FP64.
+// The old densities saved at the start of a step.
+__device__ __forceinline__ void save_old(const RunDev &R) {
+  const size_t n = (size_t)R.capacity * SLOT;
+  const double *e = VAR(R, I_ELEC), *pi = VAR(R, I_PION);
+  double *eo = VAR(R, I_ELEC_OLD), *po = VAR(R, I_PION_OLD);
+  // two slots per thread and round, all loads before the stores
+  const size_t nth = NTH();
+  for (size_t k = TID(); k < n; k += 2 * nth) {
+    const size_t k1 = k + nth;
+    const bool two = k1 < n;
+    const double a0 = e[k], b0 = pi[k], a1 = two ? e[k1] : 0.0, b1 = two ? pi[k1] : 0.0;
+    eo[k] = a0;
+    po[k] = b0;
+    if (two) {
+      eo[k1] = a1;
+      po[k1] = b1;
+    }
+  }
+  PSYNC();
+}
+// One forward-Euler stage of the densities (without its field solve).
+template <class T>
+__device__ __forceinline__ void transport(const RunDev &R, double dt) {
+  fluxes_koren<T>(R, dt);
+  PSYNC();
+  consistent_fluxes(R);
+  PSYNC();
+  update_solution<T>(R, dt);
+  PSYNC();
+  p_restrict(R, I_ELEC, I_PION);
+  p_gc_den(R, I_ELEC, I_PION, true);
+}
 template <bool MIXED>
 __device__ void step(const RunDev &R, double dt, bool deposit) {
   if (deposit) ph_deposit(R);
-  {
-    const size_t n = (size_t)R.capacity * SLOT;
-    const double *e = VAR(R, I_ELEC), *pi = VAR(R, I_PION);
-    double *eo = VAR(R, I_ELEC_OLD), *po = VAR(R, I_PION_OLD);
-    // two slots per thread and round, all loads before the stores
-    const size_t nth = NTH();
-    for (size_t k = TID(); k < n; k += 2 * nth) {
-      const size_t k1 = k + nth;
-      const bool two = k1 < n;
-      const double a0 = e[k], b0 = pi[k], a1 = two ? e[k1] : 0.0, b1 = two ? pi[k1] : 0.0;
-      eo[k] = a0;
-      po[k] = b0;
-      if (two) {
-        eo[k1] = a1;
-        po[k1] = b1;
-      }
-    }
-    PSYNC();
-  }
+  save_old(R);
   using T = typename std::conditional<MIXED, float, double>::type;
   for (int stage = 1; stage <= 2; stage++) {
-    fluxes_koren<T>(R, dt);
-    PSYNC();
-    consistent_fluxes(R);
-    PSYNC();
-    update_solution<T>(R, dt);
-    PSYNC();
-    p_restrict(R, I_ELEC, I_PION);
-    p_gc_den(R, I_ELEC, I_PION, true);
+    transport<T>(R, dt);
     if (stage == 1) {
       if (MIXED) p_compute_fld_mixed(R);
       else p_compute_fld(R, false);
@@ -2949,6 +2956,16 @@ __device__ void run_op(const RunDev &R, const Op &op) {
       if (op.i1 && LEAD()) R.blk[1] = R.blk[1] + dt;
       break;
     }
+#if A5G_GRID == 1
+    case OP_STAGE:
+      // the transport of stage i0 of a step whose field solves are launches
+      // of their own (a5g_uniform.cu); i1: the mixed form
+      if (op.i0 == 1) save_old(R);
+      if (op.i1) transport<float>(R, op.d0);
+      else transport<double>(R, op.d0);
+      if (op.i0 == 2) average_dens(R);
+      break;
+#endif
     case OP_BLOCK_DT: block_dt(R); break;
     case OP_COMPUTE_FLD_MIXED: p_compute_fld_mixed(R); break;
     case OP_PH_SOURCE:

@@ -337,7 +337,9 @@ int a5g_set_level_set(a5g_ctx *ctx, const double *lsf, const double *bval);
  * thousand cells, but uses one SM. With n_cta > 1 every operation of the run
  * (steps, field solves, reductions, flags, prolongation) is one cooperative
  * launch of n_cta co-resident blocks that share each phase's items, with a
- * grid barrier between phases; results are identical to one block. Each
+ * grid barrier between phases; results are identical to one block. (Where
+ * every level of a Cartesian run's tree is complete, the field solves with a
+ * guess run as kernels of their own on the whole GPU.) Each
  * barrier wait is bounded by wait_cycles SM clock cycles (< 0: the default,
  * A5G_DEFAULT_WAIT_CYCLES); a wait that runs out makes the launch return
  * early and the next synchronising call report A5G_TIMEOUT (0 makes every
