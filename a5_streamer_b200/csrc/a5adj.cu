@@ -28,6 +28,7 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 namespace {
@@ -666,6 +667,132 @@ static std::string build_tape(const Topo &T, const Ix &X, int n_base, Tape &tp, 
   return "";
 }
 
+// The transposed multigrid segments in gather form, for the adjoint vector
+// of the multigrid's three variables in shared memory. A phase of the tape
+// maps each row's value lam[d] to its sources, lam[s] += c lam[d], then lam[d]
+// = self lam[d]; no phase reads an entry it writes, so per source s the sum
+// over its rows can be formed by one thread, in the rows' order, without
+// atomics. Sources come in three classes, those of one term, of up to 4 and of
+// up to 16, missing terms being zeros of an entry that stays zero. A term is
+// its row's entry (15 bits) and the index of its coefficient (8 bits; 33
+// different ones on the 8 mm tree), and the source sits in the spare bits of
+// the first two terms, so a thread's part of a phase is a few vector loads at
+// places it knows in advance. The applied voltage, a source of every wall row,
+// has a list of its own.
+constexpr int JPL = 16;     // most terms of one source
+constexpr int JCO = 256;    // most distinct coefficients
+constexpr int JIX = 1 << 15;  // entries
+struct __align__(16) JRec {
+  int a, b, c, row, v;                   // offsets: sources by class, rows, voltage terms
+  unsigned short na, nb, nc, nr, nv, pad;  // numbers of these (rows: self != 1)
+};
+static_assert(sizeof(JRec) == 32, "JRec layout");
+struct Jagged {
+  int S = 0;                 // entries per variable
+  std::vector<int> gmap;     // entry -> offset in a variable's global slots
+  std::vector<JRec> rec;     // phases in the order of the reverse pass
+  int first[2] = {}, n[2] = {};  // SEG_FMG, SEG_FMG1
+  std::vector<uint2> one;    // term, source
+  std::vector<uint4> four;   // 4 terms
+  std::vector<uint4> many;   // 16 terms, 4 a piece
+  std::vector<uint32_t> row, v;
+  std::vector<double> coef;
+};
+// false: the segments touch something else, or a source has too many terms
+// or an index too many bits (the atomic form serves then).
+static bool build_jagged(const Topo &T, const Ix &X, const Tape &tp, const int seg[N_SEG + 1], Jagged &J) {
+  std::vector<int> at(X.total, -1);
+  const int var[3] = {I_PHI, I_RHS, I_FLD};
+  int S = 0;
+  for (int id = 1; id <= T.max_id; id++)
+    if (T.b[id].in_use) S += (T.b[id].nc + 2) * (T.b[id].nc + 2);
+  J.S = S;
+  if (3 * S + 1 > JIX) return false;
+  for (int id = 1, k = 0; id <= T.max_id; id++) {
+    if (!T.b[id].in_use) continue;
+    const int n = (T.b[id].nc + 2) * (T.b[id].nc + 2);
+    for (int q = 0; q < n; q++, k++) {
+      J.gmap.push_back(id * SLOT + q);
+      for (int v = 0; v < 3; v++) at[((size_t)var[v] * X.cap + id) * SLOT + q] = v * S + k;
+    }
+  }
+  std::unordered_map<uint64_t, int> known;
+  struct Last { uint64_t u; int i; } last[64];  // the coefficients seen last, by some bits
+  for (auto &l : last) l.i = -1;
+  auto word = [&](int d, double c) {
+    uint64_t u;
+    memcpy(&u, &c, sizeof u);
+    Last &l = last[(u ^ u >> 44 ^ u >> 52) & 63];
+    if (l.i < 0 || l.u != u) {
+      l.u = u;
+      l.i = known.emplace(u, (int)J.coef.size()).first->second;
+      if (l.i == (int)J.coef.size()) J.coef.push_back(c);
+    }
+    return (uint32_t)d | (uint32_t)l.i << 15;
+  };
+  const uint32_t none = word(3 * S, 0.0);
+  std::vector<int> row_of(3 * (size_t)S, -1);  // phase in which an entry is a row
+  std::vector<int> cnt(3 * (size_t)S, 0), used;
+  std::vector<uint32_t> terms(3 * (size_t)S * JPL);
+  for (int w = 0; w < 2; w++) {
+    const int p0 = seg[w ? SEG_FMG1 : SEG_FMG], p1 = seg[(w ? SEG_FMG1 : SEG_FMG) + 1];
+    J.first[w] = (int)J.rec.size();
+    J.n[w] = p1 - p0;
+    for (int p = p1 - 1; p >= p0; p--) {
+      JRec R{};
+      R.a = (int)J.one.size();
+      R.b = (int)J.four.size();
+      R.c = (int)J.many.size();
+      R.row = (int)J.row.size();
+      R.v = (int)J.v.size();
+      used.clear();
+      for (int r = tp.phase_row[p]; r < tp.phase_row[p + 1]; r++) {
+        const int d = at[tp.row_d[r]];
+        if (d < 0 || row_of[d] == p) return false;
+        row_of[d] = p;
+        for (int t = tp.row_term[r]; t < tp.row_term[r + 1]; t++) {
+          const uint32_t x = word(d, tp.term_c[t]);
+          if (tp.term_s[t] == X.v) {
+            J.v.push_back(x);
+            continue;
+          }
+          const int q = at[tp.term_s[t]];
+          if (q < 0 || cnt[q] == JPL) return false;
+          if (cnt[q] == 0) used.push_back(q);
+          terms[(size_t)q * JPL + cnt[q]++] = x;
+        }
+        if (tp.row_self[r] != 1.0) J.row.push_back(word(d, tp.row_self[r]));
+      }
+      if (J.coef.size() > JCO) return false;
+      for (int q : used) {
+        if (row_of[q] == p) return false;  // read and written: not one gather
+        uint32_t *t = &terms[(size_t)q * JPL];
+        if (cnt[q] == 1) {
+          J.one.push_back(make_uint2(t[0], (uint32_t)q));
+        } else {
+          const int m = cnt[q] <= 4 ? 4 : JPL;
+          for (int k = cnt[q]; k < m; k++) t[k] = none;
+          t[0] |= (uint32_t)q << 23;
+          t[1] |= (uint32_t)(q >> 9) << 23;
+          for (int k = 0; k < m; k += 4)
+            (m == 4 ? J.four : J.many).push_back(make_uint4(t[k], t[k + 1], t[k + 2], t[k + 3]));
+        }
+        cnt[q] = 0;
+      }
+      const size_t na = J.one.size() - R.a, nb = J.four.size() - R.b, nc = (J.many.size() - R.c) / 4,
+                   nr = J.row.size() - R.row, nv = J.v.size() - R.v;
+      if (std::max({na, nb, nc, nr, nv}) > 65535) return false;
+      R.na = (unsigned short)na;
+      R.nb = (unsigned short)nb;
+      R.nc = (unsigned short)nc;
+      R.nr = (unsigned short)nr;
+      R.nv = (unsigned short)nv;
+      J.rec.push_back(R);
+    }
+  }
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // Device side
 struct DBox {
@@ -695,6 +822,16 @@ struct AdjArgs {
   const double *tbl;           // n_rows x 4 column-major
   int tbl_rows, pad;
   double tbl_xmin, tbl_inv_dx;
+  // multigrid segments in gather form (jS 0: not used)
+  int jS, jfirst[2], jn[2];
+  const int *jmap;
+  const JRec *jrec;
+  const uint2 *jone;
+  const uint4 *jfour, *jmany;
+  const uint32_t *jrow, *jv;
+  const double *jcoef;
+  int jnco;
+  size_t vidx;
 };
 
 // Intermediate fields of one step (device pointers): cell blocks of
@@ -741,6 +878,128 @@ __device__ void tape_rev(const AdjArgs &A, int p0, int p1) {
   }
 }
 __device__ __forceinline__ void seg_rev(const AdjArgs &A, int s) { tape_rev(A, A.seg[s], A.seg[s + 1]); }
+
+// A segment of one phase, over many blocks.
+__global__ void __launch_bounds__(256) adj_rows_kernel(const __grid_constant__ AdjArgs A, int r0, int r1) {
+  for (int r = r0 + blockIdx.x * blockDim.x + threadIdx.x; r < r1; r += gridDim.x * blockDim.x) {
+    const uint32_t d = A.row_d[r];
+    const double lam = A.lam[d];
+    if (lam != 0.0) {
+      for (int t = A.row_term[r]; t < A.row_term[r + 1]; t++)
+        atomicAdd(&A.lam[A.term_s[t]], A.term_c[t] * lam);
+      A.lam[d] = A.row_self[r] * lam;
+    }
+  }
+}
+
+// The multigrid's transposed phases in gather form, w 0: SEG_FMG, 1:
+// SEG_FMG1, on the adjoints of phi, rhs and tmp in shared memory. What bounds
+// a phase of a few hundred rows is the latency of its chain, so the tape's
+// part of it is fetched two phases ahead into registers and its record five
+// ahead; the phase itself is a shared-memory round trip and two barriers.
+// 576 threads: one source of each small class each covers nearly every phase
+// of the 8 mm tree (399 phases), and what is prefetched has registers. The
+// vector in L2 with FP64 atomics took 1,000 us, 10-byte terms by jagged
+// diagonals with 1,024 threads 1,360 (spills) and with 576 586 us, this form
+// 390 us (31 % of the issue slots; a phase is 1.0 us).
+constexpr int FTHR = 576;
+struct JNext {  // one thread's part of a phase: a source of each small class, a row, a voltage term
+  uint4 four;
+  uint2 one;
+  uint32_t row, v;
+  int4 rec;  // threads 0 and 1: half of a later record
+};
+__device__ __forceinline__ void fmg_fetch(const AdjArgs &A, const JRec &R, JNext &P) {
+  const int tid = threadIdx.x;
+  if (tid < R.nb) P.four = A.jfour[R.b + tid];
+  if (tid < R.na) P.one = A.jone[R.a + tid];
+  if (tid < R.nr) P.row = A.jrow[R.row + tid];
+  if (tid < R.nv) P.v = A.jv[R.v + tid];
+}
+__global__ void __launch_bounds__(FTHR, 1) adj_fmg_kernel(const __grid_constant__ AdjArgs A, int w) {
+  extern __shared__ double s_lam[];
+  __shared__ JRec ring[4];
+  __shared__ double vsum[FTHR / 32];
+  const int S = A.jS, tid = threadIdx.x, n = A.jn[w];
+  double *sl = s_lam, *co = s_lam + 3 * S + 1;
+  double *g[3] = {A.lam + (size_t)I_PHI * A.cap * SLOT, A.lam + (size_t)I_RHS * A.cap * SLOT,
+                  A.lam + (size_t)I_FLD * A.cap * SLOT};
+  for (int k = tid; k < S; k += FTHR) {
+    const int m = A.jmap[k];
+    const double a = g[0][m], b = g[1][m], c = g[2][m];
+    sl[k] = a;
+    sl[S + k] = b;
+    sl[2 * S + k] = c;
+  }
+  for (int k = tid; k < A.jnco; k += FTHR) co[k] = A.jcoef[k];
+  if (tid == 0) sl[3 * S] = 0;  // the entry of missing terms
+  // records 0 to 2 in the ring, 3 and 4 on their way
+  const int4 *rsrc = reinterpret_cast<const int4 *>(A.jrec + A.jfirst[w]);
+  int4 *rdst = reinterpret_cast<int4 *>(ring);
+  if (tid < 6 && tid < 2 * n) rdst[tid] = rsrc[tid];
+  JNext P0, P1;
+  if (tid < 2 && 3 < n) P0.rec = rsrc[2 * 3 + tid];
+  if (tid < 2 && 4 < n) P1.rec = rsrc[2 * 4 + tid];
+  __syncthreads();
+  double vacc = 0;
+  auto term = [&](uint32_t x) { return co[x >> 15 & 0xff] * sl[x & (JIX - 1)]; };
+  auto quad = [&](const uint4 &x) { return term(x.x) + term(x.y) + term(x.z) + term(x.w); };
+  auto source = [&](const uint4 &x) { return x.x >> 23 | x.y >> 23 << 9; };
+  auto phase = [&](int p, JNext &P) {
+    const JRec &R = ring[p & 3];
+    // (no source is a row of this phase: the order of the classes is free)
+    for (int q = FTHR - 1 - tid; q < R.nc; q += FTHR) {
+      const uint4 x0 = A.jmany[R.c + 4 * q], x1 = A.jmany[R.c + 4 * q + 1], x2 = A.jmany[R.c + 4 * q + 2],
+                  x3 = A.jmany[R.c + 4 * q + 3];
+      sl[source(x0)] += quad(x0) + quad(x1) + quad(x2) + quad(x3);
+    }
+    if (tid < R.nb) sl[source(P.four)] += quad(P.four);
+    if (tid < R.na) sl[P.one.y] += term(P.one.x);
+    for (int q = tid + FTHR; q < R.nb; q += FTHR) {
+      const uint4 x = A.jfour[R.b + q];
+      sl[source(x)] += quad(x);
+    }
+    for (int q = tid + FTHR; q < R.na; q += FTHR) {
+      const uint2 x = A.jone[R.a + q];
+      sl[x.y] += term(x.x);
+    }
+    if (tid < R.nv) vacc += term(P.v);
+    for (int q = tid + FTHR; q < R.nv; q += FTHR) vacc += term(A.jv[R.v + q]);
+    const bool mine = tid < R.nr;
+    const uint32_t row = P.row;
+    if (tid < 2 && p + 3 < n) rdst[2 * ((p + 3) & 3) + tid] = P.rec;
+    if (p + 2 < n) fmg_fetch(A, ring[(p + 2) & 3], P);
+    if (tid < 2 && p + 5 < n) P.rec = rsrc[2 * (p + 5) + tid];
+    __syncthreads();
+    if (mine) sl[row & (JIX - 1)] = term(row);
+    for (int q = tid + FTHR; q < R.nr; q += FTHR) {
+      const uint32_t x = A.jrow[R.row + q];
+      sl[x & (JIX - 1)] = term(x);
+    }
+    __syncthreads();
+  };
+  if (0 < n) fmg_fetch(A, ring[0], P0);
+  if (1 < n) fmg_fetch(A, ring[1], P1);
+#pragma unroll 1
+  for (int p = 0; p < n; p += 2) {
+    phase(p, P0);
+    if (p + 1 < n) phase(p + 1, P1);
+  }
+  for (int k = tid; k < S; k += FTHR) {
+    const int m = A.jmap[k];
+    g[0][m] = sl[k];
+    g[1][m] = sl[S + k];
+    g[2][m] = sl[2 * S + k];
+  }
+  for (int o = 16; o > 0; o >>= 1) vacc += __shfl_xor_sync(0xffffffffu, vacc, o);
+  if ((tid & 31) == 0) vsum[tid >> 5] = vacc;
+  __syncthreads();
+  if (tid == 0) {
+    double v = 0;
+    for (int k = 0; k < FTHR / 32; k++) v += vsum[k];
+    A.lam[A.vidx] += v;
+  }
+}
 
 // Table location (fosito/m_lookup_table.f90:117-124): low row (1-based),
 // weight of the low row, and d(lookup)/dx per unit row difference
@@ -870,7 +1129,7 @@ __device__ void adj_fluxes(const AdjArgs &A, double *s_tbl, const double *ne, co
   const int per = 2 * (NC + 1) * NC;
   double *lam_ne = A.lam + (size_t)I_ELEC * A.cap * SLOT;
   double *lam_E = A.lam + (size_t)I_FLD * A.cap * SLOT;
-  for (int q = threadIdx.x; q < nb_all * per; q += blockDim.x) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nb_all * per; q += gridDim.x * blockDim.x) {
     int id, r;
     leaf_item(A, q, per, id, r);
     const DBox &m = A.box[id];
@@ -998,7 +1257,7 @@ __device__ void adj_update(const AdjArgs &A, double *s_tbl, const double *F, con
   const double *lam_ne = A.lam + (size_t)I_ELEC * A.cap * SLOT;
   const double *lam_ni = A.lam + (size_t)I_PION * A.cap * SLOT;
   double *lam_E = A.lam + (size_t)I_FLD * A.cap * SLOT;
-  for (int q = threadIdx.x; q < nb_all * per; q += blockDim.x) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nb_all * per; q += gridDim.x * blockDim.x) {
     int id, r;
     leaf_item(A, q, per, id, r);
     const DBox &m = A.box[id];
@@ -1042,7 +1301,7 @@ __device__ void adj_fld_norm(const AdjArgs &A, const double *ff) {
   const int n = n_ids(A);
   const int per = NC * NC;
   double *lam_E = A.lam + (size_t)I_FLD * A.cap * SLOT;
-  for (int q = threadIdx.x; q < n * per; q += blockDim.x) {
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n * per; q += gridDim.x * blockDim.x) {
     const int b = q / per, r = q - b * per;
     const int id = A.lists[A.lv_ids[0] + b];
     const int nc = A.box[id].nc;
@@ -1069,19 +1328,22 @@ __device__ void adj_fld_norm(const AdjArgs &A, const double *ff) {
 // (afivo/src/m_aX_gc.f90:28-68, 190-330). Levels in reverse order: a level's
 // fill reads the coarser level's ghost cells. X is the variable after the
 // fill (the limiter's branch).
-__device__ void adj_gc_lim(const AdjArgs &A, int iv, const double *X) {
+// Two variables at a time.
+__device__ void adj_gc_lim(const AdjArgs &A, int iv0, const double *X0, int iv1, const double *X1) {
   const double sixth = 1 / 6.0, third = 1 / 3.0;
-  double *lam = A.lam + (size_t)iv * A.cap * SLOT;
   for (int li = A.nlev - 1; li >= 0; li--) {
     const int n = A.lv_ids[li + 1] - A.lv_ids[li];
     const int *ids = A.lists + A.lv_ids[li];
     const int per = 4 * NC;
-    for (int q = threadIdx.x; q < n * per; q += blockDim.x) {
+    for (int q2 = threadIdx.x; q2 < 2 * n * per; q2 += blockDim.x) {
+      const int second = q2 >= n * per, q = second ? q2 - n * per : q2;
       const int b = q / per, r = q - b * per;
       const int id = ids[b];
       const DBox &m = A.box[id];
       const int nc = m.nc, g2 = nc + 2;
       if (r >= 4 * nc) continue;
+      const double *X = second ? X1 : X0;
+      double *lam = A.lam + (size_t)(second ? iv1 : iv0) * A.cap * SLOT;
       const int nb = r / nc, k = r % nc + 1, dim = nb >> 1;
       int gi, gj;
       if (dim == 0) { gi = (nb & 1) ? nc + 1 : 0; gj = k; }
@@ -1146,55 +1408,45 @@ __device__ void adj_gc_lim(const AdjArgs &A, int iv, const double *X) {
   }
 }
 
-// compute_fld's transpose: ghost cells of |E|, the cell |E|, the faces, the
-// FMG, the space charge.
-__device__ void adj_compute_fld(const AdjArgs &A, const double *ff, int fmg_seg) {
-  seg_rev(A, SEG_GCFLD);
-  adj_fld_norm(A, ff);
-  seg_rev(A, SEG_FACES);
-  seg_rev(A, fmg_seg);
-  seg_rev(A, SEG_RHS);
-}
-
 __device__ void zero_smem_tbl(double *s_tbl, int n) {
   for (int k = threadIdx.x; k < n; k += blockDim.x) s_tbl[k] = 0;
   __syncthreads();
 }
 __device__ void flush_smem_tbl(const AdjArgs &A, const double *s_tbl, int n) {
   __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) A.lam_tbl[k] += s_tbl[k];
+  for (int k = threadIdx.x; k < n; k += blockDim.x)
+    if (s_tbl[k] != 0.0) atomicAdd(&A.lam_tbl[k], s_tbl[k]);
 }
 
-// The reverse of one full time step (src/streamer_2d.f90:93-128).
-__global__ void __launch_bounds__(ATHR) adj_step_kernel(AdjArgs A, StepSnap S) {
+// The reverse of one full time step (src/streamer_2d.f90:93-128): operations
+// of several dependent phases on one block, the multigrid solves
+// (adj_fmg_kernel), and those without dependencies inside, on many blocks. The
+// cells' and the faces' reverse (adj_update, adj_fluxes) is bound by its
+// accumulation of table gradients -- most cells meet in a few rows of the
+// table, and a block's FP64 sums in shared memory take turns there -- which
+// blocks of 128 threads spread. (All of a step but its multigrid on one block
+// of 1,024 threads: 1,190 us on the 8 mm tree; now 240.)
+__global__ void __launch_bounds__(ATHR) adj_seg_kernel(const __grid_constant__ AdjArgs A, int seg) {
+  seg_rev(A, seg);
+}
+__global__ void __launch_bounds__(ATHR) adj_gc_kernel(const __grid_constant__ AdjArgs A, const double *Xi,
+                                                      const double *Xe) {
+  adj_gc_lim(A, I_PION, Xi, I_ELEC, Xe);
+  seg_rev(A, SEG_RSTR);
+}
+__global__ void __launch_bounds__(128) adj_norm_kernel(const __grid_constant__ AdjArgs A, const double *ff) {
+  adj_fld_norm(A, ff);
+}
+constexpr int BTHR = 128;
+template <int STAGE, bool FACES>
+__global__ void __launch_bounds__(BTHR) adj_cells_kernel(const __grid_constant__ AdjArgs A,
+                                                         const __grid_constant__ StepSnap S) {
   extern __shared__ double s_tbl[];
   const int nt = 4 * A.tbl_rows;
   zero_smem_tbl(s_tbl, nt);
-  // final compute_fld
-  adj_compute_fld(A, S.ff3, SEG_FMG);
-  seg_rev(A, SEG_AVG);
-  // stage 2
-  adj_gc_lim(A, I_PION, S.R2i);
-  adj_gc_lim(A, I_ELEC, S.R2e);
-  seg_rev(A, SEG_RSTR);
-  adj_update(A, s_tbl, S.F2, S.E1, S.dt);
-  seg_rev(A, SEG_CONS);
-  adj_fluxes(A, s_tbl, S.R1e, S.E1, S.ff1, S.dt);
-  // stage 1
-  adj_compute_fld(A, S.ff1, SEG_FMG);
-  adj_gc_lim(A, I_PION, S.R1i);
-  adj_gc_lim(A, I_ELEC, S.R1e);
-  seg_rev(A, SEG_RSTR);
-  adj_update(A, s_tbl, S.F1, S.E0, S.dt);
-  seg_rev(A, SEG_CONS);
-  adj_fluxes(A, s_tbl, S.n0, S.E0, S.ff0, S.dt);
-  seg_rev(A, SEG_COPY);
+  if (FACES) adj_fluxes(A, s_tbl, STAGE == 2 ? S.R1e : S.n0, STAGE == 2 ? S.E1 : S.E0, STAGE == 2 ? S.ff1 : S.ff0, S.dt);
+  else adj_update(A, s_tbl, STAGE == 2 ? S.F2 : S.F1, STAGE == 2 ? S.E1 : S.E0, S.dt);
   flush_smem_tbl(A, s_tbl, nt);
-}
-
-// The reverse of the first field solve (no guess).
-__global__ void __launch_bounds__(ATHR) adj_init_kernel(AdjArgs A, const double *ff0) {
-  adj_compute_fld(A, ff0, SEG_FMG1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1259,6 +1511,12 @@ struct a5a_ctx {
   uint32_t *d_row_d = nullptr, *d_term_s = nullptr;
   double *d_row_self = nullptr, *d_term_c = nullptr;
   DBox *d_box = nullptr;
+  int *d_jmap = nullptr;
+  JRec *d_jrec = nullptr;
+  uint2 *d_jone = nullptr;
+  uint4 *d_jfour = nullptr, *d_jmany = nullptr;
+  uint32_t *d_jrow = nullptr, *d_jv = nullptr;
+  double *d_jcoef = nullptr;
   double *lam = nullptr, *lam_tbl = nullptr, *tbl = nullptr;
   double *init = nullptr;       // the program's initial state (full run state)
   double *ckpt = nullptr;       // stored states, n_ckpt of them
@@ -1513,8 +1771,52 @@ int a5a_create(a5g_ctx *run, const a5a_params *p, const double *dts, a5a_ctx **o
     A.tbl_rows = a->n_rows;
     A.tbl_xmin = v.tbl_xmin;
     A.tbl_inv_dx = v.tbl_inv_dx;
-    ACK(cudaFuncSetAttribute(adj_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(4 * a->n_rows * sizeof(double))));
+    // the multigrid segments in gather form, where the three variables fit
+    // shared memory
+    A.jS = 0;
+    A.vidx = a->X.v;
+    {
+      Jagged J;
+      int dev = 0, optin = 0;
+      cudaFuncAttributes fa{};
+      ACK(cudaGetDevice(&dev));
+      ACK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+      ACK(cudaFuncGetAttributes(&fa, adj_fmg_kernel));
+      // (the attributes belong to the kernels, not to this adjoint)
+      ACK(cudaFuncSetAttribute(adj_fmg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               optin - (int)fa.sharedSizeBytes));
+      const int need = std::max(optin, (int)(4 * a->n_rows * sizeof(double)));
+      ACK(cudaFuncSetAttribute(adj_cells_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, need));
+      ACK(cudaFuncSetAttribute(adj_cells_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, need));
+      ACK(cudaFuncSetAttribute(adj_cells_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, need));
+      ACK(cudaFuncSetAttribute(adj_cells_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, need));
+      if (build_jagged(a->T, a->X, a->tape, a->seg, J) &&
+          (3 * (size_t)J.S + 1 + J.coef.size()) * sizeof(double) + fa.sharedSizeBytes <= (size_t)optin) {
+        ARC(dupload(a->d_jmap, J.gmap, s));
+        ARC(dupload(a->d_jrec, J.rec, s));
+        ARC(dupload(a->d_jone, J.one, s));
+        ARC(dupload(a->d_jfour, J.four, s));
+        ARC(dupload(a->d_jmany, J.many, s));
+        ARC(dupload(a->d_jrow, J.row, s));
+        ARC(dupload(a->d_jv, J.v, s));
+        ARC(dupload(a->d_jcoef, J.coef, s));
+        ACK(cudaStreamSynchronize(s));  // (J's copies)
+        A.jS = J.S;
+        for (int w = 0; w < 2; w++) {
+          A.jfirst[w] = J.first[w];
+          A.jn[w] = J.n[w];
+        }
+        A.jmap = a->d_jmap;
+        A.jrec = a->d_jrec;
+        A.jone = a->d_jone;
+        A.jfour = a->d_jfour;
+        A.jmany = a->d_jmany;
+        A.jrow = a->d_jrow;
+        A.jv = a->d_jv;
+        A.jcoef = a->d_jcoef;
+        A.jnco = (int)J.coef.size();
+      }
+    }
     ACK(cudaStreamSynchronize(s));
     return A5G_OK;
   }();
@@ -1539,6 +1841,14 @@ int a5a_destroy(a5a_ctx *a) {
   cudaFree(a->d_row_term);
   cudaFree(a->d_term_s);
   cudaFree(a->d_term_c);
+  cudaFree(a->d_jmap);
+  cudaFree(a->d_jrec);
+  cudaFree(a->d_jone);
+  cudaFree(a->d_jfour);
+  cudaFree(a->d_jmany);
+  cudaFree(a->d_jrow);
+  cudaFree(a->d_jv);
+  cudaFree(a->d_jcoef);
   cudaFree(a->d_box);
   cudaFree(a->d_lists);
   cudaFree(a->lam);
@@ -1584,6 +1894,28 @@ int a5a_gradient(a5a_ctx *a, double *J, double *dJ_dtable, double *dJ_dV) {
                       cudaMemcpyHostToDevice, s));
   const int E = a->p.checkpoint_every;
   const size_t smem = 4 * (size_t)a->n_rows * sizeof(double);
+  // (at most a wave or two of blocks, each with a copy of the table's sums)
+  const int n_leaf = A.lv_leaves[A.nlev] - A.lv_leaves[0];
+  const int n_cell = std::min(148, std::max(1, (n_leaf * NC * NC + BTHR - 1) / BTHR));
+  const int n_face = std::min(148, std::max(1, (n_leaf * 2 * (NC + 1) * NC + BTHR - 1) / BTHR));
+  const int n_norm = std::max(1, ((A.lv_ids[A.nlev] - A.lv_ids[0]) * NC * NC + 127) / 128);
+  auto seg = [&](int sg) {
+    const int p0 = a->seg[sg], r0 = a->tape.phase_row[p0], r1 = a->tape.phase_row[p0 + 1];
+    if (a->seg[sg + 1] == p0 + 1)
+      adj_rows_kernel<<<std::max(1, (r1 - r0 + 255) / 256), 256, 0, s>>>(A, r0, r1);
+    else
+      adj_seg_kernel<<<1, ATHR, 0, s>>>(A, sg);
+  };
+  auto fld = [&](const double *ff, int fmg) {  // compute_fld's transpose
+    seg(SEG_GCFLD);
+    adj_norm_kernel<<<n_norm, 128, 0, s>>>(A, ff);
+    seg(SEG_FACES);
+    if (A.jS > 0)
+      adj_fmg_kernel<<<1, FTHR, (3 * (size_t)A.jS + 1 + A.jnco) * sizeof(double), s>>>(A, fmg == SEG_FMG ? 0 : 1);
+    else
+      adj_seg_kernel<<<1, ATHR, 0, s>>>(A, fmg);
+    seg(SEG_RHS);
+  };
   for (int c = a->n_ckpt - 1; c >= 0; c--) {
     const int k0 = c * E, k1 = std::min(a->p.n_steps, k0 + E);
     ARC(state_copy(a, a->ckpt + a->state_n * c, true));
@@ -1604,13 +1936,24 @@ int a5a_gradient(a5a_ctx *a, double *J, double *dJ_dtable, double *dJ_dV) {
       S.R2i = snap_cell(a, q, SN_R2I);
       S.ff3 = snap_face(a, q, SF_FF3);
       S.dt = a->dts[k];
-      adj_step_kernel<<<1, ATHR, smem, s>>>(A, S);
+      fld(S.ff3, SEG_FMG);
+      seg(SEG_AVG);
+      adj_gc_kernel<<<1, ATHR, 0, s>>>(A, S.R2i, S.R2e);
+      adj_cells_kernel<2, false><<<n_cell, BTHR, smem, s>>>(A, S);
+      seg(SEG_CONS);
+      adj_cells_kernel<2, true><<<n_face, BTHR, smem, s>>>(A, S);
+      fld(S.ff1, SEG_FMG);
+      adj_gc_kernel<<<1, ATHR, 0, s>>>(A, S.R1i, S.R1e);
+      adj_cells_kernel<1, false><<<n_cell, BTHR, smem, s>>>(A, S);
+      seg(SEG_CONS);
+      adj_cells_kernel<1, true><<<n_face, BTHR, smem, s>>>(A, S);
+      seg(SEG_COPY);
       ACK(cudaGetLastError());
     }
   }
   // the first field solve: its faces are step 0's starting faces (interval 0
   // was recomputed last)
-  adj_init_kernel<<<1, ATHR, 0, s>>>(A, snap_face(a, 0, SF_FF0));
+  fld(snap_face(a, 0, SF_FF0), SEG_FMG1);
   ACK(cudaGetLastError());
   ARC(state_copy(a, a->endst, true));
   ACK(cudaMemcpyAsync(dJ_dtable, a->lam_tbl, 4 * (size_t)a->n_rows * sizeof(double),
