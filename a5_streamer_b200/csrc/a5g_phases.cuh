@@ -1187,17 +1187,17 @@ __device__ __forceinline__ VCell<T> vcell(int p, bool cyl) {
   }
   return v;
 }
-// The four neighbours of a cell (as phi_nbrs). The across and along
-// neighbours that a refinement-boundary recipe reads are among the cell's
-// direct neighbours; a wall's source is the cell itself.
+// The four neighbours of a cell (as phi_nbrs), vo the cell itself. The across
+// and along neighbours that a refinement-boundary recipe reads are among the
+// cell's direct neighbours; a wall's source is the cell itself, so that walls
+// need a sign or one subtraction beside the sum's chain and no branch.
 template <class T>
-__device__ __forceinline__ void vnbrs(const T *phi, const VCell<T> &v, T v2, T &lx, T &hx, T &ly, T &hy) {
+__device__ __forceinline__ void vnbrs(const T *phi, const VCell<T> &v, T vo, T v2, T &lx, T &hx, T &ly, T &hy) {
   lx = phi[v.lx];
   hx = phi[v.hx];
   ly = phi[v.ly];
   hy = phi[v.hy];
-  if (v.fl & (VF_RBX | VF_RBY | VF_NEG | VF_TOP)) {
-    const T vo = phi[v.own];
+  if (v.fl & (VF_RBX | VF_RBY)) {
     const T bx = (v.fl & VF_ODDJ) ? hy : ly, by = (v.fl & VF_ODDI) ? hx : lx;
     const T gx = T(0.5) * ((v.fl & VF_XL) ? lx : hx) + vo - T(0.25) * (((v.fl & VF_XL) ? hx : lx) + bx);
     const T gy = T(0.5) * ((v.fl & VF_YL) ? ly : hy) + vo - T(0.25) * (((v.fl & VF_YL) ? hy : ly) + by);
@@ -1209,9 +1209,14 @@ __device__ __forceinline__ void vnbrs(const T *phi, const VCell<T> &v, T v2, T &
       if (v.fl & VF_YL) ly = gy;
       else hy = gy;
     }
-    if (v.fl & VF_NEG) ly = -vo;
-    if (v.fl & VF_TOP) hy = v2 - vo;
   }
+  if (v.fl & VF_NEG) ly = -ly;
+  if (v.fl & VF_TOP) hy = v2 - hy;
+}
+// Barrier of the threads 0 to n - 1 of the block (n a multiple of 32).
+__device__ __forceinline__ void active_sync(int n) {
+  if (n <= 32) __syncwarp();
+  else asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
 }
 // box_gsrb_lpl (m_aX_mg.f90:636-659) / box_gsrb_clpl (:998-1024); dr: dx^2 rhs
 template <class T>
@@ -1260,12 +1265,15 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
   const bool on = c0.fl & VF_ON;
   const T dx2 = T(R.lv_dx2[li]), inv = T(R.lv_inv2[li]);
   const int nc = R.lv_nc[li], ncg = nc + 2, sh = 31 - __clz(nc);
-  T r0 = 0, r1 = 0, lx, hx, ly, hy;
+  T r0 = 0, r1 = 0, v0 = 0, v1 = 0, lx, hx, ly, hy;
+  if (on) {
+    v0 = phi[c0.own];
+    v1 = phi[c1.own];
+  }
   if (on && (flags & PV_FC) && (c0.fl & VF_PARENT)) {
-    const T v0 = phi[c0.own], v1 = phi[c1.own];
-    vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
+    vnbrs<T>(phi, c0, v0, A.v2, lx, hx, ly, hy);
     r0 = vlap<T>(c0, cyl, lx, hx, ly, hy, v0, inv) + A.tmp[c0.own];
-    vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
+    vnbrs<T>(phi, c1, v1, A.v2, lx, hx, ly, hy);
     r1 = vlap<T>(c1, cyl, lx, hx, ly, hy, v1, inv) + A.tmp[c1.own];
     A.rhs[c0.own] = r0;
     A.rhs[c1.own] = r1;
@@ -1276,7 +1284,6 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
     r1 = A.rhs[c1.own];
   }
   if (on && (flags & (PV_COPY | PV_CORRECT))) {
-    const T v0 = phi[c0.own], v1 = phi[c1.own];
     if (flags & PV_COPY) {
       A.tmp[c0.own] = v0;
       A.tmp[c1.own] = v1;
@@ -1287,8 +1294,10 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
       const int pncg = R.lv_nc[li - 1] + 2, ps = (c0.fl & VF_ODDJ) ? pc - pncg : pc + pncg;
       const T q = phi[pc] - A.tmp[pc], qy = phi[ps] - A.tmp[ps];
       const T ql = phi[pc - 1] - A.tmp[pc - 1], qh = phi[pc + 1] - A.tmp[pc + 1];
-      phi[c0.own] = v0 + T(0.5) * q + T(0.25) * (((c0.fl & VF_ODDI) ? ql : qh) + qy);
-      phi[c1.own] = v1 + T(0.5) * q + T(0.25) * (((c1.fl & VF_ODDI) ? ql : qh) + qy);
+      v0 = v0 + T(0.5) * q + T(0.25) * (((c0.fl & VF_ODDI) ? ql : qh) + qy);
+      v1 = v1 + T(0.5) * q + T(0.25) * (((c1.fl & VF_ODDI) ? ql : qh) + qy);
+      phi[c0.own] = v0;
+      phi[c1.own] = v1;
     }
   }
   // ghost cells: fill (PV_FC, and tmp of parent boxes) or copy to tmp
@@ -1311,48 +1320,52 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
   if (flags & (PV_FC | PV_COPY)) ghosts(flags & PV_FC, flags & PV_FC, flags & PV_COPY);
   if (flags & (PV_FC | PV_COPY | PV_CORRECT)) __syncthreads();
   const T d0 = dx2 * r0, d1 = dx2 * r1;
-  int it = 1;
-  if (flags & PV_STALE) {
-    if (on) {
-      lx = phi[c1.own - 1];
-      hx = phi[c1.own + 1];
-      ly = phi[c1.own - ncg];
-      hy = phi[c1.own + ncg];
-      phi[c1.own] = vgsrb<T>(c1, cyl, lx, hx, ly, hy, d1);
-    }
-    __syncthreads();
-    it = 2;
-  }
-#pragma unroll 1
-  for (; it <= n; it++) {
-    if (on) {
-      if (it & 1) {
-        vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
-        phi[c1.own] = vgsrb<T>(c1, cyl, lx, hx, ly, hy, d1);
-      } else {
-        vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
-        phi[c0.own] = vgsrb<T>(c0, cyl, lx, hx, ly, hy, d0);
+  // the half-sweeps, on the warps that hold cells and with a barrier of these
+  // alone (on the coarsest levels one warp)
+  const int nact = ((R.bx_off[li + 1] - R.bx_off[li]) * (nc * nc / 2) + 31) & ~31;
+  if (threadIdx.x < nact) {
+    int it = 1;
+    if (flags & PV_STALE) {
+      if (on) {
+        lx = phi[c1.own - 1];
+        hx = phi[c1.own + 1];
+        ly = phi[c1.own - ncg];
+        hy = phi[c1.own + ncg];
+        phi[c1.own] = v1 = vgsrb<T>(c1, cyl, lx, hx, ly, hy, d1);
       }
+      active_sync(nact);
+      it = 2;
     }
-    __syncthreads();
+#pragma unroll 1
+    for (; it <= n; it++) {
+      if (on) {
+        if (it & 1) {
+          vnbrs<T>(phi, c1, v1, A.v2, lx, hx, ly, hy);
+          phi[c1.own] = v1 = vgsrb<T>(c1, cyl, lx, hx, ly, hy, d1);
+        } else {
+          vnbrs<T>(phi, c0, v0, A.v2, lx, hx, ly, hy);
+          phi[c0.own] = v0 = vgsrb<T>(c0, cyl, lx, hx, ly, hy, d0);
+        }
+      }
+      active_sync(nact);
+    }
   }
+  if (!(flags & PV_DOWN)) __syncthreads();
   if (flags & PV_DOWN) {
-    T e0 = 0, e1 = 0, p0 = 0, p1 = 0;
+    T e0 = 0, e1 = 0;
     if (on) {
-      p0 = phi[c0.own];
-      p1 = phi[c1.own];
-      vnbrs<T>(phi, c0, A.v2, lx, hx, ly, hy);
-      e0 = r0 - vlap<T>(c0, cyl, lx, hx, ly, hy, p0, inv);
-      vnbrs<T>(phi, c1, A.v2, lx, hx, ly, hy);
-      e1 = r1 - vlap<T>(c1, cyl, lx, hx, ly, hy, p1, inv);
+      vnbrs<T>(phi, c0, v0, A.v2, lx, hx, ly, hy);
+      e0 = r0 - vlap<T>(c0, cyl, lx, hx, ly, hy, v0, inv);
+      vnbrs<T>(phi, c1, v1, A.v2, lx, hx, ly, hy);
+      e1 = r1 - vlap<T>(c1, cyl, lx, hx, ly, hy, v1, inv);
     }
     // from the item one row up: its even cell (2ii, 2jj) and odd cell (2ii-1, 2jj)
     const int hn = nc >> 1;
     const T e11 = __shfl_down_sync(0xffffffffu, e0, hn), e01 = __shfl_down_sync(0xffffffffu, e1, hn);
-    const T p11 = __shfl_down_sync(0xffffffffu, p0, hn), p01 = __shfl_down_sync(0xffffffffu, p1, hn);
+    const T p11 = __shfl_down_sync(0xffffffffu, v0, hn), p01 = __shfl_down_sync(0xffffffffu, v1, hn);
     if (on && (c0.fl & VF_ODDJ)) {
       A.tmp[pc] = T(0.25) * (e0 + e1 + e01 + e11);
-      phi[pc] = T(0.25) * (p0 + p1 + p01 + p11);
+      phi[pc] = T(0.25) * (v0 + v1 + p01 + p11);
     }
     __syncthreads();
   }
