@@ -1144,6 +1144,11 @@ __device__ __forceinline__ bool plan_fits(const RunDev &R, const MGV<T> &M, cons
   return M.plans && R.cplan_blk[L.li] >= 0;
 }
 
+// Threads of a visit of level index li, in whole warps: one per two cells.
+__device__ __forceinline__ int visit_threads(const RunDev &R, int li) {
+  return ((R.bx_off[li + 1] - R.bx_off[li]) * ((R.lv_nc[li] * R.lv_nc[li]) >> 1) + 31) & ~31;
+}
+
 // Start fetching the plans of level index li into the slots, unless they are
 // there or the level has none. Only after this thread's last read of them.
 __device__ __forceinline__ void fetch_plan(const RunDev &R, int li, bool cyl, PlanFetch &pf) {
@@ -1151,12 +1156,14 @@ __device__ __forceinline__ void fetch_plan(const RunDev &R, int li, bool cyl, Pl
   const int blk = R.cplan_blk[li];
   if (blk < 0) return;
   if (pf.li >= 0) cp_async_wait_all();
-  const size_t o = (size_t)blk * 2 * NTHR + 2 * threadIdx.x;
-  cp_async16(&plan_slots()[2 * threadIdx.x], &R.cplan[o]);
-  cp_async16(&plan_slots()[2 * threadIdx.x + 1], &R.cplan[o + 1]);
-  if (cyl) {
-    cp_async16(&wts_slots()[2 * threadIdx.x], &R.cwts[o]);
-    cp_async16(&wts_slots()[2 * threadIdx.x + 1], &R.cwts[o + 1]);
+  if (threadIdx.x < visit_threads(R, li)) {
+    const size_t o = (size_t)blk * 2 * NTHR + 2 * threadIdx.x;
+    cp_async16(&plan_slots()[2 * threadIdx.x], &R.cplan[o]);
+    cp_async16(&plan_slots()[2 * threadIdx.x + 1], &R.cplan[o + 1]);
+    if (cyl) {
+      cp_async16(&wts_slots()[2 * threadIdx.x], &R.cwts[o]);
+      cp_async16(&wts_slots()[2 * threadIdx.x + 1], &R.cwts[o + 1]);
+    }
   }
   cp_async_commit();
   pf.li = li;
@@ -1259,8 +1266,16 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
   T *phi = A.phi;
   fetch_plan(R, li, cyl, pf);
   cp_async_wait_all();
-  const VCell<T> c0 = vcell<T>(0, cyl), c1 = vcell<T>(1, cyl);
-  const int pc = plan_slots()[2 * threadIdx.x].w;
+  // (the slots of the other threads are not fetched: a level's plans are up
+  // to 64 KB, and at 64 bytes a cycle from L2 they would outlast the visit)
+  const int nact = visit_threads(R, li);
+  VCell<T> c0{}, c1{};
+  int pc = 0;
+  if (threadIdx.x < nact) {
+    c0 = vcell<T>(0, cyl);
+    c1 = vcell<T>(1, cyl);
+    pc = plan_slots()[2 * threadIdx.x].w;
+  }
   fetch_plan(R, next, cyl, pf);
   const bool on = c0.fl & VF_ON;
   const T dx2 = T(R.lv_dx2[li]), inv = T(R.lv_inv2[li]);
@@ -1322,7 +1337,6 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
   const T d0 = dx2 * r0, d1 = dx2 * r1;
   // the half-sweeps, on the warps that hold cells and with a barrier of these
   // alone (on the coarsest levels one warp)
-  const int nact = ((R.bx_off[li + 1] - R.bx_off[li]) * (nc * nc / 2) + 31) & ~31;
   if (threadIdx.x < nact) {
     int it = 1;
     if (flags & PV_STALE) {
