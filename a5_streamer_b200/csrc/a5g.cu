@@ -33,6 +33,7 @@
 #include <mutex>
 #include <string>
 #include <type_traits>
+#include <unordered_map>
 #include <vector>
 
 namespace {
@@ -112,11 +113,11 @@ struct RunDev {
   // entries), -1 where the level's colours do not fit one cell per thread
   // (or an address does not fit 16 bits)
   const int4 *cplan;
-  const double2 *cwts;
+  const double2 *cwts;         // n_wts
   int cplan_blk[MAXLEV];
   const int *pbx;
   int smem_doubles;            // per multigrid variable; 0: tree does not fit
-  int pad4;
+  int n_wts;                   // different columns of a cylindrical tree, 0 otherwise
   double *scal;                // dt reductions out
   int *flags;                  // refinement flags out
   int *status;
@@ -283,9 +284,11 @@ __shared__ GroupCtl s_grp;
 extern __shared__ double g_dsmem[];
 
 // The plan slots lead the dynamic shared memory of a shared-memory solve:
-// 2 NTHR int4 cell plans, then (cylindrical runs) 2 NTHR double2 weights.
+// 2 NTHR int4 cell plans, then (cylindrical runs) the weights of the tree's
+// different columns, R.n_wts of them. (Weights per cell, fetched with the
+// plans of a visit, took 16 KB: trees of more than 74 boxes did not fit, and
+// a step of one of 86 took 1.44 ms instead of 0.84.)
 constexpr int PLAN_DOUBLES = 2 * NTHR * 2;     // doubles taken by the cell plans
-constexpr int WTS_DOUBLES = 2 * NTHR * 2;      // doubles taken by the weights
 
 // Kinds of a ghost neighbour: copy of s0 (same-level neighbour or Neumann
 // wall), refinement boundary (mg$D_sides_rb after a$D_gc_prolong0:
@@ -296,7 +299,7 @@ enum { GK_COPY = 0, GK_RB = 1, GK_NEG = 2, GK_TOP = 3 };
 // A cell plan as an int4 of 16-bit addresses in the shared-memory arrays:
 // x = cell | lx source << 16, y = hx source | ly source << 16, z = hy source |
 // VF_ flags << 16, w = parent cell of the 2 x 2 block the cell's thread
-// restricts (p_visit). The source of a neighbour is the neighbour's cell, or
+// restricts (p_visit) | place of its column's weights << 16. The source of a neighbour is the neighbour's cell, or
 // for a ghost neighbour the first source of its recipe.
 enum { VF_ON = 1, VF_RBX = 2, VF_XL = 4, VF_RBY = 8, VF_YL = 16, VF_NEG = 32, VF_TOP = 64, VF_ODDI = 128, VF_ODDJ = 256,
        VF_PARENT = 512 };
@@ -322,7 +325,7 @@ inline void ghost_src(const BoxRec &B, int nc, int ncg, int side, int k, int &s0
   }
 }
 
-inline int4 make_plan(const BoxRec &B, int nc, int ncg, int i, int j, int parent_cell) {
+inline int4 make_plan(const BoxRec &B, int nc, int ncg, int i, int j, int parent_cell_col) {
   const int g = B.base + i + ncg * j;
   int gx, gy, xk, yk;
   ghost_src(B, nc, ncg, i == 1 ? 0 : 1, j, gx, xk);
@@ -335,7 +338,7 @@ inline int4 make_plan(const BoxRec &B, int nc, int ncg, int i, int j, int parent
   if (ey && yk == GK_RB) fl |= VF_RBY;
   if (ey && yk == GK_NEG) fl |= VF_NEG;
   if (ey && yk == GK_TOP) fl |= VF_TOP;
-  return make_int4(g | (lx << 16), hx | (ly << 16), hy | (fl << 16), parent_cell);
+  return make_int4(g | (lx << 16), hx | (ly << 16), hy | (fl << 16), parent_cell_col);
 }
 
 // box_gsrb_clpl weights (i+ioff-1)/(i+ioff-1/2) and (i+ioff)/(i+ioff-1/2)
@@ -641,6 +644,7 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
   // its colour-0 and colour-1 cells in plan slots 2k and 2k+1.
   P.cplan.clear();
   P.cwts.clear();
+  std::unordered_map<int, int> columns;  // column -> its place in cwts
   for (int li = 0; li < MAXLEV; li++) P.cplan_blk[li] = -1;
   for (int li = 0; li < nlev; li++) {
     const int nc = P.lv_nc[li], ncg = nc + 2, half = (nc * nc) >> 1, hn = nc >> 1;
@@ -651,7 +655,6 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
     for (int k = 0; k < NTHR; k++) {
       int4 c[2];
       c[0] = c[1] = make_int4(0, 0, 0, 0);
-      double2 w[2] = {make_double2(0, 0), make_double2(0, 0)};
       if (k < nb * half) {
         const BoxRec &B = P.sboxes[b0 + (k >> hsh)];
         const int item = k & (half - 1);
@@ -660,14 +663,17 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
         const int pc = li > 0 ? B.pbase + (B.o0 + m + 1) + pncg * (B.o1 + ((j - 1) >> 1) + 1) : 0;
         for (int p = 0; p < 2; p++) {
           const int i = 2 * m + 2 - ((p + j) & 1);
-          c[p] = make_plan(B, nc, ncg, i, j, pc);
-          cyl_weights(B.gi0 + i, w[p].x, w[p].y);
+          const auto col = columns.emplace(B.gi0 + i, (int)P.cwts.size());
+          if (col.second) {
+            double2 w;
+            cyl_weights(B.gi0 + i, w.x, w.y);
+            P.cwts.push_back(w);
+          }
+          c[p] = make_plan(B, nc, ncg, i, j, pc | col.first->second << 16);
         }
       }
       P.cplan.push_back(c[0]);
       P.cplan.push_back(c[1]);
-      P.cwts.push_back(w[0]);
-      P.cwts.push_back(w[1]);
     }
   }
 }
@@ -1523,7 +1529,8 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
   RunDev &h = c->h;
   {
     // keep the multigrid variables in shared memory when the tree fits
-    const size_t need = (PLAN_DOUBLES + (c->p.coord == 1 ? WTS_DOUBLES : 0)) * sizeof(double) +
+    h.n_wts = c->p.coord == 1 ? (int)P.cwts.size() : 0;
+    const size_t need = (PLAN_DOUBLES + 2 * (size_t)h.n_wts) * sizeof(double) +
                         3 * (size_t)P.smem_doubles * sizeof(double) +
                         P.boxes.size() * sizeof(BoxRec) + P.pbx.size() * sizeof(int);
     const size_t limit = dyn_smem_limit();
@@ -1531,7 +1538,7 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
     c->need64 = need;
     // the FP32 correction solve of the mixed form: three float arrays
     const int s32 = (P.smem_doubles + 3) & ~3;
-    const size_t need32 = (PLAN_DOUBLES + (c->p.coord == 1 ? WTS_DOUBLES : 0)) * sizeof(double) +
+    const size_t need32 = (PLAN_DOUBLES + 2 * (size_t)h.n_wts) * sizeof(double) +
                           3 * (size_t)s32 * sizeof(float) + P.boxes.size() * sizeof(BoxRec) +
                           P.pbx.size() * sizeof(int);
     c->fit32 = need32 <= limit ? s32 : 0;

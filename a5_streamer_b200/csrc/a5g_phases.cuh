@@ -1112,7 +1112,7 @@ struct SmArr {
 };
 template <class T>
 __device__ __forceinline__ SmArr<T> sm_arrays(const RunDev &R) {
-  double *base = g_dsmem + PLAN_DOUBLES + (R.coord == 1 ? WTS_DOUBLES : 0);
+  double *base = g_dsmem + PLAN_DOUBLES + 2 * R.n_wts;
   T *b = reinterpret_cast<T *>(base);
   const int S = std::is_same<T, double>::value ? R.smem_doubles : R.mx_smem;
   return SmArr<T>{b, b + S, b + 2 * S, reinterpret_cast<const BoxRec *>(b + 3 * S),
@@ -1151,7 +1151,7 @@ __device__ __forceinline__ int visit_threads(const RunDev &R, int li) {
 
 // Start fetching the plans of level index li into the slots, unless they are
 // there or the level has none. Only after this thread's last read of them.
-__device__ __forceinline__ void fetch_plan(const RunDev &R, int li, bool cyl, PlanFetch &pf) {
+__device__ __forceinline__ void fetch_plan(const RunDev &R, int li, PlanFetch &pf) {
   if (li < 0 || li >= R.nlev || pf.li == li) return;
   const int blk = R.cplan_blk[li];
   if (blk < 0) return;
@@ -1160,10 +1160,6 @@ __device__ __forceinline__ void fetch_plan(const RunDev &R, int li, bool cyl, Pl
     const size_t o = (size_t)blk * 2 * NTHR + 2 * threadIdx.x;
     cp_async16(&plan_slots()[2 * threadIdx.x], &R.cplan[o]);
     cp_async16(&plan_slots()[2 * threadIdx.x + 1], &R.cplan[o + 1]);
-    if (cyl) {
-      cp_async16(&wts_slots()[2 * threadIdx.x], &R.cwts[o]);
-      cp_async16(&wts_slots()[2 * threadIdx.x + 1], &R.cwts[o + 1]);
-    }
   }
   cp_async_commit();
   pf.li = li;
@@ -1188,7 +1184,7 @@ __device__ __forceinline__ VCell<T> vcell(int p, bool cyl) {
   v.fl = (unsigned)c.z >> 16;
   v.wx = v.wy = T(1);
   if (cyl) {
-    const double2 w = wts_slots()[2 * threadIdx.x + p];
+    const double2 w = wts_slots()[(unsigned)c.w >> 16];
     v.wx = T(w.x);
     v.wy = T(w.y);
   }
@@ -1264,19 +1260,19 @@ __device__ __noinline__ PlanFetch p_visit(const RunDev &R, int li, int n, int fl
   const SmArr<T> A = sm_arrays<T>(R);
   const bool cyl = R.coord == 1;
   T *phi = A.phi;
-  fetch_plan(R, li, cyl, pf);
+  fetch_plan(R, li, pf);
   cp_async_wait_all();
-  // (the slots of the other threads are not fetched: a level's plans are up
-  // to 64 KB, and at 64 bytes a cycle from L2 they would outlast the visit)
+  // (the slots of the other threads are not fetched: all 16 KB at 64 bytes a
+  // cycle from L2 take as long as a half-sweep)
   const int nact = visit_threads(R, li);
   VCell<T> c0{}, c1{};
   int pc = 0;
   if (threadIdx.x < nact) {
     c0 = vcell<T>(0, cyl);
     c1 = vcell<T>(1, cyl);
-    pc = plan_slots()[2 * threadIdx.x].w;
+    pc = plan_slots()[2 * threadIdx.x].w & 0xffff;
   }
-  fetch_plan(R, next, cyl, pf);
+  fetch_plan(R, next, pf);
   const bool on = c0.fl & VF_ON;
   const T dx2 = T(R.lv_dx2[li]), inv = T(R.lv_inv2[li]);
   const int nc = R.lv_nc[li], ncg = nc + 2, sh = 31 - __clz(nc);
@@ -1716,7 +1712,7 @@ __device__ __forceinline__ void mg_staged(const RunDev &R, const F &body) {
   if (R.diel || R.has_lsf) p_set_tags(R);
   if (R.smem_doubles > 0 && !R.diel && !R.has_lsf) {
     const int S = R.smem_doubles, nbx = R.bx_off[R.nlev], npb = R.pb_off[R.nlev];
-    double *base = g_dsmem + PLAN_DOUBLES + (R.coord == 1 ? WTS_DOUBLES : 0);
+    double *base = g_dsmem + PLAN_DOUBLES + 2 * R.n_wts;
     BoxRec *sb = reinterpret_cast<BoxRec *>(base + 3 * S);
     int *spb = reinterpret_cast<int *>(sb + nbx);
     const int size = kClu ? s_grp.size : 1;
@@ -1727,6 +1723,7 @@ __device__ __forceinline__ void mg_staged(const RunDev &R, const F &body) {
       const int n4 = nbx * (int)(sizeof(BoxRec) / sizeof(int4));
       for (int k = threadIdx.x; k < n4; k += NTHR) dst[k] = src[k];
       for (int k = threadIdx.x; k < npb; k += NTHR) spb[k] = R.pbx[k];
+      for (int k = threadIdx.x; k < R.n_wts; k += NTHR) wts_slots()[k] = R.cwts[k];
     }
     PSYNC();  // (and every block of a cluster runs before its window is used)
     MGV<double> M{base, base + S, base + 2 * S, sb, spb, true, R.applied_voltage,
@@ -1886,7 +1883,7 @@ __device__ void p_solve_mixed(const RunDev &R) {
   const bool local = kClu && R.mx_smem > 0;  // the FP32 cycles on the first block
   if (R.mx_smem > 0) {
     const int S = R.mx_smem, nbx = R.bx_off[R.nlev], npb = R.pb_off[R.nlev];
-    float *base = reinterpret_cast<float *>(g_dsmem + PLAN_DOUBLES + (R.coord == 1 ? WTS_DOUBLES : 0));
+    float *base = reinterpret_cast<float *>(g_dsmem + PLAN_DOUBLES + 2 * R.n_wts);
     BoxRec *sb = reinterpret_cast<BoxRec *>(base + 3 * S);
     int *spb = reinterpret_cast<int *>(sb + nbx);
     const int4 *src = reinterpret_cast<const int4 *>(R.sboxes);
@@ -1894,6 +1891,7 @@ __device__ void p_solve_mixed(const RunDev &R) {
     const int n4 = nbx * (int)(sizeof(BoxRec) / sizeof(int4));
     for (int k = threadIdx.x; k < n4; k += NTHR) dst[k] = src[k];
     for (int k = threadIdx.x; k < npb; k += NTHR) spb[k] = R.pbx[k];
+    for (int k = threadIdx.x; k < R.n_wts; k += NTHR) wts_slots()[k] = R.cwts[k];
     __syncthreads();
     M = MGV<float>{base, base + S, base + 2 * S, sb, spb, true, 0.0, R.mx_sw_down, R.mx_sw_up,
                    R.mx_sw_base};
@@ -2517,7 +2515,6 @@ __device__ __forceinline__ void warp_scan2(int a, int b, int &ea, int &eb, int &
 //   ph_cnt               absorbed photons per cell, zeroed here
 __device__ void ph_source(const RunDev &R, double dt, bool has_dt) {
   __shared__ double s_fac;
-  __shared__ double s_prod[NTHR / 32][64];
   const bool cyl = R.coord == 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long W = R.ph_team;
@@ -2572,19 +2569,18 @@ __device__ void ph_source(const RunDev &R, double dt, bool has_dt) {
       const BoxMeta &m = R.meta[id];
       const int nc = m.nc, ncg = nc + 2, nn = nc * nc;
       const double *x = CC(R, I_PHO, id);
-      for (int t = lane; t < nn; t += 32) {
-        const int i = t % nc + 1, j = t / nc + 1;
-        const double v = x[i + ncg * j];
-        s_prod[warp][t] = cyl ? v * (m.r0 + (i - 0.5) * m.dr) : v;
+      double v[2] = {0, 0};  // products of cells lane and lane + 32
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int t = lane + 32 * q, i = t % nc + 1, j = t / nc + 1;
+        if (t >= nn) continue;
+        v[q] = x[i + ncg * j];
+        if (cyl) v[q] = v[q] * (m.r0 + (i - 0.5) * m.dr);
       }
-      __syncwarp();
-      if (lane == 0) {
-        double res = 0;
+      double res = 0;
 #pragma unroll 8
-        for (int t = 0; t < nn; t++) res = res + s_prod[warp][t];
-        box_sum[k] = cyl ? res * TWOPI_DP : res;
-      }
-      __syncwarp();
+      for (int t = 0; t < nn; t++) res = res + __shfl_sync(0xffffffffu, t < 32 ? v[0] : v[1], t & 31);
+      if (lane == 0) box_sum[k] = cyl ? res * TWOPI_DP : res;
     }
   }
   __syncthreads();
