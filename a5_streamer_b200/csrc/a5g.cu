@@ -33,7 +33,6 @@
 #include <mutex>
 #include <string>
 #include <type_traits>
-#include <unordered_map>
 #include <vector>
 
 namespace {
@@ -644,7 +643,7 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
   // its colour-0 and colour-1 cells in plan slots 2k and 2k+1.
   P.cplan.clear();
   P.cwts.clear();
-  std::unordered_map<int, int> columns;  // column -> its place in cwts
+  std::vector<int> columns;  // 1 + place in cwts of a column, 0: none yet
   for (int li = 0; li < MAXLEV; li++) P.cplan_blk[li] = -1;
   for (int li = 0; li < nlev; li++) {
     const int nc = P.lv_nc[li], ncg = nc + 2, half = (nc * nc) >> 1, hn = nc >> 1;
@@ -663,13 +662,15 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
         const int pc = li > 0 ? B.pbase + (B.o0 + m + 1) + pncg * (B.o1 + ((j - 1) >> 1) + 1) : 0;
         for (int p = 0; p < 2; p++) {
           const int i = 2 * m + 2 - ((p + j) & 1);
-          const auto col = columns.emplace(B.gi0 + i, (int)P.cwts.size());
-          if (col.second) {
+          const size_t gi = (size_t)(B.gi0 + i);
+          if (gi >= columns.size()) columns.resize(2 * gi, 0);
+          if (columns[gi] == 0) {
             double2 w;
-            cyl_weights(B.gi0 + i, w.x, w.y);
+            cyl_weights((int)gi, w.x, w.y);
             P.cwts.push_back(w);
+            columns[gi] = (int)P.cwts.size();
           }
-          c[p] = make_plan(B, nc, ncg, i, j, pc | col.first->second << 16);
+          c[p] = make_plan(B, nc, ncg, i, j, pc | (columns[gi] - 1) << 16);
         }
       }
       P.cplan.push_back(c[0]);
