@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(256) adj_rows_kernel(const __grid_constant__ A
 // ahead; the phase itself is a shared-memory round trip and two barriers.
 // 576 threads: one source of each small class each covers nearly every phase
 // of the 8 mm tree (399 phases), and what is prefetched has registers. The
-// vector in L2 with FP64 atomics took 1,000 us, 10-byte terms by jagged
+// vector in L2 with FP64 atomics takes 1,170 us, 10-byte terms by jagged
 // diagonals with 1,024 threads 1,360 (spills) and with 576 586 us, this form
 // 390 us (31 % of the issue slots; a phase is 1.0 us).
 constexpr int FTHR = 576;

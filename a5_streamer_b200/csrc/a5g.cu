@@ -5,9 +5,11 @@
 // ghost fill or restriction is a dependency point across the boxes of a
 // level: one step holds about a thousand of them. Launching a kernel (or
 // crossing a grid-wide barrier) per phase would make the step launch-bound.
-// Instead one persistent thread block runs a whole operation -- up to a full
-// time step -- for one run, with __syncthreads() between phases; independent
-// runs are batched as one block each in the same launch. All box data stay
+// Instead one launch runs a whole operation -- up to a full time step -- for
+// one run: one thread block with __syncthreads() between phases, or for a
+// single run on an otherwise empty device a cluster of eight, with the
+// multigrid on the first (cluster_run); independent runs are batched as one
+// block each in the same launch. All box data stay
 // resident in device memory (L2-resident for these sizes) between calls.
 //
 // Thread mapping: a block of NTHR threads is split into groups of GT = 64

@@ -1,7 +1,8 @@
 // a5g3 -- the 3D octree form of the device path on sm_100a (see
 // include/a5g3.h): uniformly refined octrees of 8^3-cell boxes resident in
-// HBM, one kernel per phase over a level's (or the leaves') box list, one
-// thread block per box, the whole time step replayed from a CUDA graph.
+// HBM; transport in fused kernels over the leaves' boxes, the multigrid on
+// dense levels split by colour (a5g3_mg.cuh), one kernel per phase, the whole
+// time step replayed from a CUDA graph.
 //
 // Arithmetic follows the reference expression by expression (compiled with
 // --fmad=false, so every multiply and add is rounded on its own) and gives
