@@ -16,7 +16,9 @@ struct A5UniformArgs {
 };
 // The dense levels of a topology, or null where it is not uniform (or too
 // large for their 32-bit indices, or without memory): the box phases serve.
-A5Uniform *a5u_build(const A5Topo &topo, const double *lv_dr);
+// Its tables are uploaded on the run's stream, which does not order with the
+// default stream.
+A5Uniform *a5u_build(const A5Topo &topo, const double *lv_dr, void *stream);
 void a5u_destroy(A5Uniform *u);
 // Settings or storage behind a captured solve have changed.
 void a5u_changed(A5Uniform *u);

@@ -790,10 +790,9 @@ static int check_status(a5g_ctx *c) {
   CK(cudaMemcpyAsync(&st, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   if (st != 0) {
-    int z = 0;
-    CK(cudaMemcpy(c->status, &z, sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     // a barrier that gave up leaves its words mid-count: start clean
-    if (st == A5G_TIMEOUT) CK(cudaMemset(c->gbar, 0, 4 * sizeof(unsigned)));
+    if (st == A5G_TIMEOUT) CK(cudaMemsetAsync(c->gbar, 0, 4 * sizeof(unsigned), c->stream));
     return fail(st, st == A5G_TIMEOUT ? "a grid barrier wait ran out (A5G_TIMEOUT)"
                                       : "device reported status " + std::to_string(st));
   }
@@ -898,7 +897,7 @@ static A5Uniform *uniform_of(a5g_ctx *c, bool mixed, A5UniformArgs &a) {
     return nullptr;
   if (!c->uni_checked) {
     c->uni_checked = true;
-    c->uni = a5u_build(c->topo, c->h.lv_dr);
+    c->uni = a5u_build(c->topo, c->h.lv_dr, c->stream);
   }
   if (!c->uni) return nullptr;
   a = A5UniformArgs{};
@@ -1077,14 +1076,17 @@ int a5g_create(const a5g_params *p, a5g_ctx **out) {
     a5g_destroy(c);
     return fail(A5G_ENOMEM, "cudaMalloc failed");
   }
-  cudaMemset(c->status, 0, sizeof(int));
-  cudaMemset(c->gbar, 0, 4 * sizeof(unsigned));
+  // What a run holds is set on its own stream, here and wherever it changes:
+  // the stream does not order with the default stream, on which a clear, or a
+  // copy from pageable memory, may still be under way when the call returns.
+  e = cudaMemsetAsync(c->status, 0, sizeof(int), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(c->gbar, 0, 4 * sizeof(unsigned), c->stream);
   {
     // scalars: [0..2] reductions, [8..11] block state (dt, time, end time, active)
     double z[16] = {0};
     z[10] = HUGE_VAL;
     z[11] = 1.0;
-    cudaMemcpy(c->scal, z, sizeof(z), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c->scal, z, sizeof(z), cudaMemcpyHostToDevice, c->stream);
   }
   RunDev &h = c->h;
   std::memset(&h, 0, sizeof(RunDev));
@@ -1128,9 +1130,10 @@ int a5g_create(const a5g_params *p, a5g_ctx **out) {
       a5g_destroy(c);
       return fail(A5G_ENOMEM, "cudaMalloc failed");
     }
-    cudaMemcpy(c->ph_rng, p->rng_seed, 4 * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(c->ph_jump, J.data(), jbytes, cudaMemcpyHostToDevice);
-    cudaMemset(c->ph_scal, 0, sizeof(PhScal));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c->ph_rng, p->rng_seed, 4 * sizeof(int), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c->ph_jump, J.data(), jbytes, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->ph_scal, 0, sizeof(PhScal), c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // (J's copy)
     h.ph_enabled = 1;
     h.ph_team = p->photoi_team;
     h.ph_coeff = p->photoi_coeff;
@@ -1138,6 +1141,10 @@ int a5g_create(const a5g_params *p, a5g_ctx **out) {
     h.ph_rng = c->ph_rng;
     h.ph_scal = c->ph_scal;
     h.ph_jump = c->ph_jump;
+  }
+  if (e != cudaSuccess) {
+    a5g_destroy(c);
+    return fail(A5G_ECUDA, std::string("setting up the run: ") + cudaGetErrorString(e));
   }
   *out = c;
   return A5G_OK;
@@ -1287,7 +1294,7 @@ int a5g_set_photon_table(a5g_ctx *c, int n_rows, double x_min, double inv_dx, co
   cudaFree(c->ph_tbl);
   c->ph_tbl = nullptr;
   CK(cudaMalloc(&c->ph_tbl, sizeof(double) * n_rows));
-  CK(cudaMemcpy(c->ph_tbl, dist, sizeof(double) * n_rows, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->ph_tbl, dist, sizeof(double) * n_rows, cudaMemcpyHostToDevice, c->stream));
   c->h_ph_tbl.assign(dist, dist + n_rows);
   // pi_lengthscale = LT_get_col(tbl, 1, fac_dx) and get_lvl_length
   // (src/m_photons.f90:142-155, 331-336)
@@ -1924,7 +1931,7 @@ int a5g_set_ctas(a5g_ctx *c, int n_cta, long long wait_cycles) {
                                   " blocks that can be co-resident on this device");
   }
   CK(cudaStreamSynchronize(c->stream));
-  CK(cudaMemset(c->gbar, 0, 4 * sizeof(unsigned)));
+  CK(cudaMemsetAsync(c->gbar, 0, 4 * sizeof(unsigned), c->stream));
   c->n_cta = n_cta;
   c->h.gbudget = wait_cycles < 0 ? A5G_DEFAULT_WAIT_CYCLES : wait_cycles;
   apply_staging(c);
@@ -2232,8 +2239,8 @@ static int batch_build_ops(a5g_batch *b) {
   }
   b->ph_smem = std::min(ph, dyn_smem_limit());
   b->dyn = dyn_smem_limit();
-  CK(cudaMemcpy(b->d_rp, rp.data(), n * sizeof(void *), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(b->d_ops, ops.data(), 3 * n * sizeof(Op), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(b->d_rp, rp.data(), n * sizeof(void *), cudaMemcpyHostToDevice, b->stream));
+  CK(cudaMemcpyAsync(b->d_ops, ops.data(), 3 * n * sizeof(Op), cudaMemcpyHostToDevice, b->stream));
   // box-to-block mapping: each member's group of c->n_cta blocks
   b->mapped = false;
   int total = 0;
@@ -2254,9 +2261,10 @@ static int batch_build_ops(a5g_batch *b) {
         gmap[3 * blk + 1] = r;
         gmap[3 * blk + 2] = b->ctxs[k]->n_cta;
       }
-    CK(cudaMemcpy(b->d_gmap, gmap.data(), gmap.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(b->d_gmap, gmap.data(), gmap.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
     b->n_blocks = total;
   }
+  CK(cudaStreamSynchronize(b->stream));
   batch_drop_graph(b);
   return A5G_OK;
 }
@@ -2356,7 +2364,7 @@ int a5g_batch_begin(a5g_batch *b, const double *time, const double *t_end) {
     a5g_ctx *c = b->ctxs[k];
     CK(cudaStreamSynchronize(c->stream));
     const double st[4] = {0.0, time[k], t_end[k], 1.0};
-    CK(cudaMemcpy(c->scal + 8, st, sizeof(st), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(c->scal + 8, st, sizeof(st), cudaMemcpyHostToDevice, c->stream));
   }
   return batch_build_ops(b);
 }

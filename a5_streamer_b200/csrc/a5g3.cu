@@ -2040,7 +2040,7 @@ int a5g3_set_table(a5g3_ctx *c, int n_rows, int n_cols, double x_min, double inv
   for (int r = 0; r < n_rows; r++)
     for (int q = 0; q < 4; q++) both[4 * (size_t)n_rows + 4 * (size_t)r + q] = rc[(size_t)q * n_rows + r];
   CK3(cudaMalloc((void **)&c->d_lt, both.size() * sizeof(double)));
-  CK3(cudaMemcpy(c->d_lt, both.data(), both.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK3(cudaMemcpyAsync(c->d_lt, both.data(), both.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   {
     // FP32 copy for the lookups of the mixed form
     std::vector<float> t32(both.size());
@@ -2048,7 +2048,8 @@ int a5g3_set_table(a5g3_ctx *c, int n_rows, int n_cols, double x_min, double inv
     if (c->d_lt32) cudaFree(c->d_lt32);
     c->d_lt32 = nullptr;
     CK3(cudaMalloc((void **)&c->d_lt32, t32.size() * sizeof(float)));
-    CK3(cudaMemcpy(c->d_lt32, t32.data(), t32.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CK3(cudaMemcpyAsync(c->d_lt32, t32.data(), t32.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    CK3(cudaStreamSynchronize(c->stream));  // (both's and t32's copies)
   }
   c->lt_rows = n_rows;
   c->lt_xmin = x_min;

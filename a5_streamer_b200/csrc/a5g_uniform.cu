@@ -712,7 +712,8 @@ void a5u_changed(A5Uniform *u) {
 // Every level of the tree a complete rectangular grid of same-level
 // neighbours with walls around it, leaves on the finest level only (which the
 // level lists must say: a box on level lvls_max is in neither list).
-A5Uniform *a5u_build(const A5Topo &t, const double *lv_dr) {
+A5Uniform *a5u_build(const A5Topo &t, const double *lv_dr, void *stream) {
+  const cudaStream_t s = (cudaStream_t)stream;
   const int lo = t.min_lvl, hi = t.max_lvl, nlev = hi - lo + 1;
   if (nlev < 2 || nlev > UMAXLV || hi < 1 || lo > 0) return nullptr;
   auto A = new A5Uniform();
@@ -803,10 +804,11 @@ A5Uniform *a5u_build(const A5Topo &t, const double *lv_dr) {
     return no();
   }
   auto up = [&](void **d, const void *h, size_t bytes) {
-    return cudaMalloc(d, bytes) == cudaSuccess && (!h || cudaMemcpy(*d, h, bytes, cudaMemcpyHostToDevice) == cudaSuccess);
+    return cudaMalloc(d, bytes) == cudaSuccess && (!h || cudaMemcpyAsync(*d, h, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess);
   };
   if (!up((void **)&A->org, org.data(), nid * sizeof(int4)) || !up((void **)&A->nbr, nbr.data(), nid * sizeof(int4)) ||
-      !up((void **)&A->ids, ids.data(), ids.size() * sizeof(int)) || !up((void **)&A->d64, nullptr, 3 * off * sizeof(double))) {
+      !up((void **)&A->ids, ids.data(), ids.size() * sizeof(int)) || !up((void **)&A->d64, nullptr, 3 * off * sizeof(double)) ||
+      cudaStreamSynchronize(s) != cudaSuccess) {
     cudaGetLastError();
     return no();
   }
