@@ -23,5 +23,5 @@ void a5u_destroy(A5Uniform *u);
 // Settings or storage behind a captured solve have changed.
 void a5u_changed(A5Uniform *u);
 bool a5u_ready(A5Uniform *u, const A5UniformArgs &a, void *stream);
-int a5u_solve(A5Uniform *u, const A5UniformArgs &a, void *stream);  // a cudaError_t
+int a5u_solve(A5Uniform *u, bool mixed, void *stream);  // a cudaError_t
 #endif

@@ -887,13 +887,22 @@ static int launch_smem(a5g_ctx *c, const Op &op, size_t smem) {
   CK(cudaGetLastError());
   return A5G_OK;
 }
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+}
 // The dense levels of a run on several blocks (grid mode) whose tree is
 // uniformly refined and whose operators are the plain Laplacian's; null: the
-// box phases serve. Every level complete is what the dense form needs.
+// box phases serve. Every level complete is what the dense form needs. A
+// caller who captures the run's stream gets the box phases: they read the
+// applied field, the schedule and the storage from device memory when the
+// capture is replayed, where the dense launches hold them as parameters, and
+// the dense levels cannot be allocated during a capture.
 // Measured with all blocks, first solve and 8 steps with fields in and out:
 // 1,048,576 cells FP64 31.7 -> 14.7 ms, 245,760 cells mixed 16.4 -> 7.0 ms.
 static A5Uniform *uniform_of(a5g_ctx *c, bool mixed, A5UniformArgs &a) {
-  if (c->n_cta <= 1 || !c->has_tree || !c->has_table || c->p.coord != 0 || c->h.diel || c->h.has_lsf || c->p.photoi_enabled)
+  if (c->n_cta <= 1 || !c->has_tree || !c->has_table || c->p.coord != 0 || c->h.diel || c->h.has_lsf || c->p.photoi_enabled ||
+      capturing(c->stream))
     return nullptr;
   if (!c->uni_checked) {
     c->uni_checked = true;
@@ -1707,7 +1716,7 @@ static bool solve_uniform(a5g_ctx *c, bool mixed, int &r) {
   A5UniformArgs a;
   A5Uniform *u = uniform_of(c, mixed, a);
   if (!u) return false;
-  const cudaError_t e = (cudaError_t)a5u_solve(u, a, c->stream);
+  const cudaError_t e = (cudaError_t)a5u_solve(u, mixed, c->stream);
   r = e == cudaSuccess ? A5G_OK : fail(A5G_ECUDA, std::string("dense field solve: ") + cudaGetErrorString(e));
   return true;
 }
@@ -1879,7 +1888,7 @@ int a5g_step(a5g_ctx *c, double dt) {
       for (int stage = 1; stage <= 2; stage++) {
         const int r = launch(c, mkop(OP_STAGE, stage, mixed ? 1 : 0, dt));
         if (r) return r;
-        CK((cudaError_t)a5u_solve(u, a, c->stream));
+        CK((cudaError_t)a5u_solve(u, mixed, c->stream));
       }
       return A5G_OK;
     }

@@ -815,23 +815,16 @@ A5Uniform *a5u_build(const A5Topo &t, const double *lv_dr, void *stream) {
   return A;
 }
 
-// Whether a solve with these settings can run: its memory is there, and
-// unless the caller is capturing the stream its graph.
-static bool capturing(cudaStream_t s) {
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
-}
+// Whether a solve with these settings can run: its memory is there and its
+// launches are captured. The caller is not capturing the stream.
 bool a5u_ready(A5Uniform *u, const A5UniformArgs &a, void *stream) {
   const cudaStream_t s = (cudaStream_t)stream;
-  const bool cap = capturing(s);
-  if (a.mixed && !u->d32) {
-    if (cap || cudaMalloc((void **)&u->d32, 3 * (size_t)u->cells * sizeof(float)) != cudaSuccess) {
-      if (!cap) cudaGetLastError();
-      return false;
-    }
+  if (a.mixed && !u->d32 && cudaMalloc((void **)&u->d32, 3 * (size_t)u->cells * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
   const int k = a.mixed ? 1 : 0;
-  if (cap || u->exec[k]) return true;
+  if (u->exec[k]) return true;
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return false;
   enqueue(u, a, s);
   if (cudaStreamEndCapture(s, &u->graph[k]) != cudaSuccess ||
@@ -842,11 +835,8 @@ bool a5u_ready(A5Uniform *u, const A5UniformArgs &a, void *stream) {
   }
   return true;
 }
-// compute_fld with a guess on the run's stream (after a5u_ready): the graph
-// replayed, or its launches where the caller is capturing the stream.
-int a5u_solve(A5Uniform *u, const A5UniformArgs &a, void *stream) {
-  const cudaStream_t s = (cudaStream_t)stream;
-  if (!capturing(s)) return (int)cudaGraphLaunch(u->exec[a.mixed ? 1 : 0], s);
-  enqueue(u, a, s);
-  return (int)cudaGetLastError();
+// compute_fld with a guess on the run's stream, after a5u_ready with the same
+// settings.
+int a5u_solve(A5Uniform *u, bool mixed, void *stream) {
+  return (int)cudaGraphLaunch(u->exec[mixed ? 1 : 0], (cudaStream_t)stream);
 }
