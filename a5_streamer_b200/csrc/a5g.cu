@@ -496,7 +496,6 @@ struct a5g_ctx {
   PhScal *ph_scal = nullptr;
   MzJump *ph_jump = nullptr;
   PhBox *ph_boxes = nullptr;
-  int ph_capacity = 0;   // capacity the per-box photon buffers are sized for
   size_t ph_boxes_cap = 0;
   // mixed precision
   int precision = 0;     // A5G_FP64 or A5G_MIXED
@@ -531,7 +530,25 @@ struct a5g_ctx {
   double *lsf = nullptr, *bval = nullptr;
   // host copy of the last uploaded topology (a5g_internal_view)
   A5Topo topo;
+  // diagnostics: which of the next storage allocations of a tree upload fails
+  // (a5g_debug_fail_alloc), 0: none
+  int fail_alloc = 0;
 };
+
+// Device storage that follows the tree.
+template <class T>
+static cudaError_t tree_malloc(a5g_ctx *c, T **p, size_t n) {
+  if (c->fail_alloc > 0 && --c->fail_alloc == 0) return cudaErrorMemoryAllocation;
+  return cudaMalloc((void **)p, n * sizeof(T));
+}
+// The uploaded tree no longer holds (its storage or lists are about to
+// change): calls that need one are refused until an upload has gone through.
+static void forget_tree(a5g_ctx *c) {
+  a5u_destroy(c->uni);  // (its captured solves hold the old storage)
+  c->uni = nullptr;
+  c->uni_checked = false;
+  c->has_tree = false;
+}
 
 // Shared-memory staging of the multigrid variables as allowed and as fits
 // (never in grid mode: a block holds only part of the tree's work).
@@ -684,10 +701,12 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
 template <class T>
 static int upload_vec(a5g_ctx *c, T *&dev, size_t &cap, const std::vector<T> &v) {
   if (v.size() + 1 > cap) {
+    const size_t n = std::max(v.size() + 1, 2 * cap);
     cudaFree(dev);
     dev = nullptr;
-    cap = std::max(v.size() + 1, 2 * cap);
-    CK(cudaMalloc(&dev, cap * sizeof(T)));
+    cap = 0;
+    CK(tree_malloc(c, &dev, n));
+    cap = n;
   }
   if (!v.empty())
     CK(cudaMemcpyAsync(dev, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
@@ -979,43 +998,6 @@ static std::vector<MzJump> mz_run_table(long long W) {
   for (int b = 0; b < nblk; b++)
     T[MZ_JBLK + b] = mz_power(T.data(), 4ull * (unsigned long long)W + 4ull * PH_THREADS * b);
   return T;
-}
-
-// Photon buffers sized for the current box capacity: per cell a draw, a
-// first photon number and an absorption count; per box and per team thread
-// scratch. At most num_photons + one per leaf cell are created (the expected
-// total is at most num_photons and stochastic rounding adds at most one per
-// cell); photon numbers must stay below 2^31.
-static int ph_resize(a5g_ctx *c) {
-  if (!c->p.photoi_enabled || c->capacity == c->ph_capacity) return A5G_OK;
-  const size_t cells = (size_t)c->capacity * SLOT;
-  const size_t src = (size_t)c->p.photoi_num_photons + (size_t)c->capacity * NC * NC + 1024;
-  if (src > (size_t)INT_MAX) return fail(A5G_EINVAL, "photon numbers above 2^31");
-  CK(cudaStreamSynchronize(c->stream));
-  cudaFree(c->ph_ncr);
-  cudaFree(c->ph_cnt);
-  cudaFree(c->ph_ipart);
-  cudaFree(c->ph_part);
-  cudaFree(c->ph_u);
-  c->ph_ncr = c->ph_cnt = c->ph_ipart = nullptr;
-  c->ph_part = c->ph_u = nullptr;
-  if (cudaMalloc(&c->ph_ncr, cells * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&c->ph_cnt, cells * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&c->ph_ipart, 5 * (size_t)c->capacity * sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&c->ph_part, 2 * (size_t)c->capacity * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&c->ph_u, cells * sizeof(double)) != cudaSuccess)
-    return fail(A5G_ENOMEM, "cannot allocate photon buffers");
-  CK(cudaMemsetAsync(c->ph_ncr, 0, cells * sizeof(int), c->stream));
-  CK(cudaMemsetAsync(c->ph_cnt, 0, cells * sizeof(int), c->stream));
-  c->ph_capacity = c->capacity;
-  RunDev &h = c->h;
-  h.ph_ncr = c->ph_ncr;
-  h.ph_cnt = c->ph_cnt;
-  h.ph_ipart = c->ph_ipart;
-  h.ph_part = c->ph_part;
-  h.ph_u = c->ph_u;
-  h.ph_cap = (int)src;
-  return A5G_OK;
 }
 
 static int ph_ready(a5g_ctx *c) {
@@ -1359,94 +1341,122 @@ int a5g_set_rng(a5g_ctx *c, const int *st) {
   return A5G_OK;
 }
 
+// Storage for at least need boxes, with the contents of those there are. All
+// of it is allocated before any of the old is given up: where that fails, the
+// run is as it was.
 static int grow(a5g_ctx *c, int need) {
   if (need <= c->capacity) return A5G_OK;
-  const int old_cap = c->capacity;
-  int cap = std::max(need, c->capacity + c->capacity / 2);
-  cap = std::max(cap, 64);
-  double *ncc = nullptr, *nfx = nullptr, *nfy = nullptr;
-  BoxMeta *nmeta = nullptr;
-  int *nflags = nullptr;
-  size_t scc = (size_t)cap * SLOT * A5G_N_VAR_CELL, sfc = (size_t)cap * FSLOT * A5G_N_VAR_FACE;
-  if (cudaMalloc(&ncc, scc * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&nfx, sfc * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&nfy, sfc * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&nmeta, (size_t)cap * sizeof(BoxMeta)) != cudaSuccess ||
-      cudaMalloc(&nflags, (size_t)cap * sizeof(int)) != cudaSuccess) {
-    cudaFree(ncc); cudaFree(nfx); cudaFree(nfy); cudaFree(nmeta); cudaFree(nflags);
-    return fail(A5G_ENOMEM, "cannot grow box storage to " + std::to_string(cap) + " boxes");
+  const size_t old = c->capacity;
+  const int cap = std::max(std::max(need, c->capacity + c->capacity / 2), 64);
+  const size_t cells = (size_t)cap * SLOT, scc = cells * A5G_N_VAR_CELL, sfc = (size_t)cap * FSLOT * A5G_N_VAR_FACE;
+  const bool ph = c->p.photoi_enabled != 0, ls = c->lsf != nullptr;
+  // Photon buffers: per cell a draw, a first photon number and an absorption
+  // count; per box scratch. At most num_photons + one per leaf cell are
+  // created (the expected total is at most num_photons and stochastic rounding
+  // adds at most one per cell); photon numbers must stay below 2^31.
+  const size_t src = (size_t)c->p.photoi_num_photons + (size_t)cap * NC * NC + 1024;
+  if (ph && src > (size_t)INT_MAX) return fail(A5G_EINVAL, "photon numbers above 2^31");
+  struct {
+    double *cc = nullptr, *fx = nullptr, *fy = nullptr, *sumbuf = nullptr, *lsf = nullptr, *bval = nullptr;
+    double *ph_part = nullptr, *ph_u = nullptr;
+    BoxMeta *meta = nullptr;
+    int *flags = nullptr, *tags = nullptr, *ph_ncr = nullptr, *ph_cnt = nullptr, *ph_ipart = nullptr;
+  } n;
+  cudaError_t e = cudaSuccess;
+  auto get = [&](auto &p, size_t k) {
+    if (e == cudaSuccess) e = tree_malloc(c, &p, k);
+  };
+  get(n.cc, scc);
+  get(n.fx, sfc);
+  get(n.fy, sfc);
+  get(n.meta, (size_t)cap);
+  get(n.flags, (size_t)cap);
+  get(n.tags, (size_t)cap);  // box tags of the dielectric multigrid
+  get(n.sumbuf, (size_t)cap);
+  if (ls) {
+    get(n.lsf, cells);
+    get(n.bval, cells);
   }
-  CK(cudaMemsetAsync(ncc, 0, scc * sizeof(double), c->stream));
-  CK(cudaMemsetAsync(nfx, 0, sfc * sizeof(double), c->stream));
-  CK(cudaMemsetAsync(nfy, 0, sfc * sizeof(double), c->stream));
-  CK(cudaMemsetAsync(nmeta, 0, (size_t)cap * sizeof(BoxMeta), c->stream));
-  if (c->capacity > 0) {
-    for (int v = 0; v < A5G_N_VAR_CELL; v++)
-      CK(cudaMemcpyAsync(ncc + (size_t)v * cap * SLOT, c->cc + (size_t)v * c->capacity * SLOT,
-                         (size_t)c->capacity * SLOT * sizeof(double), cudaMemcpyDeviceToDevice,
-                         c->stream));
-    for (int f = 0; f < A5G_N_VAR_FACE; f++) {
-      CK(cudaMemcpyAsync(nfx + (size_t)f * cap * FSLOT, c->fx + (size_t)f * c->capacity * FSLOT,
-                         (size_t)c->capacity * FSLOT * sizeof(double), cudaMemcpyDeviceToDevice,
-                         c->stream));
-      CK(cudaMemcpyAsync(nfy + (size_t)f * cap * FSLOT, c->fy + (size_t)f * c->capacity * FSLOT,
-                         (size_t)c->capacity * FSLOT * sizeof(double), cudaMemcpyDeviceToDevice,
-                         c->stream));
-    }
+  if (ph) {
+    get(n.ph_ncr, cells);
+    get(n.ph_cnt, cells);
+    get(n.ph_ipart, 5 * (size_t)cap);
+    get(n.ph_part, 2 * (size_t)cap);
+    get(n.ph_u, cells);
   }
-  CK(cudaStreamSynchronize(c->stream));
-  cudaFree(c->cc); cudaFree(c->fx); cudaFree(c->fy); cudaFree(c->meta); cudaFree(c->flags);
-  c->cc = ncc; c->fx = nfx; c->fy = nfy; c->meta = nmeta; c->flags = nflags;
-  c->capacity = cap;
-  c->h.capacity = cap;
-  c->h.cc = ncc; c->h.fx = nfx; c->h.fy = nfy; c->h.meta = nmeta; c->h.flags = nflags;
-  {
-    // box tags of the dielectric multigrid: recomputed at every solve
-    int *nt = nullptr;
-    if (cudaMalloc(&nt, (size_t)cap * sizeof(int)) != cudaSuccess)
-      return fail(A5G_ENOMEM, "cannot grow the box tags to " + std::to_string(cap) + " boxes");
-    CK(cudaMemsetAsync(nt, 0, (size_t)cap * sizeof(int), c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    cudaFree(c->tags);
-    c->tags = nt;
-    c->h.tags = nt;
+  const bool got = e == cudaSuccess;
+  auto zero = [&](void *p, size_t bytes) {
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, c->stream);
+  };
+  auto copy = [&](double *to, const double *from, size_t k) {
+    if (e == cudaSuccess && k) e = cudaMemcpyAsync(to, from, k * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
+  };
+  zero(n.cc, scc * sizeof(double));
+  zero(n.fx, sfc * sizeof(double));
+  zero(n.fy, sfc * sizeof(double));
+  zero(n.meta, (size_t)cap * sizeof(BoxMeta));
+  zero(n.tags, (size_t)cap * sizeof(int));
+  for (int v = 0; v < A5G_N_VAR_CELL; v++) copy(n.cc + v * cells, c->cc + v * old * SLOT, old * SLOT);
+  for (int f = 0; f < A5G_N_VAR_FACE; f++) {
+    copy(n.fx + f * (size_t)cap * FSLOT, c->fx + f * old * FSLOT, old * FSLOT);
+    copy(n.fy + f * (size_t)cap * FSLOT, c->fy + f * old * FSLOT, old * FSLOT);
   }
-  {
-    double *ns = nullptr;
-    if (cudaMalloc(&ns, (size_t)cap * sizeof(double)) != cudaSuccess)
-      return fail(A5G_ENOMEM, "cannot grow the reduction buffer to " + std::to_string(cap) + " boxes");
-    cudaFree(c->sumbuf);
-    c->sumbuf = ns;
-    c->h.sumbuf = ns;
+  if (ls) {  // (new boxes hold 0 until set)
+    zero(n.lsf, cells * sizeof(double));
+    zero(n.bval, cells * sizeof(double));
+    copy(n.lsf, c->lsf, old * SLOT);
+    copy(n.bval, c->bval, old * SLOT);
   }
-  if (c->lsf) {
-    // level-set arrays follow the box storage (new boxes hold 0 until set)
-    double *nl = nullptr, *nb = nullptr;
-    const size_t old = (size_t)old_cap * SLOT, sz = (size_t)cap * SLOT;
-    if (cudaMalloc(&nl, sz * sizeof(double)) != cudaSuccess || cudaMalloc(&nb, sz * sizeof(double)) != cudaSuccess) {
-      cudaFree(nl);
-      cudaFree(nb);
-      return fail(A5G_ENOMEM, "cannot grow the level-set arrays");
-    }
-    CK(cudaMemsetAsync(nl, 0, sz * sizeof(double), c->stream));
-    CK(cudaMemsetAsync(nb, 0, sz * sizeof(double), c->stream));
-    CK(cudaMemcpyAsync(nl, c->lsf, old * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaMemcpyAsync(nb, c->bval, old * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    cudaFree(c->lsf);
-    cudaFree(c->bval);
-    c->lsf = nl;
-    c->bval = nb;
-    c->h.lsf = nl;
-    c->h.bval = nb;
+  if (ph) {
+    zero(n.ph_ncr, cells * sizeof(int));
+    zero(n.ph_cnt, cells * sizeof(int));
+  }
+  const cudaError_t es = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) e = es;
+  if (e != cudaSuccess) {
+    for (void *p : {(void *)n.cc, (void *)n.fx, (void *)n.fy, (void *)n.sumbuf, (void *)n.lsf, (void *)n.bval,
+                    (void *)n.ph_part, (void *)n.ph_u, (void *)n.meta, (void *)n.flags, (void *)n.tags,
+                    (void *)n.ph_ncr, (void *)n.ph_cnt, (void *)n.ph_ipart})
+      cudaFree(p);
+    cudaGetLastError();
+    return got ? fail(A5G_ECUDA, std::string("growing the box storage: ") + cudaGetErrorString(e))
+               : fail(A5G_ENOMEM, "cannot grow box storage to " + std::to_string(cap) + " boxes");
+  }
+  forget_tree(c);
+  RunDev &h = c->h;
+  auto take = [](auto *&mine, auto *&dev, auto *now) {
+    cudaFree(mine);
+    mine = now;
+    dev = now;
+  };
+  take(c->cc, h.cc, n.cc);
+  take(c->fx, h.fx, n.fx);
+  take(c->fy, h.fy, n.fy);
+  take(c->meta, h.meta, n.meta);
+  take(c->flags, h.flags, n.flags);
+  take(c->tags, h.tags, n.tags);
+  take(c->sumbuf, h.sumbuf, n.sumbuf);
+  if (ls) {
+    take(c->lsf, h.lsf, n.lsf);
+    take(c->bval, h.bval, n.bval);
+  }
+  if (ph) {
+    take(c->ph_ncr, h.ph_ncr, n.ph_ncr);
+    take(c->ph_cnt, h.ph_cnt, n.ph_cnt);
+    take(c->ph_ipart, h.ph_ipart, n.ph_ipart);
+    take(c->ph_part, h.ph_part, n.ph_part);
+    take(c->ph_u, h.ph_u, n.ph_u);
+    h.ph_cap = (int)src;
   }
   if (c->cc32) {  // scratch of the mixed form: reallocated at the next mixed launch
     cudaFree(c->cc32);
     c->cc32 = nullptr;
     c->cc32_cap = 0;
-    c->h.cc32 = nullptr;
+    h.cc32 = nullptr;
   }
-  return ph_resize(c);
+  c->capacity = cap;
+  h.capacity = cap;
+  return A5G_OK;
 }
 
 int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int *meta16,
@@ -1526,13 +1536,16 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
   }
   int r = grow(c, max_id + 1);
   if (r) return r;
+  forget_tree(c);
   CK(cudaMemcpyAsync(c->meta, hm.data(), hm.size() * sizeof(BoxMeta), cudaMemcpyHostToDevice,
                      c->stream));
   if (lists.size() + 1 > c->lists_cap) {
+    const size_t n = std::max(lists.size() + 1, 2 * c->lists_cap);
     cudaFree(c->lists);
     c->lists = nullptr;
-    c->lists_cap = std::max(lists.size() + 1, 2 * c->lists_cap);
-    CK(cudaMalloc(&c->lists, c->lists_cap * sizeof(int)));
+    c->lists_cap = 0;
+    CK(tree_malloc(c, &c->lists, n));
+    c->lists_cap = n;
   }
   if (!lists.empty())
     CK(cudaMemcpyAsync(c->lists, lists.data(), lists.size() * sizeof(int), cudaMemcpyHostToDevice,
@@ -1620,14 +1633,10 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
   c->topo.ids = lv_ids;
   c->topo.leaves = lv_leaves;
   c->topo.parents = lv_parents;
-  // (the dense levels and their captured solves belong to the old topology
-  // and storage)
-  a5u_destroy(c->uni);
-  c->uni = nullptr;
-  c->uni_checked = false;
-  c->has_tree = true;
   CK(cudaStreamSynchronize(c->stream));
-  return push_run(c);
+  if ((r = push_run(c))) return r;
+  c->has_tree = true;
+  return A5G_OK;
 }
 
 int a5g_upload_cc(a5g_ctx *c, int iv, const double *host) {
@@ -2384,6 +2393,7 @@ int a5g_batch_launch(a5g_batch *b, int num_steps, int use_graph) {
   for (int k = 0; k < n; k++) {
     a5g_ctx *c = b->ctxs[k];
     int r;
+    if (!c->has_tree) return fail(A5G_ESTATE, "batch member without tree");
     if (c->p.photoi_enabled && (r = ph_ready(c))) return r;
     if ((r = mx_ready(c))) return r;
   }
@@ -2468,6 +2478,15 @@ extern "C" int a5g_debug_set_staging(a5g_ctx *c, int allow_smem) {
   int r = push_run(c);
   if (r) return r;
   return mx_ready(c);
+}
+
+// Diagnostics: the n-th of the next device allocations that follow the tree
+// (box storage, lists, plans) reports that memory is short, as the call that
+// made it would. 0: none. Not part of the public interface.
+extern "C" int a5g_debug_fail_alloc(a5g_ctx *c, int n) {
+  if (!c || n < 0) return fail(A5G_EINVAL, "bad argument");
+  c->fail_alloc = n;
+  return A5G_OK;
 }
 
 int a5g_set_applied_field(a5g_ctx *c, double applied_fld) {

@@ -123,7 +123,10 @@ int a5g_set_rng(a5g_ctx *ctx, const int *state4);
 
 /* Topology upload after a$D_set_base / a$D_adjust_refinement
  * (afivo/src/m_aX_core.f90:134-217, 456-520). Cell and face data of ids
- * that stay in use are preserved on the device; storage grows as needed. */
+ * that stay in use are preserved on the device; storage grows as needed.
+ * Where the storage cannot grow (A5G_ENOMEM) the run keeps its old tree; a
+ * failure after that leaves it without one, and calls that need a tree return
+ * A5G_ESTATE until an upload has gone through. */
 int a5g_upload_tree(a5g_ctx *ctx, int max_id, int min_lvl, int max_lvl,
                     const int *meta16, const double *geom4,
                     const int *lvl_counts, const int *lvl_ids);
