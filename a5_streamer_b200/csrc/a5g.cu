@@ -343,7 +343,8 @@ inline int4 make_plan(const BoxRec &B, int nc, int ncg, int i, int j, int parent
 }
 
 // box_gsrb_clpl weights (i+ioff-1)/(i+ioff-1/2) and (i+ioff)/(i+ioff-1/2)
-__host__ __device__ __forceinline__ void cyl_weights(int gi, double &rf1, double &rf2) {
+template <class I>
+__host__ __device__ __forceinline__ void cyl_weights(I gi, double &rf1, double &rf2) {
   const double den = gi - 0.5;
   rf1 = (gi - 1) / den;
   rf2 = gi / den;
@@ -575,7 +576,7 @@ static size_t step_smem(const a5g_ctx *c) { return c->precision == A5G_MIXED ? c
 struct HostPlans {
   std::vector<BoxRec> boxes, sboxes;
   std::vector<int4> cplan;      // per fitting level: 2 NTHR cell plans
-  std::vector<double2> cwts;    // and their cylindrical weights
+  std::vector<double2> cwts;    // cylindrical runs: the weights of the different columns of these levels
   int cplan_blk[MAXLEV];
   int smem_doubles = 0;  // doubles per variable of the compact shared-memory copy
   std::vector<int> pbx;
@@ -596,7 +597,7 @@ static void host_child_offset(const BoxMeta &m, int &o0, int &o1) {
 static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::vector<int>> &ids,
                         const std::vector<std::vector<int>> &leaves,
                         const std::vector<std::vector<int>> &parents, int min_lvl, int nlev,
-                        double dr_base, HostPlans &P) {
+                        double dr_base, bool cyl, HostPlans &P) {
   std::vector<char> is_leaf(hm.size(), 0), is_parent(hm.size(), 0);
   for (const auto &v : leaves)
     for (int id : v) is_leaf[id] = 1;
@@ -656,20 +657,42 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
       b.ch[q] = sb(b.ch[q]);
     }
   }
-  // Cell plans of every level whose colours have at most one cell per thread
-  // (the per-thread slots make_level_plan fills), on the shared-memory
-  // records: thread k takes cell item k & (half-1) of box k >> log2(half),
-  // its colour-0 and colour-1 cells in plan slots 2k and 2k+1.
+  // Cell plans of every level whose colours have at most one cell per thread,
+  // on the shared-memory records: thread k takes cell item k & (half-1) of box
+  // k >> log2(half), its colour-0 and colour-1 cells in plan slots 2k and
+  // 2k+1.
   P.cplan.clear();
   P.cwts.clear();
-  std::vector<int> columns;  // 1 + place in cwts of a column, 0: none yet
   for (int li = 0; li < MAXLEV; li++) P.cplan_blk[li] = -1;
+  if (P.smem_doubles > 65535) return;
+  auto planned = [&](int li) {
+    const int nb = P.bx_off[li + 1] - P.bx_off[li];
+    return nb * ((P.lv_nc[li] * P.lv_nc[li]) >> 1) <= NTHR;
+  };
+  // The different columns of these levels' boxes, sorted: a level has few
+  // boxes, however many columns it spans. A box's own are consecutive there.
+  std::vector<long long> columns;
+  auto column0 = [&](const BoxRec &B, int nc) { return (long long)(hm[B.gbase / SLOT].ix0 - 1) * nc; };
+  if (cyl) {
+    for (int li = 0; li < nlev; li++)
+      for (int b = P.bx_off[li]; planned(li) && b < P.bx_off[li + 1]; b++)
+        for (int i = 1; i <= P.lv_nc[li]; i++) columns.push_back(column0(P.sboxes[b], P.lv_nc[li]) + i);
+    std::sort(columns.begin(), columns.end());
+    columns.erase(std::unique(columns.begin(), columns.end()), columns.end());
+    P.cwts.resize(columns.size());
+    for (size_t k = 0; k < columns.size(); k++) cyl_weights(columns[k], P.cwts[k].x, P.cwts[k].y);
+  }
   for (int li = 0; li < nlev; li++) {
+    if (!planned(li)) continue;
     const int nc = P.lv_nc[li], ncg = nc + 2, half = (nc * nc) >> 1, hn = nc >> 1;
     const int sh = __builtin_ctz(nc), hsh = 2 * sh - 1;
     const int b0 = P.bx_off[li], nb = P.bx_off[li + 1] - b0;
-    if (nb * half > NTHR || P.smem_doubles > 65535) continue;
     P.cplan_blk[li] = (int)(P.cplan.size() / (2 * NTHR));
+    std::vector<int> place(nb, 0);  // of the box's first column, minus 1
+    if (cyl)
+      for (int b = 0; b < nb; b++)
+        place[b] = (int)(std::lower_bound(columns.begin(), columns.end(), column0(P.sboxes[b0 + b], nc) + 1) -
+                         columns.begin()) - 1;
     for (int k = 0; k < NTHR; k++) {
       int4 c[2];
       c[0] = c[1] = make_int4(0, 0, 0, 0);
@@ -681,15 +704,7 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
         const int pc = li > 0 ? B.pbase + (B.o0 + m + 1) + pncg * (B.o1 + ((j - 1) >> 1) + 1) : 0;
         for (int p = 0; p < 2; p++) {
           const int i = 2 * m + 2 - ((p + j) & 1);
-          const size_t gi = (size_t)(B.gi0 + i);
-          if (gi >= columns.size()) columns.resize(2 * gi, 0);
-          if (columns[gi] == 0) {
-            double2 w;
-            cyl_weights((int)gi, w.x, w.y);
-            P.cwts.push_back(w);
-            columns[gi] = (int)P.cwts.size();
-          }
-          c[p] = make_plan(B, nc, ncg, i, j, pc | (columns[gi] - 1) << 16);
+          c[p] = make_plan(B, nc, ncg, i, j, cyl ? pc | (place[k >> hsh] + i) << 16 : pc);
         }
       }
       P.cplan.push_back(c[0]);
@@ -745,7 +760,7 @@ extern "C" int a5g_debug_plans(int max_id, int min_lvl, int max_lvl, const int *
         if (kind == 2) lv_parents[li].push_back(id);
       }
   HostPlans P;
-  build_plans(hm, lv_ids, lv_leaves, lv_parents, min_lvl, nlev, dr_base, P);
+  build_plans(hm, lv_ids, lv_leaves, lv_parents, min_lvl, nlev, dr_base, true, P);
   if (sizes) {
     sizes[0] = (int)P.boxes.size();
     sizes[1] = (int)P.pbx.size();
@@ -1551,7 +1566,7 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
     CK(cudaMemcpyAsync(c->lists, lists.data(), lists.size() * sizeof(int), cudaMemcpyHostToDevice,
                        c->stream));
   HostPlans P;
-  build_plans(hm, lv_ids, lv_leaves, lv_parents, min_lvl, nlev, c->p.dr_base, P);
+  build_plans(hm, lv_ids, lv_leaves, lv_parents, min_lvl, nlev, c->p.dr_base, c->p.coord == 1, P);
   if ((r = upload_vec(c, c->p_boxes, c->cap_boxes, P.boxes)) ||
       (r = upload_vec(c, c->p_sboxes, c->cap_sboxes, P.sboxes)) ||
       (r = upload_vec(c, c->p_pbx, c->cap_pbx, P.pbx)) ||
@@ -1561,7 +1576,7 @@ int a5g_upload_tree(a5g_ctx *c, int max_id, int min_lvl, int max_lvl, const int 
   RunDev &h = c->h;
   {
     // keep the multigrid variables in shared memory when the tree fits
-    h.n_wts = c->p.coord == 1 ? (int)P.cwts.size() : 0;
+    h.n_wts = (int)P.cwts.size();
     const size_t need = (PLAN_DOUBLES + 2 * (size_t)h.n_wts) * sizeof(double) +
                         3 * (size_t)P.smem_doubles * sizeof(double) +
                         P.boxes.size() * sizeof(BoxRec) + P.pbx.size() * sizeof(int);
