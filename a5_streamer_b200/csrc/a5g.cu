@@ -457,6 +457,7 @@ struct a5g_ctx {
   bool uni_checked = false;
   BatchSlot *batch_tbl = nullptr;  // descriptors of a5g_step_batch with this run first: 2 batch_cap entries
   int batch_cap = 0;
+  std::vector<BatchSlot *> batch_old;  // outgrown tables (batch_table)
   cudaStream_t stream = nullptr;
   RunDev h{};
   RunDev *d_run = nullptr;
@@ -1161,6 +1162,7 @@ int a5g_destroy(a5g_ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   a5u_destroy(c->uni);
   cudaFree(c->batch_tbl);
+  for (BatchSlot *t : c->batch_old) cudaFree(t);
   cudaFree(c->d_run);
   cudaFree(c->cc);
   cudaFree(c->fx);
@@ -2050,6 +2052,25 @@ static int static_fill(BatchSlot *table, const BatchSlot *slots, int n, cudaStre
   }
   return A5G_OK;
 }
+// The table c0 keeps for batches it leads, of 2 n entries at least. It grows
+// by doubling, and an outgrown one lives on with c0: launches under way read
+// it, and a caller's captured batch holds its address (together they are
+// smaller than the one in use). A capture on this thread does not object to
+// the allocation.
+static int batch_table(a5g_ctx *c0, int n) {
+  if (n <= c0->batch_cap) return A5G_OK;
+  const int cap = std::max(n, 2 * c0->batch_cap);
+  BatchSlot *t = nullptr;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CK(cudaThreadExchangeStreamCaptureMode(&mode));
+  const cudaError_t e = cudaMalloc((void **)&t, 2 * (size_t)cap * sizeof(BatchSlot));
+  CK(cudaThreadExchangeStreamCaptureMode(&mode));
+  CK(e);
+  if (c0->batch_tbl) c0->batch_old.push_back(c0->batch_tbl);
+  c0->batch_tbl = t;
+  c0->batch_cap = cap;
+  return A5G_OK;
+}
 int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts) {
   if (!ctxs || !dts || n < 1) return fail(A5G_EINVAL, "bad batch");
   for (int k = 0; k < n; k++) {
@@ -2087,14 +2108,8 @@ int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts) {
   // table can be written again, and a call neither allocates nor copies (two
   // stream-ordered allocations a call, given back to the system at every
   // synchronisation, made single calls tens of milliseconds long).
-  if (c0->batch_cap < n) {
-    CK(cudaStreamSynchronize(c0->stream));
-    cudaFree(c0->batch_tbl);
-    c0->batch_tbl = nullptr;
-    c0->batch_cap = 0;
-    CK(cudaMalloc((void **)&c0->batch_tbl, 2 * (size_t)n * sizeof(BatchSlot)));
-    c0->batch_cap = n;
-  }
+  const int rt = batch_table(c0, n);
+  if (rt) return rt;
   const int rf = static_fill(c0->batch_tbl, slots.data(), any_ph ? 2 * n : n, c0->stream);
   if (rf) return rf;
   size_t dyn = 0;

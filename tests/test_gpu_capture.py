@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import a5ref
-from a5_streamer_b200 import _lib, config
+from a5_streamer_b200 import _lib, config, device
 from parity import device_from_oracle
 
 pytestmark = pytest.mark.gpu
@@ -82,4 +82,33 @@ def test_captured_grid_mode_call(what, mixed, solved_before):
     call(other)
     for iv in CELLS:
         assert np.array_equal(_inner(run, sim, iv), _inner(other, sim, iv)), iv
+    del g
+
+
+@pytest.mark.parametrize("name", ["cart", "photoi"])
+def test_captured_step_batch_outlives_larger_batches(name):
+    """A batch captured as the run's first (its descriptor table is made
+    during the capture), then larger batches that the run leads."""
+    cfg = config.cartesian_8mm() if name == "cart" else config.cylindrical_16mm(photoi=True)
+    sim = a5ref.Sim(cfg, n_threads=4)
+    sim.init()
+    runs = [device_from_oracle(sim, cfg) for _ in range(24)]
+    one = device_from_oracle(sim, cfg)
+    for r in runs + [one]:
+        if cfg.photoi_enabled:
+            r.set_photon_table(*sim.photon_table()[:2])
+            r.set_rng_state(sim.rng_state())
+    dt = [sim.get_max_dt()] * len(runs)
+    g, s = _capture(runs[0], lambda: device.step_batch(runs[:1], dt[:1]))
+    _replay(g, s)
+    for n in (2, 3, 24):
+        device.step_batch(runs[:n], dt[:n])
+        _replay(g, s)
+    for r in runs:
+        r.sync()
+    for _ in range(7):  # what the first run has done
+        device.step_batch([one], dt[:1])
+    one.sync()
+    for iv in range(device.N_VAR_CELL):
+        assert np.array_equal(runs[0].cc(iv), one.cc(iv)), iv
     del g
