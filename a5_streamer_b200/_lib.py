@@ -175,6 +175,8 @@ SIGNATURES.update({
     "a5g3_set_precision": (_I, [_P, _I, ctypes.POINTER(MGSchedule)]),
     "a5g3_get_precision": (_I, [_P, _PI, ctypes.POINTER(MGSchedule)]),
     "a5g3_stream": (_I, [_P, _PP]),
+    "a5g3_debug_set_dense": (_I, [_P, _I]), "a5g3_debug_fail_alloc": (_I, [_P, _I]),
+    "a5g3_debug_info": (_I, [_P, _PI]),
 })
 
 

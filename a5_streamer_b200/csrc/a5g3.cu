@@ -1207,6 +1207,7 @@ struct a5g3_ctx {
   // level grids fit its index arithmetic and its arrays could be allocated;
   // the box-slot phases serve otherwise.
   bool dense = false;
+  int fail_alloc = 0;  // diagnostics: which of the next resources of the dense or FP32 solve is short (0: none)
   int dtop = 0;        // levels min_lvl..dtop run in one block (k3d_coarse)
   long long dcells = 0;
   double *d_den = nullptr, *d_corr = nullptr;
@@ -1821,9 +1822,43 @@ static int ready(a5g3_ctx *c) {
   return A5G_OK;
 }
 
+// A device resource of the dense levels or the FP32 solve is to be had
+// (a5g3_debug_fail_alloc).
+static bool got(a5g3_ctx *c, cudaError_t e) {
+  if (c->fail_alloc > 0 && --c->fail_alloc == 0) return false;
+  return e == cudaSuccess;
+}
+template <class T>
+static bool solve_malloc(a5g3_ctx *c, T *&p, long long n) {
+  if (got(c, cudaMalloc((void **)&p, n * sizeof(T)))) return true;
+  if (p) cudaFree(p);
+  p = nullptr;
+  cudaGetLastError();
+  return false;
+}
+// Gives back what the dense levels take; the box-slot phases serve.
+static void drop_dense(a5g3_ctx *c) {
+  cudaStreamSynchronize(c->stream);
+  drop_graph(c);
+  c->dense = false;
+  if (c->d_org) cudaFree(c->d_org);
+  if (c->d_den) cudaFree(c->d_den);
+  if (c->d_den32) cudaFree(c->d_den32);
+  c->d_org = nullptr;
+  c->d_den = c->d_corr = c->d_dens = nullptr;
+  c->d_den32 = nullptr;
+  for (cudaEvent_t &e : c->ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
+  if (c->side) cudaStreamDestroy(c->side);
+  c->side = nullptr;
+  cudaGetLastError();
+}
+
 // The dense levels and their arrays. Leaves c->dense false (the box-slot
-// phases serve) where a level's grid is too large for the 32-bit index
-// arithmetic or device memory for the arrays is short.
+// phases serve) and nothing allocated where a level's grid is too large for
+// the 32-bit index arithmetic or device memory for the arrays is short.
 static void setup_dense(a5g3_ctx *c) {
   const a5g3_params &p = c->p;
   const int lo = c->min_lvl, hi = c->max_lvl, nlev = hi - lo + 1;
@@ -1857,9 +1892,8 @@ static void setup_dense(a5g3_ctx *c) {
   c->dcells = off;
   // the coarse section: levels of at most DCOARSE cells, never the finest
   DCoarse &C = c->dco;
+  C = DCoarse{};
   c->dtop = lo - 1;
-  C.cells = 0;
-  C.nwarp = 0;
   for (int l = lo; l < hi && C.n < 8 && 2 * D.lv[c->li(l)].half <= DCOARSE; l++) {
     const int q = c->li(l);
     C.lv[q] = D.lv[q];
@@ -1886,20 +1920,13 @@ static void setup_dense(a5g3_ctx *c) {
     cudaGetLastError();
     return;
   }
-  if (upload(c->d_org, org, c->stream) != A5G_OK) {
-    cudaGetLastError();
-    return;
-  }
   // P, F of every level, O of every level but the finest, the corrections,
   // and the step's dense densities
   const long long nO = D.lv[nlev - 1].off, nd = 2 * off + nO + coff + 6LL * D.lv[nlev - 1].half;
-  if (cudaMalloc((void **)&c->d_den, nd * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  for (cudaEvent_t &e : c->ev)
-    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return;
-  if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess) return;
+  bool ok = upload(c->d_org, org, c->stream) == A5G_OK && got(c, cudaSuccess) && solve_malloc(c, c->d_den, nd);
+  for (cudaEvent_t &e : c->ev) ok = ok && got(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  ok = ok && got(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+  if (!ok) return drop_dense(c);
   c->d_corr = c->d_den + 2 * off + nO;
   c->d_dens = c->d_corr + coff;
   c->dense = true;
@@ -2068,15 +2095,14 @@ int a5g3_set_precision(a5g3_ctx *c, int precision, const a5g_mg_schedule *sched)
     return fail3(A5G_EINVAL, "bad schedule (fmg 0/1, cycles 1..8, base 1..64, corrections 1..8)");
   if (precision == A5G_MIXED && c->dense && !c->d_den32) {
     const long long n = 2 * c->dcells + std::max(c->dall.lv[c->li(c->max_lvl)].off, 1LL);
-    if (cudaMalloc((void **)&c->d_den32, n * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      return fail3(A5G_ENOMEM, "device allocation of the FP32 multigrid storage failed");
-    }
+    // (where the dense levels leave no room for it, the box-slot phases, which
+    // take less in all, serve the run)
+    if (!solve_malloc(c, c->d_den32, n)) drop_dense(c);
   }
   if (precision == A5G_MIXED && !c->dense && !c->d_c32) {
-    const size_t n = (size_t)3 * c->cap * SLOT3;
-    if (cudaMalloc((void **)&c->d_c32, n * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
+    const long long n = 3 * c->cap * SLOT3;
+    if (!solve_malloc(c, c->d_c32, n)) {
+      setup_dense(c);  // as it was, for the FP64 form
       return fail3(A5G_ENOMEM, "device allocation of the FP32 multigrid storage failed");
     }
     // defined contents everywhere (ghost cells of coarse rhs are carried along)
@@ -2085,6 +2111,31 @@ int a5g3_set_precision(a5g3_ctx *c, int precision, const a5g_mg_schedule *sched)
   c->precision = precision;
   c->sched = s;
   drop_graph(c);
+  return A5G_OK;
+}
+
+// Diagnostics, not part of the public interface: the dense levels made (1,
+// where they can be) or given back (0), so that tests can run the box-slot
+// solves; in the FP64 form only, whose storage does not depend on it.
+int a5g3_debug_set_dense(a5g3_ctx *c, int on) {
+  if (!c) return fail3(A5G_EINVAL, "null context");
+  if (c->precision != A5G_FP64) return fail3(A5G_ESTATE, "change the form before the precision");
+  if (!on) drop_dense(c);
+  else if (!c->dense) setup_dense(c);
+  return launched(c);
+}
+// The n-th of the next resources of the dense levels or the FP32 solve is
+// refused, as the device would when memory is short; 0: none.
+int a5g3_debug_fail_alloc(a5g3_ctx *c, int n) {
+  if (!c || n < 0) return fail3(A5G_EINVAL, "bad argument");
+  c->fail_alloc = n;
+  return A5G_OK;
+}
+// out2: the dense levels are there; the step's transport is the fused one.
+int a5g3_debug_info(a5g3_ctx *c, int *out2) {
+  if (!c || !out2) return fail3(A5G_EINVAL, "null argument");
+  out2[0] = c->dense;
+  out2[1] = c->dense && c->eps_one && c->max_lvl > 1;
   return A5G_OK;
 }
 
