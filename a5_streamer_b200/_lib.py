@@ -109,6 +109,7 @@ SIGNATURES = {
     "a5g_get_stream": (_I, [_P, ctypes.POINTER(_P)]),
     "a5g_debug_set_staging": (_I, [_P, _I]),
     "a5g_debug_fail_alloc": (_I, [_P, _I]),
+    "a5g_debug_form": (_I, [_P, _PI]),
     "a5g_debug_info": (_I, [_P, ctypes.POINTER(ctypes.c_longlong)]),
     "a5g_debug_params_layout": (_I, [_PI, _I]),
     "a5g_debug_plans": (_I, [_I, _I, _I, _PI, _PD, _PI, _PI, _D, _PI, _PI, _P, _PI, _PD, _PI]),
@@ -193,6 +194,7 @@ SIGNATURES.update({
     "a5a_destroy": (_I, [_P]),
     "a5a_forward": (_I, [_P, _PD]),
     "a5a_gradient": (_I, [_P, _PD, _PD, _PD]),
+    "a5a_debug_form": (_I, [_P, _PI]),
     "a5a_debug_tape": (_I, [_I, _I, _I, _PI, _PD, _PI, _PI, _I, _I, _I,
                             ctypes.POINTER(ctypes.c_longlong), _PI, _PU, _PD, _PI, _PU, _PD]),
     "a5g_set_applied_field": (_I, [_P, _D]),

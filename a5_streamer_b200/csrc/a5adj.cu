@@ -1965,6 +1965,14 @@ int a5a_gradient(a5a_ctx *a, double *J, double *dJ_dtable, double *dJ_dV) {
   return A5G_OK;
 }
 
+// Diagnostics: the form of the multigrid's transpose, 1 the gather form in
+// shared memory, 2 the tape.
+int a5a_debug_form(a5a_ctx *a, int *out) {
+  if (!a || !out) return afail(A5G_EINVAL, "null argument");
+  *out = a->args.jS > 0 ? 1 : 2;
+  return A5G_OK;
+}
+
 int a5a_debug_tape(int max_id, int min_lvl, int max_lvl, const int *meta16, const double *geom4,
                    const int *lvl_counts, const int *lvl_ids, int capacity, int n_cycle_base,
                    int seg, long long *sizes, int *phase_row, unsigned *row_d, double *row_self,

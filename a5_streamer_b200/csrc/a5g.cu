@@ -449,9 +449,11 @@ static int fail(int code, const std::string &msg) {
                   std::string(#call) + ": " + cudaGetErrorString(e_));              \
   } while (0)
 
+enum { LF_BLOCK = 1, LF_CLUSTER, LF_GROUP, LF_DENSE };
 struct a5g_ctx {
   a5g_params p{};
   int device = -1;       // counted in g_alive
+  int last_form = 0;     // LF_: of the last single-run operation or step
   // grid mode on a uniformly refined tree: its dense levels (uniform_of)
   A5Uniform *uni = nullptr;
   bool uni_checked = false;
@@ -912,12 +914,15 @@ static int launch_smem(a5g_ctx *c, const Op &op, size_t smem) {
     const Op *ops = nullptr;
     void *args[] = {(void *)&run, (void *)&o, (void *)&runs, (void *)&ops};
     CK(cudaLaunchCooperativeKernel((const void *)F.run, dim3(c->n_cta), dim3(NTHR), args, 0, c->stream));
+    c->last_form = LF_GROUP;
     return A5G_OK;
   }
   if (cluster_run(c, op.code)) {
     CK(launch_cluster(kClusterForm.run, smem, c->stream, c->d_run, op, nullptr, nullptr));
+    c->last_form = LF_CLUSTER;
     return A5G_OK;
   }
+  c->last_form = &F == &kBlockForm ? LF_BLOCK : LF_GROUP;
   F.run<<<1, NTHR, smem, c->stream>>>(c->d_run, op, nullptr, nullptr);
   CK(cudaGetLastError());
   return A5G_OK;
@@ -1743,6 +1748,7 @@ static bool solve_uniform(a5g_ctx *c, bool mixed, int &r) {
   A5Uniform *u = uniform_of(c, mixed, a);
   if (!u) return false;
   const cudaError_t e = (cudaError_t)a5u_solve(u, mixed, c->stream);
+  c->last_form = LF_DENSE;
   r = e == cudaSuccess ? A5G_OK : fail(A5G_ECUDA, std::string("dense field solve: ") + cudaGetErrorString(e));
   return true;
 }
@@ -1916,20 +1922,24 @@ int a5g_step(a5g_ctx *c, double dt) {
         if (r) return r;
         CK((cudaError_t)a5u_solve(u, mixed, c->stream));
       }
+      c->last_form = LF_DENSE;
       return A5G_OK;
     }
     const RunDev *run = c->d_run;
     void *args[] = {(void *)&run, (void *)&dt, (void *)&deposit};
     CK(cudaLaunchCooperativeKernel(fn, dim3(c->n_cta), dim3(NTHR), args, 0, c->stream));
+    c->last_form = LF_GROUP;
     return A5G_OK;
   }
   if (cluster_run(c, OP_STEP)) {
+    c->last_form = LF_CLUSTER;
     if (c->precision == A5G_MIXED)
       CK(launch_cluster(kClusterForm.step_mixed, c->dyn_smem32, c->stream, c->d_run, dt, deposit));
     else
       CK(launch_cluster(kClusterForm.step, c->dyn_smem, c->stream, c->d_run, dt, deposit));
     return A5G_OK;
   }
+  c->last_form = &F == &kBlockForm ? LF_BLOCK : LF_GROUP;
   if (c->precision == A5G_MIXED)
     F.step_mixed<<<1, NTHR, c->dyn_smem32, c->stream>>>(c->d_run, dt, deposit);
   else
@@ -2508,6 +2518,15 @@ extern "C" int a5g_debug_set_staging(a5g_ctx *c, int allow_smem) {
   int r = push_run(c);
   if (r) return r;
   return mx_ready(c);
+}
+
+// Diagnostics: the form of the run's last operation or step outside a batch:
+// 1 one block, 2 a cluster, 3 the group form (several blocks, or level-set
+// boxes), 4 with its field solves on dense levels; 0: none yet.
+extern "C" int a5g_debug_form(a5g_ctx *c, int *out) {
+  if (!c || !out) return fail(A5G_EINVAL, "null argument");
+  *out = c->last_form;
+  return A5G_OK;
 }
 
 // Diagnostics: the n-th of the next device allocations that follow the tree
