@@ -672,18 +672,31 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
     const int nb = P.bx_off[li + 1] - P.bx_off[li];
     return nb * ((P.lv_nc[li] * P.lv_nc[li]) >> 1) <= NTHR;
   };
-  // The different columns of these levels' boxes, sorted: a level has few
-  // boxes, however many columns it spans. A box's own are consecutive there.
-  std::vector<long long> columns;
-  auto column0 = [&](const BoxRec &B, int nc) { return (long long)(hm[B.gbase / SLOT].ix0 - 1) * nc; };
+  // The different columns of these levels' boxes, and each box's place of its
+  // first one, minus 1: a level has few boxes, however many columns it spans,
+  // and a box's columns are consecutive.
+  std::vector<int> place(P.boxes.size(), 0);
   if (cyl) {
+    struct Span {
+      long long first;
+      int n, box;
+    };
+    std::vector<Span> spans;
     for (int li = 0; li < nlev; li++)
       for (int b = P.bx_off[li]; planned(li) && b < P.bx_off[li + 1]; b++)
-        for (int i = 1; i <= P.lv_nc[li]; i++) columns.push_back(column0(P.sboxes[b], P.lv_nc[li]) + i);
-    std::sort(columns.begin(), columns.end());
-    columns.erase(std::unique(columns.begin(), columns.end()), columns.end());
-    P.cwts.resize(columns.size());
-    for (size_t k = 0; k < columns.size(); k++) cyl_weights(columns[k], P.cwts[k].x, P.cwts[k].y);
+        spans.push_back({(long long)(hm[P.boxes[b].gbase / SLOT].ix0 - 1) * P.lv_nc[li] + 1, P.lv_nc[li], b});
+    std::sort(spans.begin(), spans.end(), [](const Span &a, const Span &b) { return a.first < b.first; });
+    long long next = LLONG_MIN;  // the column after those that have a place
+    for (const Span &s : spans) {
+      next = std::max(next, s.first);
+      for (; next < s.first + s.n; next++) {
+        double2 w;
+        cyl_weights(next, w.x, w.y);
+        P.cwts.push_back(w);
+      }
+      // (columns up to next - 1 have the last places, without gaps from s.first on)
+      place[s.box] = (int)((long long)P.cwts.size() - (next - s.first)) - 1;
+    }
   }
   for (int li = 0; li < nlev; li++) {
     if (!planned(li)) continue;
@@ -691,11 +704,6 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
     const int sh = __builtin_ctz(nc), hsh = 2 * sh - 1;
     const int b0 = P.bx_off[li], nb = P.bx_off[li + 1] - b0;
     P.cplan_blk[li] = (int)(P.cplan.size() / (2 * NTHR));
-    std::vector<int> place(nb, 0);  // of the box's first column, minus 1
-    if (cyl)
-      for (int b = 0; b < nb; b++)
-        place[b] = (int)(std::lower_bound(columns.begin(), columns.end(), column0(P.sboxes[b0 + b], nc) + 1) -
-                         columns.begin()) - 1;
     for (int k = 0; k < NTHR; k++) {
       int4 c[2];
       c[0] = c[1] = make_int4(0, 0, 0, 0);
@@ -707,7 +715,7 @@ static void build_plans(const std::vector<BoxMeta> &hm, const std::vector<std::v
         const int pc = li > 0 ? B.pbase + (B.o0 + m + 1) + pncg * (B.o1 + ((j - 1) >> 1) + 1) : 0;
         for (int p = 0; p < 2; p++) {
           const int i = 2 * m + 2 - ((p + j) & 1);
-          c[p] = make_plan(B, nc, ncg, i, j, cyl ? pc | (place[k >> hsh] + i) << 16 : pc);
+          c[p] = make_plan(B, nc, ncg, i, j, cyl ? pc | (place[b0 + (k >> hsh)] + i) << 16 : pc);
         }
       }
       P.cplan.push_back(c[0]);
