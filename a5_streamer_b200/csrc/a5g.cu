@@ -869,13 +869,14 @@ static const Form &batch_form(a5g_ctx *const *ctxs, int n) {
 }
 
 // A run outside a batch takes a cluster of CLUSTER blocks while the clusters
-// of all runs alive on the device fit its SMs together, one block otherwise.
-// The transport, the field and the staging of a solve spread over the
-// cluster; the shared-memory multigrid stays on its first block, so more
-// blocks gain less and less (8 mm tree, ten steps: 5.64 ms on one block,
-// 5.28, 4.77 and 4.58 on 2, 4 and 8; axisymmetric tree with photons 8.46 and
-// 8.45, 8.13, 7.93). Many runs on streams of their own use the SMs better
-// with one block each: 48 field solves 0.89 ms, as clusters 1.9 ms.
+// of all runs alive on the device fit its SMs together, and its tree has
+// enough boxes for the operation (cluster_pays); one block otherwise. The
+// transport, the field and the staging of a solve spread over the cluster; the
+// shared-memory multigrid stays on its first block, so more blocks gain less
+// and less (8 mm tree, ten steps: 5.64 ms on one block, 5.28, 4.77 and 4.58 on
+// 2, 4 and 8; axisymmetric tree with photons 8.46 and 8.45, 8.13, 7.93). Many
+// runs on streams of their own use the SMs better with one block each: 48
+// field solves 0.89 ms, as clusters 1.9 ms.
 constexpr int CLUSTER = 8;
 static std::mutex g_alive_mu;
 static int g_alive[256], g_sms[256];  // contexts and SMs per device
@@ -888,8 +889,42 @@ static void count_alive(int dev, int d) {
     g_sms[dev] = 0;
   }
 }
+// Whether the cluster's blocks outweigh its barriers, from times of both forms
+// on trees of 7 to 3,132 boxes (cluster / one block):
+// - whole-tree phases gain from some 40 boxes on (fluxes of 48 boxes 0.82, of
+//   96 0.40; with 7 to 28 boxes the launch costs what they gain), and so do
+//   steps and solves in shared memory (step of 7 boxes 1.17, 28 1.03, 54
+//   0.94, 96 0.80), in the mixed form, whose FP32 cycles are shorter, from 64
+//   (48 boxes 1.10 to 1.17, 54 1.01 to 1.08, 96 0.83);
+// - phases level by level in device memory pay a cluster barrier each, so what
+//   counts is the boxes a level has: steps of trees and of dielectric runs that
+//   do not fit shared memory 1.70 at 6 boxes a level, 1.42 at 20, 1.14 at 30,
+//   0.69 at 60, 0.61 at 74, 0.29 at 230; ghost cells likewise;
+// - restriction, step-size reductions and prolongation have a phase or two a
+//   level and little in it: 1.2 at 30, 0.95 to 1.08 at 60, 0.9 at 74.
+static bool cluster_pays(const a5g_ctx *c, int code) {
+  const RunDev &h = c->h;
+  const int boxes = h.bx_off[h.nlev];
+  const bool mixed = code == OP_COMPUTE_FLD_MIXED || (code == OP_STEP && c->precision == A5G_MIXED);
+  if (boxes < 40) return false;
+  switch (code) {
+    case OP_STEP:
+    case OP_COMPUTE_FLD:
+    case OP_COMPUTE_FLD_MIXED:
+    case OP_FMG:
+    case OP_VCYCLE:
+      if (mixed ? h.mx_smem > 0 : h.smem_doubles > 0 && !h.diel) return !mixed || boxes >= 64;
+      return boxes >= 40 * h.nlev;
+    case OP_GC: return boxes >= 40 * h.nlev;
+    case OP_RESTRICT:
+    case OP_DT_RED:
+    case OP_PROLONG_NEW: return boxes >= 64 * h.nlev;
+    default: return true;
+  }
+}
 static bool cluster_run(const a5g_ctx *c, int code) {
   if (c->n_cta > 1 || c->h.has_lsf || !grid_op(code) || c->device < 0 || c->device >= 256) return false;
+  if (!cluster_pays(c, code)) return false;
   std::lock_guard<std::mutex> lock(g_alive_mu);
   return CLUSTER * g_alive[c->device] <= g_sms[c->device];
 }

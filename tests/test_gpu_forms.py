@@ -29,10 +29,21 @@ def _equal(a, b, ivs, where):
         assert np.array_equal(a.cc(iv), b.cc(iv), equal_nan=True), (where, iv)
 
 
-@pytest.mark.parametrize("mixed", [False, True])
-@pytest.mark.parametrize("name", ["cart", "cyl_photoi"])
-def test_cluster_and_one_block(name, mixed):
-    cfg = config.cartesian_8mm() if name == "cart" else config.cylindrical_16mm(photoi=True)
+WIDE = dict(n_base=(12, 12), domain_len=(96e-3, 96e-3), lvls_max=6)
+# configuration, precision; form of a step and a solve on an otherwise empty device
+CLUSTERS = {
+    "cart": (config.cartesian_8mm(), False),  # 96 boxes, solves in shared memory
+    "cart_mixed": (config.cartesian_8mm(), True),
+    "cyl_photoi": (config.cylindrical_16mm(photoi=True), False),  # 54
+    "wide": (config.cylindrical_16mm(**WIDE), False),  # 484, in device memory
+    "wide_mixed": (config.cylindrical_16mm(**WIDE), True),
+    "wide_diel": (config.cylindrical_16mm(epsilon_diel=3.0, **WIDE), False),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CLUSTERS))
+def test_cluster_and_one_block(name):
+    cfg, mixed = CLUSTERS[name]
     gc.collect()  # runs that earlier tests have dropped
     sim = streamer.Simulation(cfg)
     sim.init()
@@ -56,6 +67,37 @@ def test_cluster_and_one_block(name, mixed):
     advance(b, BLOCK)
     _equal(a, b, range(9), name)
     del crowd
+
+
+def test_cluster_rule():
+    """Forms by tree and operation on an otherwise empty device: few boxes, or
+    few boxes a level where the phases go through device memory, take one
+    block."""
+    gc.collect()
+
+    def forms(cfg, mixed=False):
+        sim = streamer.Simulation(cfg)
+        sim.init()
+        r = device.clone_state(sim, mixed)
+        out = []
+        for f in (lambda: r.step(1e-15), lambda: r.compute_fld(False), lambda: r.fluxes_koren(1e-15),
+                  lambda: r.gc_tree(0), lambda: r.restrict_tree(0), r.dt_reductions):
+            f()
+            out.append("-BC"[_form(r)])
+        return "".join(out)
+
+    uni = lambda level, n: config.cartesian_uniform(level, n_base=n, domain_len=tuple(2e-3 * k for k in n))
+    # step, solve, fluxes, ghost cells, restriction, reductions
+    assert forms(uni(2, (1, 1))) == "BBBBBB"  # 7 boxes
+    assert forms(config.cylindrical_16mm()) == "CCCBBB"  # 54
+    assert forms(config.cylindrical_16mm(), True) == "BBCBBB"
+    assert forms(config.cartesian_8mm()) == "CCCBBB"  # 96
+    assert forms(config.cartesian_8mm(), True) == "CCCBBB"
+    assert forms(config.cylindrical_16mm(epsilon_diel=3.0)) == "BBCBBB"  # dielectric: solves in device memory
+    assert forms(uni(2, (4, 4))) == "BBCBBB"  # 112: beyond shared memory in FP64, not in FP32
+    assert forms(uni(2, (4, 4)), True) == "CCCBBB"
+    assert forms(uni(2, (6, 6))) == "CCCCBB"  # 63 a level
+    assert forms(uni(3, (4, 4))) == "CCCCCC"  # 73
 
 
 @pytest.mark.parametrize("mixed", [False, True])
