@@ -300,8 +300,9 @@ enum { GK_COPY = 0, GK_RB = 1, GK_NEG = 2, GK_TOP = 3 };
 // A cell plan as an int4 of 16-bit addresses in the shared-memory arrays:
 // x = cell | lx source << 16, y = hx source | ly source << 16, z = hy source |
 // VF_ flags << 16, w = parent cell of the 2 x 2 block the cell's thread
-// restricts (p_visit) | place of its column's weights << 16. The source of a neighbour is the neighbour's cell, or
-// for a ghost neighbour the first source of its recipe.
+// restricts (p_visit) | place of its column's weights << 16. The source of a
+// neighbour is the neighbour's cell, or for a ghost neighbour the first source
+// of its recipe.
 enum { VF_ON = 1, VF_RBX = 2, VF_XL = 4, VF_RBY = 8, VF_YL = 16, VF_NEG = 32, VF_TOP = 64, VF_ODDI = 128, VF_ODDJ = 256,
        VF_PARENT = 512 };
 
@@ -2093,7 +2094,9 @@ static int batch_order_out(a5g_ctx *const *ctxs, int n, cudaStream_t s, cudaEven
   return A5G_OK;
 }
 
-// The descriptors of a launch into a table on the device, by kernel parameters.
+// Writes the n descriptors of one launch into a table on the device on stream
+// s, as kernel parameters of fill launches (ordered with the launch that reads
+// them like any other work of the stream).
 static int static_fill(BatchSlot *table, const BatchSlot *slots, int n, cudaStream_t s) {
   for (int k0 = 0; k0 < n; k0 += SLOT_FILL) {
     const int m = std::min(SLOT_FILL, n - k0);
@@ -2187,10 +2190,6 @@ int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts) {
 // device current.
 static std::mutex g_static_mu;
 static BatchSlot *g_static_dev[256] = {};
-
-// Writes the n descriptors of one launch into the fixed table on stream s,
-// as kernel parameters of fill launches (ordered with the launch that reads
-// them like any other work of the stream).
 
 int a5g_step_batch_static(a5g_ctx **ctxs, int n, const double *dts) {
   if (!ctxs || !dts || n < 1) return fail(A5G_EINVAL, "bad batch");

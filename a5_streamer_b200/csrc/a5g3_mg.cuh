@@ -14,11 +14,10 @@
 // launch latency bounds the small levels', which is why the set-up of the
 // coarse right-hand side is part of the sweeps of a level's first visit and
 // the smallest levels run in one block (k3d_coarse).
-// Measured against the box-slot phases (launch list of one step, us): FP64
-// cube of level 4 (262,144 cells) 1,644 -> 926, of it the one-block section
-// 880 -> 385 and the half-sweeps 249 -> 185; level 6 (16.8M cells) 11,319 ->
-// 8,460, half-sweeps 2,593 -> 1,362 (a finest one 140 -> about 50); mixed
-// form on 2 x 1 x 3 base boxes, level 4 (1.6M cells) 2,481 -> 1,454.
+// Measured against the box-slot phases (launch list of one FP64 step, us; the
+// step's transport apart, which was fused later): cube of level 4 (262,144
+// cells) one-block section 880 -> 246, half-sweeps 249 -> 182; level 6 (16.8M
+// cells) half-sweeps 2,593 -> 1,226, a finest one 140 -> 35 (5.8 TB/s).
 //
 // Every value is formed by the reference's expression in its order, as the
 // slot form does (k3_phase), so both give the same doubles. Notation of a
@@ -37,8 +36,8 @@ struct DLv {
   double dx2, inv_dx2;
 };
 
-// t / d through the high product; exact for t * d < 2^32 with m = ceil(2^32 / d)
-// (t below the rows or cells of a level, checked at creation), d = 1 apart
+// t / d through the high product; exact for t (m d - 2^32) < 2^32 with m =
+// ceil(2^32 / d), which setup_dense checks for every t of a level; m 0 for d = 1
 __host__ __device__ __forceinline__ unsigned fastdiv(unsigned t, unsigned m) {
 #ifdef __CUDA_ARCH__
   return m ? __umulhi(t, m) : t;

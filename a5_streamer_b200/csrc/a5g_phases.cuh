@@ -67,8 +67,9 @@ __device__ __forceinline__ void PSYNC() {
   else cluster_sync();
 }
 
-// Cluster form: the shared-memory multigrid is the first block's. The other blocks reach its arrays by their addresses in that block's
-// window (cluster_map), to stage the potential in and out together.
+// Cluster form: the shared-memory multigrid is the first block's. The other
+// blocks reach its arrays by their addresses in that block's window
+// (cluster_map), to stage the potential in and out together.
 template <class T>
 __device__ __forceinline__ T *cluster_map(T *p, int rank) {
   unsigned long long a = reinterpret_cast<unsigned long long>(p), r;
@@ -1435,8 +1436,8 @@ __device__ __forceinline__ void local_end(int size) {
 // coarse ghost fill + rhs; base: 2 n_cycle_base half-sweeps + ghost fill;
 // up: correction, 4 half-sweeps, ghost fill. In grid mode the levels up to
 // local_top run on one block (the down, base and up phases of those levels
-// are consecutive). enter: flags of the first visit (p_enter); after: the level index whose plans the caller's next
-// visit takes (out of range: none).
+// are consecutive). enter: flags of the first visit (p_enter); after: the
+// level index whose plans the caller's next visit takes (out of range: none).
 template <class T>
 __device__ __forceinline__ void vcycle_body(const RunDev &R, const MGV<T> &M, int max_lvl, bool stale_base,
                                             PlanFetch &pf, int after, int enter) {

@@ -98,7 +98,11 @@ const char *a5g_last_error(void);
 int a5g_version(void);
 
 /* Context life cycle. Replaces a$D_init (afivo/src/m_aX_core.f90:47-116):
- * the device context owns all box storage. */
+ * the device context owns all box storage. Operations of a single run take a
+ * cluster of eight thread blocks where its tree is large enough for them to
+ * gain, and while eight blocks for every context alive on the device fit its
+ * SMs (up to 18 contexts on a B200); idle contexts count, so destroy those no
+ * longer needed. Otherwise they take one block. Results do not depend on it. */
 int a5g_create(const a5g_params *p, a5g_ctx **out);
 int a5g_destroy(a5g_ctx *ctx);
 
@@ -267,8 +271,8 @@ int a5g_step_batch(a5g_ctx **ctxs, int n, const double *dts);
  *
  * Some callers cannot allocate device memory while they step: a host that
  * fixed its device-memory budget before the time loop, or one whose stepping
- * path must not block on the allocator (cudaMallocAsync may wait on the
- * memory pool). This entry point keeps the per-run descriptor table of the
+ * path must not block on the allocator (a5g_step_batch allocates when a run
+ * leads a larger batch than before). This entry point keeps the per-run descriptor table of the
  * launch in a fixed file-scope device array of A5G_STATIC_BATCH_MAX entries
  * (40 KiB), held by every GPU that loads the library until the process
  * exits, and calls no allocating routine. The caller still creates the
@@ -342,7 +346,8 @@ int a5g_set_level_set(a5g_ctx *ctx, const double *lsf, const double *bval);
  * launch of n_cta co-resident blocks that share each phase's items, with a
  * grid barrier between phases; results are identical to one block. (Where
  * every level of a Cartesian run's tree is complete, the field solves with a
- * guess run as kernels of their own on the whole GPU.) Each
+ * guess run as kernels of their own on the whole GPU, except in a caller's
+ * capture of the run's stream.) Each
  * barrier wait is bounded by wait_cycles SM clock cycles (< 0: the default,
  * A5G_DEFAULT_WAIT_CYCLES); a wait that runs out makes the launch return
  * early and the next synchronising call report A5G_TIMEOUT (0 makes every

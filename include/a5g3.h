@@ -82,6 +82,9 @@ int a5g3_set_table(a5g3_ctx *ctx, int n_rows, int n_cols, double x_min, double i
 int a5g3_set_init_cond(a5g3_ctx *ctx, double bg_dens, int n_seeds, const double *r0, const double *r1,
                        const double *dens, const double *width, const int *falloff);
 
+/* Steps run fastest while eps is known to be 1 everywhere: from
+ * a5g3_set_init_cond until eps (variable 8) is written by an upload or a copy,
+ * whatever its values. */
 int a5g3_upload_cc(a5g3_ctx *ctx, int iv, const double *host);
 int a5g3_download_cc(a5g3_ctx *ctx, int iv, double *host);
 int a5g3_upload_fc(a5g3_ctx *ctx, int dimf, int f, const double *host);
@@ -121,7 +124,9 @@ int a5g3_step(a5g3_ctx *ctx, double dt);
  * wall values and the schedule sched (NULL: the reference's FMG, 2, 2,
  * n_cycle_base, one pass), and the FP64 accumulation of the potential. The
  * densities, potential, field and step-size reductions stay FP64. The first
- * call allocates 3 FP32 variables of the box capacity. A first solve (no
+ * call allocates the FP32 multigrid storage (about 2.4 floats a leaf cell;
+ * where that does not fit beside the dense levels, these are given back and
+ * the solves work on box slots with 3 floats a slot entry). A first solve (no
  * guess) stays FP64. */
 int a5g3_set_precision(a5g3_ctx *ctx, int precision, const a5g_mg_schedule *sched);
 int a5g3_get_precision(a5g3_ctx *ctx, int *precision, a5g_mg_schedule *sched);
