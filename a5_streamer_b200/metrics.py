@@ -83,6 +83,51 @@ def bytes_per_step_3d(run) -> float:
     return bytes_per_step(census3(run.meta(), run.levels(), run.nc))
 
 
+def moved_bytes_per_step_3d(c: Census, n_down: int = 2, n_up: int = 2, n_base: int = 8,
+                            word: int = 8) -> float:
+    """What the kernels of one FP64 step of the 3D form must move (eps 1
+    everywhere: fused transport, dense levels), each array a kernel needs read
+    once and each it forms written once, on the cells of the level it works on
+    (ghost entries left out). The model above counts the reference's separate
+    operations instead, more than half of which the fused kernels do not move.
+
+    Per leaf cell, in words: stage 1 reads n_e, n_i, |E|, phi and three face
+    fields and writes both old densities, P, F and both new densities (13);
+    stage 2 reads n_e, n_i and P and writes both densities and three fluxes
+    (8); the end of the transport reads the old and new densities and writes
+    both averages and the space charge twice (8); the field reads P and writes
+    phi, |E| and three face fields (6); the restriction reads both (2). Per
+    cell of a parent box on levels >= 1: copies 4, restriction 2 and average 6,
+    and twice the right-hand side (2) and the field (6).
+
+    A half-sweep of a dense level reads one colour of P and of F and writes
+    the other colour (1.5 words a cell), 2.5 more on the two that first visit a
+    level. Residual and restriction read P and F and write three arrays of the
+    coarser level; a correction reads and writes one colour and reads two
+    coarser arrays (and writes the kept one)."""
+    lo, hi, n = c.min_lvl, c.max_lvl, c.cells
+    leaf = n[hi]
+    par = sum(v for l, v in n.items() if 1 <= l < hi)
+    total = (13 + 8 + 8 + 6 + 2) * leaf + (4 + 2 + 6 + 2 * (2 + 6)) * par
+
+    def down(l):
+        return 2 * n[l] + 3 * n[l - 1]
+
+    def up(l):
+        return n[l] + 3 * n[l - 1]
+
+    solve = sum(down(l) + (n[l] if l < hi else 0) for l in range(hi, lo, -1))
+    for top in range(lo, hi + 1):
+        if top > lo:
+            solve += up(top)
+        for l in range(top, lo, -1):
+            solve += 2 * n_down * 1.5 * n[l] + (2.5 * n[l] if l < top else 0) + down(l)
+        solve += 2 * n_base * 1.5 * n[lo]
+        for l in range(lo + 1, top + 1):
+            solve += up(l) + 2 * n_up * 1.5 * n[l]
+    return word * (total + 2 * solve)
+
+
 def bytes_per_step(c: Census, n_down: int = 2, n_up: int = 2, word: int = 8,
                    photons: float = 0.0) -> float:
     """Algorithmic bytes of one full step; photons > 0 adds the photon
