@@ -1352,6 +1352,7 @@ int a5g_set_photon_table(a5g_ctx *c, int n_rows, double x_min, double inv_dx, co
   c->ph_tbl = nullptr;
   CK(cudaMalloc(&c->ph_tbl, sizeof(double) * n_rows));
   CK(cudaMemcpyAsync(c->ph_tbl, dist, sizeof(double) * n_rows, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));  // (dist is the caller's again)
   c->h_ph_tbl.assign(dist, dist + n_rows);
   // pi_lengthscale = LT_get_col(tbl, 1, fac_dx) and get_lvl_length
   // (src/m_photons.f90:142-155, 331-336)
